@@ -361,8 +361,11 @@ def work(case):
 def tolerance(case):
     kind = case["kind"]
     if kind == "density":
-        # sums in double; a target whose residual sits at the tolerance may stop an iteration apart
-        return {"rel": 1e-9, "max": 1e-6, "differ": 1e-5}
+        # Sums in double, but the face-closure correction switches on and off with h: some targets near
+        # its threshold do not settle (up to 100 iterations), and the last bit of a sum then decides
+        # where one of them stops.  Against the same solve in another order: h 9e-5, rho 4e-4 apart in
+        # the norm, from one target in some tens of thousands; four times that.
+        return {"rel": 1.6e-3, "max": 1.0 - 1e-9, "differ": 1e-3}
     if kind == "lists":
         return "exact"
     if kind == "direct":
