@@ -10,6 +10,7 @@
 //   FP32: the pair offset is differenced in double and narrowed, everything after it is float
 //         (grav_cuda.cu:108-134 without zeta terms or a periodic wrap).
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <mutex>
 
@@ -24,8 +25,10 @@ static __device__ __align__(256) double g_direct_noalloc_scratch[GT_DIRECT_NOALL
 namespace gt {
 namespace {
 
-constexpr int kDirThreads = 256;
+constexpr int kDirThreads = 128;
+constexpr int kDirPer = 2;  // targets per thread
 constexpr int kDirTile = 256;
+constexpr int kDirUnroll = 4;  // sources per iteration
 
 __device__ __forceinline__ void spline_d(double r, double h, double& f, double& p) {
     const double hinv = 1.0 / h;
@@ -84,8 +87,75 @@ __device__ __forceinline__ double kernel_dwdr_d(double r, double h) {
     return norm * fp / h;
 }
 
-// GAS (FP64 only): the adaptive-softening zeta terms of gas-gas pairs (tree.cc:39-53); type
-// (0 = gas; null = every particle gas) and zeta (null = none) are indexed like the particles.
+// One pair of two particles in double with every case of the pair rule: r = 0, the spline inside the
+// larger softening, the zeta terms of a gas-gas pair.
+// GAS: the adaptive-softening zeta terms of gas-gas pairs (tree.cc:39-53); type (0 = gas; null =
+// every particle gas) and zeta (null = none) are indexed like the particles.
+struct GasTarget {
+    double tzm = 0.0, tm = 0.0, tzeta = 0.0;  // zeta_t / m_t, m_t and zeta_t of a gas target
+    bool gas = false;
+};
+template <bool GAS>
+__device__ __noinline__ void pair_d(double ox, double oy, double oz, double ps, double ss, double m,
+                                    const GasTarget& gt, double szeta, bool sgas, double& mf, double& mp) {
+    mf = mp = 0.0;
+    const double r = sqrt(ox * ox + oy * oy + oz * oz);
+    if (r <= 0) return;
+    const double e = fmax(fmax(ps, ss), 1e-300);
+    double f, p;
+    spline_d(r, e, f, p);
+    mf = m * f;
+    mp = m * p;
+    if (GAS && gt.gas && sgas && gt.tm > 0.0) {
+        const double es = fmax(ss, 1e-300);
+        if (gt.tzeta != 0.0 && r < e) mf -= gt.tzm * kernel_dwdr_d(r, e) / r;
+        if (szeta != 0.0 && r < es) mf -= (szeta / gt.tm) * kernel_dwdr_d(r, es) / r;
+    }
+}
+
+__device__ __noinline__ void pair_f(float dx, float dy, float dz, float ps, float ss, float m, float& mf, float& mp) {
+    mf = mp = 0.0f;
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    if (r2 <= 0.0f) return;
+    float e = fmaxf(ps, ss);
+    if (!(e > 0.0f)) e = 1e-30f;
+    float f, p;
+    spline_f(sqrtf(r2), e, f, p);
+    mf = m * f;
+    mp = m * p;
+}
+
+// The sources of one tile, in the order the inner loop reads them: two 16-byte broadcasts of shared
+// memory give position and mass, a word the limit below which a pair leaves the short path.
+struct alignas(16) DirSrc {
+    double x, y, z, m;
+};
+
+// 1/sqrt(x) of a normal x: the approximate reciprocal square root y, then one step of the binomial
+// series of (1 - e)^(-1/2) about it, y (1 + e/2 + 3/8 e^2) with e = 1 - x y^2.  The approximation's
+// relative error is below 2^-20, so e is below 2^-19 and the term left out, 5/16 e^3, below 2^-58: the
+// result is off by the rounding of the step's few operations (tests/test_gpu_parity.py bounds the
+// direct sum against the oracle).  Five FP64 instructions and no branch, so that the pairs of an
+// iteration overlap; the library function's check for special operands would keep them apart.
+__device__ __forceinline__ double rsqrt_d(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// Direct sum of kDirPer targets per thread over one chunk of the sources.
+//
+// What bounds it: the FP64 pipe (64 lanes a clock per SM).  A pair outside both softenings needs 18
+// FP64 instructions -- 3 differences, 3 for r^2, 5 for the reciprocal square root, 3 products for
+// m / r^3, 3 + 1 accumulations -- and that path holds nothing else in double: whether a pair is
+// outside is an integer comparison of the high words of r^2 and of the larger squared softening.  The
+// high word rounds down, so pairs within one part in 10^6 of the softening, the pair of a particle
+// with itself, r = 0 and every subnormal, infinite or NaN r^2 are left out of it (1/r taken as 0) and taken by pair_d, which treats each case as the rule says, after the iteration's pairs: one
+// branch per kDirUnroll sources and kDirPer targets, rarely taken, instead of one per pair, which
+// kept every pair's chain of dependent instructions to itself.
+//   FP32: the offset is differenced in double and narrowed, the interaction is FP32 with the
+//   approximate reciprocal square root, and each tile's FP32 sums are added into double totals.
 template <bool FP64, bool GAS = false>
 __global__ void __launch_bounds__(kDirThreads)
 direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
@@ -93,83 +163,149 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
               const uint32_t* __restrict__ targets, int64_t nt, int64_t chunk,
               double* __restrict__ partial, const uint8_t* __restrict__ type = nullptr,
               const double* __restrict__ zeta = nullptr) {
-    __shared__ double shx[kDirTile], shy[kDirTile], shz[kDirTile], shm[kDirTile], shs[kDirTile];
+    __shared__ DirSrc sh[kDirTile];
+    __shared__ double shs[kDirTile];
+    __shared__ int shlim[kDirTile];
+    __shared__ float shm[FP64 ? 1 : kDirTile];
     __shared__ double shzeta[GAS ? kDirTile : 1];
     __shared__ unsigned char shgas[GAS ? kDirTile : 1];
-    const int64_t t = (int64_t)blockIdx.x * kDirThreads + threadIdx.x;
-    // a target index at or beyond n (device target arrays are not checked on the host) reads
-    // nothing and sums nothing: its outputs are zero
-    const bool slot = t < nt;
-    const int64_t self = slot ? (int64_t)targets[t] : -1;
-    const bool live = slot && self < n;
-    const double px = live ? x[self] : 0.0, py = live ? y[self] : 0.0, pz = live ? z[self] : 0.0;
-    const double ps = (live && soft) ? soft[self] : 0.0;
-    // a gas target with mass: zeta_t / m_t and 1 / m_t of its pair terms
-    double tzm = 0.0, tm = 0.0, tzeta = 0.0;
-    bool tgas = false;
-    if (GAS && live) {
-        tgas = !type || type[self] == 0;
-        tzeta = zeta ? zeta[self] : 0.0;
-        tm = m[self];
-        if (tm > 0) tzm = tzeta / tm;
+    // high word of the square of a softening: r^2 above it lies outside
+    auto limit = [](double s) {
+        if (FP64) return max(__double2hiint(s * s), 0x000fffff);  // at least every subnormal r^2
+        const float f = (float)s;
+        return __float_as_int(f * f);
+    };
+    const int64_t t0 = (int64_t)blockIdx.x * (kDirThreads * kDirPer) + threadIdx.x;
+    int64_t self[kDirPer];
+    double px[kDirPer], py[kDirPer], pz[kDirPer], ps[kDirPer];
+    int plim[kDirPer];
+    GasTarget gas[GAS ? kDirPer : 1];
+    double ax[kDirPer], ay[kDirPer], az[kDirPer], ap[kDirPer];
+#pragma unroll
+    for (int k = 0; k < kDirPer; ++k) {
+        // a target index at or beyond n (device target arrays are not checked on the host) reads
+        // nothing; its outputs are zero
+        const int64_t t = t0 + k * kDirThreads;
+        self[k] = t < nt ? (int64_t)targets[t] : n;
+        const bool live = self[k] < n;
+        px[k] = live ? x[self[k]] : 0.0;
+        py[k] = live ? y[self[k]] : 0.0;
+        pz[k] = live ? z[self[k]] : 0.0;
+        ps[k] = (live && soft) ? soft[self[k]] : 0.0;
+        plim[k] = limit(ps[k]);
+        ax[k] = ay[k] = az[k] = ap[k] = 0.0;
+        if (GAS && live) {
+            GasTarget& g = gas[GAS ? k : 0];
+            g.gas = !type || type[self[k]] == 0;
+            g.tzeta = zeta ? zeta[self[k]] : 0.0;
+            g.tm = m[self[k]];
+            if (g.tm > 0) g.tzm = g.tzeta / g.tm;
+        }
     }
     const int64_t s0 = (int64_t)blockIdx.y * chunk, s1 = min(n, s0 + chunk);
-    double ax = 0, ay = 0, az = 0, ap = 0;
-    float fx = 0, fy = 0, fz = 0, fp = 0;
     for (int64_t base = s0; base < s1; base += kDirTile) {
-        const int64_t q = base + threadIdx.x;
-        if (q < s1) {
-            shx[threadIdx.x] = x[q]; shy[threadIdx.x] = y[q]; shz[threadIdx.x] = z[q];
-            shm[threadIdx.x] = m[q];
-            shs[threadIdx.x] = soft ? soft[q] : 0.0;
+        for (int q = threadIdx.x; q < kDirTile; q += kDirThreads) {
+            const int64_t j = base + q;
+            if (j >= s1) {
+                shlim[q] = INT_MAX;  // past the chunk: every pair is left out of the short path
+                sh[q] = DirSrc{0.0, 0.0, 0.0, 0.0};
+                if (!FP64) shm[q] = 0.0f;
+                continue;
+            }
+            sh[q] = DirSrc{x[j], y[j], z[j], m[j]};
+            const double s = soft ? soft[j] : 0.0;
+            shs[q] = s;
+            shlim[q] = limit(s);
+            if (!FP64) shm[q] = (float)m[j];
             if (GAS) {
-                shzeta[threadIdx.x] = zeta ? zeta[q] : 0.0;
-                shgas[threadIdx.x] = (!type || type[q] == 0) ? 1 : 0;
+                shzeta[q] = zeta ? zeta[j] : 0.0;
+                shgas[q] = (!type || type[j] == 0) ? 1 : 0;
             }
         }
         __syncthreads();
         const int nq = (int)min((int64_t)kDirTile, s1 - base);
-        if (live) {
-            for (int k = 0; k < nq; ++k) {
-                if (base + k == self) continue;
-                const double ox = shx[k] - px, oy = shy[k] - py, oz = shz[k] - pz;
-                if (FP64) {
-                    const double r = sqrt(ox * ox + oy * oy + oz * oz);
-                    if (r <= 0) continue;
-                    const double e = fmax(fmax(ps, shs[k]), 1e-300);
-                    double f, p;
-                    spline_d(r, e, f, p);
-                    double mf = shm[k] * f;
-                    if (GAS && tgas && shgas[k] && tm > 0.0) {
-                        const double es = fmax(shs[k], 1e-300);
-                        if (tzeta != 0.0 && r < e) mf -= tzm * kernel_dwdr_d(r, e) / r;
-                        if (shzeta[k] != 0.0 && r < es) mf -= (shzeta[k] / tm) * kernel_dwdr_d(r, es) / r;
+        float fx[kDirPer], fy[kDirPer], fz[kDirPer], fp[kDirPer];
+#pragma unroll
+        for (int k = 0; k < kDirPer; ++k) fx[k] = fy[k] = fz[k] = fp[k] = 0.0f;
+        for (int q0 = 0; q0 < nq; q0 += kDirUnroll) {
+            unsigned slow = 0;
+#pragma unroll
+            for (int i = 0; i < kDirUnroll; ++i) {
+                const int q = q0 + i;
+                const DirSrc s = sh[q];
+                const int sl = shlim[q];
+#pragma unroll
+                for (int k = 0; k < kDirPer; ++k) {
+                    const double ox = s.x - px[k], oy = s.y - py[k], oz = s.z - pz[k];
+                    const int lim = max(plim[k], sl);
+                    if (FP64) {
+                        const double r2 = ox * ox + oy * oy + oz * oz;
+                        const int hi = __double2hiint(r2);
+                        const bool ok = hi > lim && hi < 0x7ff00000;
+                        if (!ok) slow |= 1u << (i * kDirPer + k);
+                        const double ri = ok ? rsqrt_d(r2) : 0.0;
+                        const double mri = s.m * ri;
+                        const double mf = mri * (ri * ri);
+                        ax[k] += ox * mf; ay[k] += oy * mf; az[k] += oz * mf;
+                        ap[k] -= mri;
+                    } else {
+                        const float dx = (float)ox, dy = (float)oy, dz = (float)oz;
+                        const float r2 = dx * dx + dy * dy + dz * dz;
+                        const int hi = __float_as_int(r2);
+                        const bool ok = hi > lim && hi < 0x7f800000;
+                        if (!ok) slow |= 1u << (i * kDirPer + k);
+                        const float ri = ok ? rsqrtf(r2) : 0.0f;
+                        const float mri = shm[q] * ri;
+                        const float mf = mri * (ri * ri);
+                        fx[k] += dx * mf; fy[k] += dy * mf; fz[k] += dz * mf;
+                        fp[k] -= mri;
                     }
-                    ax += ox * mf; ay += oy * mf; az += oz * mf;
-                    ap += shm[k] * p;
-                } else {
-                    const float dx = (float)ox, dy = (float)oy, dz = (float)oz;
-                    const float r2 = dx * dx + dy * dy + dz * dz;
-                    if (r2 <= 0.0f) continue;
-                    const float r = sqrtf(r2);
-                    float e = fmaxf((float)ps, (float)shs[k]);
-                    if (!(e > 0.0f)) e = 1e-30f;
-                    float f, p;
-                    spline_f(r, e, f, p);
-                    const float mf = (float)shm[k] * f;
-                    fx += dx * mf; fy += dy * mf; fz += dz * mf;
-                    fp += (float)shm[k] * p;
                 }
+            }
+            if (slow) {
+#pragma unroll 1
+                for (int i = 0; i < kDirUnroll; ++i)
+#pragma unroll
+                    for (int k = 0; k < kDirPer; ++k) {
+                        const int q = q0 + i;
+                        if (!((slow >> (i * kDirPer + k)) & 1u) || q >= nq || base + q == self[k]) continue;
+                        const DirSrc s = sh[q];
+                        const double ox = s.x - px[k], oy = s.y - py[k], oz = s.z - pz[k];
+                        if (FP64) {
+                            double mf, mp;
+                            pair_d<GAS>(ox, oy, oz, ps[k], shs[q], s.m, gas[GAS ? k : 0], GAS ? shzeta[q] : 0.0,
+                                        GAS && shgas[q], mf, mp);
+                            ax[k] += ox * mf; ay[k] += oy * mf; az[k] += oz * mf;
+                            ap[k] += mp;
+                        } else {
+                            const float dx = (float)ox, dy = (float)oy, dz = (float)oz;
+                            float mf, mp;
+                            pair_f(dx, dy, dz, (float)ps[k], (float)shs[q], shm[q], mf, mp);
+                            fx[k] += dx * mf; fy[k] += dy * mf; fz[k] += dz * mf;
+                            fp[k] += mp;
+                        }
+                    }
+            }
+        }
+        if (!FP64) {
+#pragma unroll
+            for (int k = 0; k < kDirPer; ++k) {
+                ax[k] += (double)fx[k]; ay[k] += (double)fy[k]; az[k] += (double)fz[k];
+                ap[k] += (double)fp[k];
             }
         }
         __syncthreads();
     }
-    if (slot) {
+#pragma unroll
+    for (int k = 0; k < kDirPer; ++k) {
+        const int64_t t = t0 + k * kDirThreads;
+        if (t >= nt) continue;
+        const bool live = self[k] < n && n > 1;  // the sum over no other particle is 0, wherever it is
         double* P = partial + (int64_t)blockIdx.y * 4 * nt;
-        P[t] = FP64 ? ax : (double)fx;
-        P[nt + t] = FP64 ? ay : (double)fy;
-        P[2 * nt + t] = FP64 ? az : (double)fz;
-        P[3 * nt + t] = FP64 ? ap : (double)fp;
+        P[t] = live ? ax[k] : 0.0;
+        P[nt + t] = live ? ay[k] : 0.0;
+        P[2 * nt + t] = live ? az[k] : 0.0;
+        P[3 * nt + t] = live ? ap[k] : 0.0;
     }
 }
 
@@ -191,9 +327,9 @@ __global__ void direct_reduce_kernel(const double* __restrict__ partial, int64_t
 // Source chunking: enough chunks that (target blocks x chunks) fills the GPU, at most
 // `max_chunks`.  Returns the chunk length and sets nchunk.
 int64_t plan_chunks(int64_t n, int64_t nt, int num_sms, int64_t max_chunks, int& nchunk) {
-    const int bx = div_up(nt, kDirThreads);
+    const int bx = div_up(nt, kDirThreads * kDirPer);
     int64_t c = std::max(1, div_up((int64_t)num_sms * 4, bx));
-    c = std::min<int64_t>(c, std::max<int64_t>(1, div_up(n, 4 * kDirTile)));
+    c = std::min<int64_t>(c, std::max<int64_t>(1, div_up(n, 2 * kDirTile)));
     c = std::min<int64_t>(c, std::min<int64_t>(65535, std::max<int64_t>(1, max_chunks)));
     const int64_t chunk = std::max<int64_t>(1, div_up(n, c));
     nchunk = std::max(1, div_up(n, chunk));
@@ -204,7 +340,7 @@ void launch_direct(cudaStream_t st, int num_sms, int64_t n, const double* x, con
                    const double* z, const double* m, const double* soft, int64_t nt,
                    const uint32_t* targets, double G, int precision, double* ax, double* ay,
                    double* az, double* phi, double* partial, int nchunk, int64_t chunk) {
-    const dim3 grid(div_up(nt, kDirThreads), nchunk);
+    const dim3 grid(div_up(nt, kDirThreads * kDirPer), nchunk);
     if (precision == GT_DIRECT_FP32)
         direct_kernel<false><<<grid, kDirThreads, 0, st>>>(x, y, z, m, soft, n, targets, nt, chunk, partial);
     else
@@ -222,7 +358,7 @@ void run_direct_gas(gt_context* ctx, int64_t n, const double* x, const double* y
     int nchunk = 1;
     const int64_t chunk = plan_chunks(n, nt, ctx->num_sms, 65535, nchunk);
     double* partial = (double*)scratch(ctx, kSlotDirect, (size_t)nchunk * 4 * nt * 8);
-    const dim3 grid(div_up(nt, kDirThreads), nchunk);
+    const dim3 grid(div_up(nt, kDirThreads * kDirPer), nchunk);
     direct_kernel<true, true><<<grid, kDirThreads, 0, ctx->stream>>>(x, y, z, m, soft, n, targets, nt, chunk, partial,
                                                                      type, zeta);
     direct_reduce_kernel<<<std::max(1, std::min(div_up(nt, 256), ctx->num_sms * 4)), 256, 0, ctx->stream>>>(

@@ -330,6 +330,39 @@ def test_direct_fp64_and_fp32(gpu_ctx, oracle, plummer):
     assert np.median(e) <= 1e-5 and e.max() <= 1e-3
 
 
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 255, 256, 257, 1023, 3001])
+@pytest.mark.parametrize("soft", [None, 0.0, 0.3])
+def test_direct_edges_of_tiles(gpu_ctx, oracle, n, soft):
+    """Sizes around the source tile (256), the sources per iteration (4) and the targets per block
+    (256), with a coincident pair, a close pair (1e-160 apart: r^2 below the FP64 range) and, at 0.3,
+    most pairs inside the kernel.  FP64 to 1e-12 of the larger of the sum and its terms' absolute
+    sum: n terms of at most a few roundings (1e-16) each.  FP32 to 1e-5 of that sum: a term is off by
+    about ten roundings of 6e-8."""
+    P = ics.plummer(n=n, seed=n + 5)
+    P["soft"] = None if soft is None else np.full(n, soft)
+    if n > 4:
+        for k in ("x", "y", "z"):
+            P[k][3] = P[k][1]
+    if n > 2:
+        P["x"][2], P["y"][2], P["z"][2] = 0.0, 0.0, 0.0
+        P["x"][0], P["y"][0], P["z"][0] = (1e-160, 0.0, 0.0) if soft else (1e-3, 0.0, 0.0)
+    tg = np.arange(n, dtype=np.uint32)[::-1].copy()
+    O = dict(P, soft=np.zeros(n) if P["soft"] is None else P["soft"])
+    ox, oy, oz, op = oracle.direct(O, tg)
+    d = np.sqrt(sum((P[k][None, :] - P[k][tg][:, None]) ** 2 for k in ("x", "y", "z")))
+    e = np.maximum(d, 1e-300 if not soft else soft / 4)
+    with np.errstate(over="ignore", divide="ignore", invalid="ignore"):
+        scale = np.where(d > 0, P["m"][None, :] * np.minimum(d / e ** 3, 1.0 / e ** 2), 0.0).sum(1)
+        pscale = np.where(d > 0, P["m"][None, :] * 2.8 / np.maximum(e, soft or 0.0), 0.0).sum(1)
+    for prec, tol in ((g.GT_DIRECT_FP64, 1e-12), (g.GT_DIRECT_FP32, 1e-5)):
+        ax, ay, az, phi = gpu_ctx.direct(P, tg, precision=prec)
+        err = np.sqrt((ax - ox) ** 2 + (ay - oy) ** 2 + (az - oz) ** 2)
+        assert (err <= tol * scale).all()
+        # FP32 narrows the offset of the close pair to 0, and so skips the pair and its potential
+        seen = (prec == g.GT_DIRECT_FP64) | ~np.isin(tg, [0, 2])
+        assert (np.abs(phi - op) <= tol * pscale)[seen].all()
+
+
 # ---- edge cases -----------------------------------------------------------------------------
 
 def test_empty_single_and_pair(gpu_ctx, oracle):
