@@ -109,29 +109,111 @@ struct NgbTally {
     unsigned long long nodes = 0, examined = 0, pad = 0;
 };
 
+// The particles [s, e) of one opened leaf against a centre: FP64 |d|^2 as x*x + y*y + z*z without
+// contraction (Vec3d::norm_sq).  True when particle s (index j in the input) is a neighbour.
+template <bool REVERSE>
+__device__ __forceinline__ bool is_neighbour(const SearchGeom& g, int s, double px, double py, double pz,
+                                             double r2max, const double* __restrict__ h, int64_t n_gas, uint32_t& j) {
+    const double2 xy = __ldg(reinterpret_cast<const double2*>(g.src + s));
+    const double zz = __ldg(reinterpret_cast<const double*>(g.src + s) + 2);
+    const double ox = min_image(xy.x - px, g.box), oy = min_image(xy.y - py, g.box), oz = min_image(zz - pz, g.box);
+    const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(ox, ox), __dmul_rn(oy, oy)), __dmul_rn(oz, oz));
+    if (!REVERSE) return r2 < r2max;
+    if (r2 < r2max) return false;
+    j = __ldg(g.order + s);
+    if ((int64_t)j >= n_gas) return false;
+    const double hj = __ldg(h + j);
+    return r2 >= r2max && r2 < hj * hj;
+}
+
 // One traversal for one centre in the reference's node order, from roots r0 .. r1-1 in turn.
 // REVERSE: gas particles j < n_gas with radius <= r < h[j] (ngb_search_reverse); otherwise
-// r < radius (ngb_search).  emit(j, s) receives the particle index and its tree position.  COUNT
-// (gather only, as the reference counts): the tally.
-template <bool REVERSE, bool COUNT = false, typename F>
+// r < radius (ngb_search).  emit(s) receives the tree position; false ends the search.
+//
+// A thread follows the threading alone, so what bounds the search is how many of a warp's lanes do
+// the same thing at once.  Opening each leaf where the traversal meets it kept 5.5 of 32 lanes
+// active: the lanes reach their leaves at different steps, and every leaf held up the whole warp.
+// Here the traversal only notes the leaves it opens (kLeafBuf of them, in thread-local memory, which
+// the hardware interleaves across the warp); then every lane runs through the particles of its own
+// leaves in one flat loop, a particle an iteration, and the traversal goes on.  Both loops keep
+// nearly all lanes busy, because neighbouring targets visit nearly as many nodes and particles.
+// The prune is the reference's box and circumsphere test in FP32, widened by the rounding of the
+// centre, the distances and the squares, so it never drops a node that the FP64 test keeps; the
+// particle test decides in FP64, so the lists are the same, in the same order.
+constexpr int kLeafBuf = 32;
+template <bool REVERSE, typename F>
 __device__ __forceinline__ void search(const SearchGeom& g, int r0, int r1, double px, double py, double pz,
-                                       double radius, const double* __restrict__ h, int64_t n_gas, F&& emit,
-                                       NgbTally* tally = nullptr) {
+                                       double radius, const double* __restrict__ h, int64_t n_gas, F&& emit) {
+    const double r2max = radius * radius;
+    const float fx = (float)px, fy = (float)py, fz = (float)pz;
+    const float fbox = (float)g.box, fhalf = 0.5f * fbox;
+    // the rounding of fx, fy, fz, of the differences and of the minimum image, four times over
+    const float slack = 8.0f * FLT_EPSILON * (fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) + fbox);
+    const float reach = REVERSE ? slack : __fadd_ru(__double2float_ru(radius), slack);
+    const float felapsed = g.elapsed > 0 ? __double2float_ru(g.elapsed) : 0.0f;
+    const bool moving = g.elapsed > 0 && g.vmax;
+    auto image = [&](float s) {
+        if (fbox > 0.0f) {
+            if (s > fhalf) s -= fbox;
+            else if (s < -fhalf) s += fbox;
+        }
+        return s;
+    };
+    int2 leaf[kLeafBuf];
+    for (int root = r0; root < r1; ++root) {
+        int node = root;
+        while (node >= 0) {
+            int nl = 0;
+            while (node >= 0 && nl < kLeafBuf) {
+                const float4 a = __ldg(reinterpret_cast<const float4*>(g.sn + node));
+                const int4 b = __ldg(reinterpret_cast<const int4*>(g.sn + node) + 1);
+                float dist = reach + a.w;
+                bool keep = true;
+                if (REVERSE) {
+                    const float hm = __ldg(g.hmax + node);
+                    keep = !((double)hm <= radius);
+                    dist += hm;
+                }
+                if (g.xpad) dist += __ldg(g.xpad + node);
+                if (moving) dist = fmaf(__ldg(g.vmax + node), felapsed, dist);
+                dist *= 1.000002f;
+                const float dx = image(a.x - fx), dy = image(a.y - fy), dz = image(a.z - fz);
+                const float ball = fmaf(0.73205090f, a.w, dist) * 1.000002f;
+                keep = keep && !(fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz))) > dist) &&
+                       !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > ball * ball);
+                if (keep && b.x < 0) leaf[nl++] = make_int2(b.z, b.w);
+                node = keep && b.x >= 0 ? b.x : b.y;
+            }
+            int s = 0, e = 0, li = 0;
+            for (;;) {
+                while (s >= e && li < nl) {
+                    s = leaf[li].x;
+                    e = leaf[li].y;
+                    ++li;
+                }
+                if (s >= e) break;
+                uint32_t j = 0;
+                if (is_neighbour<REVERSE>(g, s, px, py, pz, r2max, h, n_gas, j) && !emit(s)) return;
+                ++s;
+            }
+        }
+    }
+}
+
+// The gather search as the reference counts it (SHMEM_NGB_COUNT): its own FP64 prune, node by node,
+// so that the nodes visited and the pads that admitted them are the reference's.  The lists are
+// search()'s.
+template <typename F>
+__device__ __forceinline__ void search_counted(const SearchGeom& g, int r0, int r1, double px, double py, double pz,
+                                               double radius, F&& emit, NgbTally* tally) {
     const double r2max = radius * radius;
     for (int root = r0; root < r1; ++root)
     for (int node = root; node >= 0;) {
-        if (COUNT) ++tally->nodes;
+        ++tally->nodes;
         const float4 a = __ldg(reinterpret_cast<const float4*>(g.sn + node));
         const int4 b = __ldg(reinterpret_cast<const int4*>(g.sn + node) + 1);
         const double half = (double)a.w;
-        double dist;
-        if (REVERSE) {
-            const double hm = (double)__ldg(g.hmax + node);
-            if (hm <= radius) { node = b.y; continue; }
-            dist = hm + half;
-        } else {
-            dist = radius + half;
-        }
+        double dist = radius + half;
         if (g.xpad) dist += (double)__ldg(g.xpad + node);
         if (g.elapsed > 0 && g.vmax) dist += (double)__ldg(g.vmax + node) * g.elapsed;
         const double dx = min_image((double)a.x - px, g.box);
@@ -142,30 +224,15 @@ __device__ __forceinline__ void search(const SearchGeom& g, int r0, int r1, doub
         if (dz > dist || -dz > dist) { node = b.y; continue; }
         dist += 0.7320508075688772 * half;
         if (dx * dx + dy * dy + dz * dz > dist * dist) { node = b.y; continue; }
-        if (COUNT && g.elapsed > 0) {
+        if (g.elapsed > 0) {
             const double nopad = radius + 1.7320508075688772 * half;
             if (dx * dx + dy * dy + dz * dz > nopad * nopad) ++tally->pad;
         }
         if (b.x < 0) {
-            if (COUNT) tally->examined += (unsigned long long)(b.w - b.z);
-            for (int s = b.z; s < b.w; ++s) {
-                const uint32_t j = __ldg(g.order + s);
-                if (REVERSE && (int64_t)j >= n_gas) continue;
-                const double2 xy = __ldg(reinterpret_cast<const double2*>(g.src + s));
-                const double zz = __ldg(reinterpret_cast<const double*>(g.src + s) + 2);
-                const double ox = min_image(xy.x - px, g.box), oy = min_image(xy.y - py, g.box),
-                             oz = min_image(zz - pz, g.box);
-                // |d|^2 as x*x + y*y + z*z without contraction (Vec3d::norm_sq)
-                const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(ox, ox), __dmul_rn(oy, oy)), __dmul_rn(oz, oz));
-                bool keep;
-                if (REVERSE) {
-                    const double hj = __ldg(h + j);
-                    keep = r2 >= r2max && r2 < hj * hj;
-                } else {
-                    keep = r2 < r2max;
-                }
-                if (keep) emit(j, s);
-            }
+            tally->examined += (unsigned long long)(b.w - b.z);
+            uint32_t j = 0;
+            for (int s = b.z; s < b.w; ++s)
+                if (is_neighbour<false>(g, s, px, py, pz, r2max, nullptr, 0, j)) emit(s);
             node = b.y;
         } else {
             node = b.x;
@@ -227,13 +294,15 @@ __global__ void __launch_bounds__(kBlk) ngb_kernel(const NgbArgs a) {
         roots_of(a.g, a.systems, c, r0, r1, FILL ? nullptr : a.total + 1);
         if (FILL && a.kcache > 0 && a.count[c] <= (uint32_t)a.kcache) continue;  // copied from the cache
         int64_t k = FILL ? a.start[c] : 0;
-        auto emit = [&](uint32_t j, int) {
-            if (FILL) a.found[k] = j;
-            else if (k < a.kcache) a.cache[k * a.n + c] = j;
+        auto emit = [&](int s) {
+            if (FILL) a.found[k] = __ldg(a.g.order + s);
+            else if (k < a.kcache) a.cache[k * a.n + c] = __ldg(a.g.order + s);
             ++k;
+            return true;
         };
         if (a.mode != GT_NGB_REVERSE) {
-            search<false, COUNT>(a.g, r0, r1, px, py, pz, r, nullptr, 0, emit, &tl);
+            if (COUNT) search_counted(a.g, r0, r1, px, py, pz, r, emit, &tl);
+            else search<false>(a.g, r0, r1, px, py, pz, r, nullptr, 0, emit);
             if (COUNT) {
                 ++calls;
                 kept += (unsigned long long)k;
@@ -316,7 +385,20 @@ struct DensArgs {
     uint32_t* cand;
     int cand_cap;
     int64_t n_threads;
+    int run;  // targets a warp takes at a time
+    // targets with more candidates than a thread's cache holds, finished by a warp each:
+    // heavy_ctr[0] the targets handed over, [1] the next one to take, [2] the next target of density_kernel
+    struct DensHeavy* heavy;
+    int heavy_cap;
+    unsigned int* heavy_ctr;
+    uint32_t* warp_cand;  // kWarpCand tree positions per warp
 };
+// A target's solve at the evaluation that found too many candidates.
+struct DensHeavy {
+    double h, h_lo, h_hi;
+    int t, iter;
+};
+constexpr int kHeavyCap = 1 << 18;  // 8 MB; a target beyond it is finished by its own thread
 
 __device__ __forceinline__ void dens_zero(DensSums& s) {
     s.wsum = s.dwdh = s.rho = 0.0;
@@ -325,33 +407,54 @@ __device__ __forceinline__ void dens_zero(DensSums& s) {
     s.inside = 0;
 }
 
-// One gas neighbour at offset (dx, dy, dz) from the target, inside h: its kernel weight and the
-// sums the solve reads (hydro.cc:209-222).
-__device__ __forceinline__ void dens_add(double dx, double dy, double dz, double m, double h, double norm, int dim,
-                                         DensSums& s) {
-    const double r = sqrt(dx * dx + dy * dy + dz * dz);
-    const double q = r / h;
-    double w = 0.0, dh = 0.0;
+// One gas neighbour's terms at offset (dx, dy, dz) from the target (hydro.cc:209-222): its kernel
+// weight w and dW/dh.  Every rounding is spelled out, so that the solve's forms -- a thread per target
+// and a warp per target -- add the same terms in the same order and agree to the last bit.
+struct DensNorm {
+    double h, norm, dnorm;  // dnorm: -dim / h of the kernel's norm
+};
+__device__ __forceinline__ DensNorm dens_norm(double h, int dim) {
+    const double norm = kernel_norm(h, dim);
+    return DensNorm{h, norm, __dmul_rn(-((double)dim / h), norm)};
+}
+__device__ __forceinline__ void dens_terms(double dx, double dy, double dz, const DensNorm& n, double& w, double& dh,
+                                           bool& inside) {
+    const double r = sqrt(__fma_rn(dz, dz, __fma_rn(dx, dx, __dmul_rn(dy, dy))));
+    const double q = r / n.h;
+    w = dh = 0.0;
     if (q < 1.0) {
-        double f, fp;
+        double f, fp;  // the spline and its derivative
         if (q < 0.5) {
-            f = 1.0 - 6.0 * q * q + 6.0 * q * q * q;
-            fp = -12.0 * q + 18.0 * q * q;
+            const double q6 = __dmul_rn(6.0, q), q66 = __dmul_rn(q6, q);
+            f = __fma_rn(q66, q, __dadd_rn(1.0, -q66));
+            fp = __fma_rn(__dmul_rn(18.0, q), q, __dmul_rn(-12.0, q));
         } else {
-            const double u = 1.0 - q;
-            f = 2.0 * u * u * u;
-            fp = -6.0 * u * u;
+            const double u = __dadd_rn(1.0, -q);
+            f = __dmul_rn(__dmul_rn(__dmul_rn(2.0, u), u), u);
+            fp = __dmul_rn(__dmul_rn(-6.0, u), u);
         }
-        w = norm * f;
-        dh = -((double)dim / h) * norm * f - (q / h) * norm * fp;
+        w = __dmul_rn(n.norm, f);
+        dh = __fma_rn(-__dmul_rn(q / n.h, n.norm), fp, __dmul_rn(n.dnorm, f));
     }
-    s.wsum += w;
-    s.dwdh += dh;
-    s.rho += m * w;
-    s.mom[0] += dx * dx * w; s.mom[1] += dy * dy * w; s.mom[2] += dz * dz * w;
-    s.mom[3] += dx * dy * w; s.mom[4] += dy * dz * w; s.mom[5] += dx * dz * w;
-    s.face[0] += dx * w; s.face[1] += dy * w; s.face[2] += dz * w;
-    if (r < h) ++s.inside;
+    inside = r < n.h;
+}
+__device__ __forceinline__ void dens_add(double dx, double dy, double dz, double m, const DensNorm& n, DensSums& s) {
+    double w, dh;
+    bool inside;
+    dens_terms(dx, dy, dz, n, w, dh, inside);
+    s.wsum = __dadd_rn(s.wsum, w);
+    s.dwdh = __dadd_rn(s.dwdh, dh);
+    s.rho = __fma_rn(m, w, s.rho);
+    s.mom[0] = __fma_rn(__dmul_rn(dx, dx), w, s.mom[0]);
+    s.mom[1] = __fma_rn(__dmul_rn(dy, dy), w, s.mom[1]);
+    s.mom[2] = __fma_rn(__dmul_rn(dz, dz), w, s.mom[2]);
+    s.mom[3] = __fma_rn(__dmul_rn(dx, dy), w, s.mom[3]);
+    s.mom[4] = __fma_rn(__dmul_rn(dy, dz), w, s.mom[4]);
+    s.mom[5] = __fma_rn(__dmul_rn(dx, dz), w, s.mom[5]);
+    s.face[0] = __fma_rn(dx, w, s.face[0]);
+    s.face[1] = __fma_rn(dy, w, s.face[1]);
+    s.face[2] = __fma_rn(dz, w, s.face[2]);
+    if (inside) ++s.inside;
 }
 
 // One evaluation at h: the sums over the GAS neighbours inside h, in tree order (hydro.cc:205-222).
@@ -366,11 +469,10 @@ constexpr double kCacheFirst = 1.1;
 constexpr double kCacheGrow = 1.4;
 
 template <bool COUNT>
-__device__ void dens_eval(const DensArgs& a, int r0, int r1, double px, double py, double pz, double h, DensSums& s,
+__device__ __noinline__ void dens_eval(const DensArgs& a, int r0, int r1, double px, double py, double pz, double h, DensSums& s,
                           NgbTally& tl, unsigned long long& kept) {
     dens_zero(s);
-    const int dim = a.n_dims;
-    const double norm = kernel_norm(h, dim);
+    const DensNorm nrm = dens_norm(h, a.n_dims);
     int buf[kDensBuf];
     int nb = 0;
     auto drain = [&]() {
@@ -380,15 +482,18 @@ __device__ void dens_eval(const DensArgs& a, int r0, int r1, double px, double p
             const double2 xy = __ldg(reinterpret_cast<const double2*>(a.g.src + sp));
             const double zz = __ldg(reinterpret_cast<const double*>(a.g.src + sp) + 2);
             dens_add(min_image(xy.x - px, a.g.box), min_image(xy.y - py, a.g.box), min_image(zz - pz, a.g.box),
-                     __ldg(a.smass + sp), h, norm, dim, s);
+                     __ldg(a.smass + sp), nrm, s);
         }
         nb = 0;
     };
-    search<false, COUNT>(a.g, r0, r1, px, py, pz, h, nullptr, 0, [&](uint32_t, int sp) {
+    auto found = [&](int sp) {
         if (COUNT) ++kept;
         if (nb == kDensBuf) drain();
         buf[nb++] = sp;
-    }, &tl);
+        return true;
+    };
+    if (COUNT) search_counted(a.g, r0, r1, px, py, pz, h, found, &tl);
+    else search<false>(a.g, r0, r1, px, py, pz, h, nullptr, 0, found);
     drain();
 }
 
@@ -398,25 +503,23 @@ __device__ void dens_eval(const DensArgs& a, int r0, int r1, double px, double p
 // r^2 expression.  That is the set a search at h would keep, in the same order (a larger radius
 // only adds particles between them: the order is the threading's), so the sums are bit-identical,
 // and an iteration that shrinks h costs a scan of a few dozen candidates instead of a traversal.
-// A search that finds more than cand_cap gas particles leaves the cache empty.
+// A search that finds more than cand_cap gas particles ends there and returns -1.
 __device__ __forceinline__ int cache_fill(const DensArgs& a, int r0, int r1, double px, double py, double pz,
                                           double R, uint32_t* __restrict__ slot, int64_t stride) {
     int k = 0;
     const int cap = a.cand_cap;
-    NgbTally none;
-    search<false>(a.g, r0, r1, px, py, pz, R, nullptr, 0, [&](uint32_t, int sp) {
-        if (a.stype && __ldg(a.stype + sp) != 0) return;
+    search<false>(a.g, r0, r1, px, py, pz, R, nullptr, 0, [&](int sp) {
+        if (a.stype && __ldg(a.stype + sp) != 0) return true;
         if (k < cap) slot[(int64_t)k * stride] = (uint32_t)sp;
-        ++k;
-    }, &none);
+        return ++k <= cap;
+    });
     return k <= cap ? k : -1;
 }
 
-__device__ void cache_eval(const DensArgs& a, const uint32_t* __restrict__ slot, int64_t stride, int n, double px,
-                           double py, double pz, double h, DensSums& s) {
+__device__ __forceinline__ void cache_eval(const DensArgs& a, const uint32_t* __restrict__ slot, int64_t stride, int n,
+                                           double px, double py, double pz, double h, DensSums& s) {
     dens_zero(s);
-    const int dim = a.n_dims;
-    const double norm = kernel_norm(h, dim);
+    const DensNorm nrm = dens_norm(h, a.n_dims);
     const double r2max = h * h;
     for (int k = 0; k < n; ++k) {
         const int sp = (int)slot[(int64_t)k * stride];
@@ -425,7 +528,7 @@ __device__ void cache_eval(const DensArgs& a, const uint32_t* __restrict__ slot,
         const double ox = min_image(xy.x - px, a.g.box), oy = min_image(xy.y - py, a.g.box),
                      oz = min_image(zz - pz, a.g.box);
         const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(ox, ox), __dmul_rn(oy, oy)), __dmul_rn(oz, oz));
-        if (r2 < r2max) dens_add(ox, oy, oz, __ldg(a.smass + sp), h, norm, dim, s);
+        if (r2 < r2max) dens_add(ox, oy, oz, __ldg(a.smass + sp), nrm, s);
     }
 }
 
@@ -465,7 +568,8 @@ struct NewtonParams {
     int n_dims, face_corr;
 };
 
-__device__ __forceinline__ bool dens_newton(const NewtonParams a, uint32_t p, const DensSums& s, int iter, double& h,
+// Not inlined: one compiled copy, so that every form of the solve takes the same steps to the last bit.
+__device__ __noinline__ bool dens_newton(const NewtonParams a, uint32_t p, const DensSums& s, int iter, double& h,
                                          double& h_lo, double& h_hi) {
     const int dim = a.n_dims;
     const double n_eff = ball_vol(h, dim) * s.wsum;
@@ -513,22 +617,19 @@ __device__ __forceinline__ NewtonParams newton_params(const DensArgs& a) {
     return NewtonParams{a.des_ngb, a.ngb_tol, a.cond_prev, a.n_dims, a.face_corr};
 }
 
-// One thread per target: up to 100 iterations of evaluation and Newton step, then, when the solve
-// did not converge, one more evaluation at the final h (hydro.cc:189-297).  In a forest the target
-// searches the system that owns its particle index.  COUNT: every evaluation is one gather search
-// of the tally, and the target's iterations go to the histogram (hydro.cc:293-296).  ONE_ROOT: a
-// single-system tree with nodes, whose one root (node 0) the compiler then knows, which keeps the
-// traversal's registers those of a plain tree walk.
-template <bool COUNT, bool ONE_ROOT>
-__global__ void __launch_bounds__(kBlk, 6) density_kernel(const DensArgs a) {
+// The counting solve, one thread per target: up to 100 iterations of evaluation and Newton step, then,
+// when the solve did not converge, one more evaluation at the final h (hydro.cc:189-297).  Every
+// evaluation is one gather search of the tally, and the target's iterations go to the histogram
+// (hydro.cc:293-296).  In a forest the target searches the system that owns its particle index.
+__global__ void __launch_bounds__(kBlk, 6) density_count_kernel(const DensArgs a) {
     NgbTally tl;
     unsigned long long calls = 0, kept = 0, hist[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.nt; t += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t p = a.targets[t];
         const uint32_t sp = a.rank[p];
         const double px = a.g.src[sp].x, py = a.g.src[sp].y, pz = a.g.src[sp].z;
-        int r0 = 0, r1 = ONE_ROOT ? 1 : a.g.n_roots;
-        if (!ONE_ROOT && a.g.in_off) {
+        int r0 = 0, r1 = a.g.n_roots;
+        if (a.g.in_off) {
             r0 = system_of(a.g.in_off, a.g.n_systems, (int64_t)p);
             r1 = r0 + 1;
         }
@@ -537,44 +638,279 @@ __global__ void __launch_bounds__(kBlk, 6) density_kernel(const DensArgs a) {
         int iter = 0;
         bool converged = false;
         DensSums s;
-        // the candidate cache (not for the counting variant, whose tallies are per search):
-        // filled at the first h, refilled at kCacheGrow times h when h outgrows it
-        uint32_t* slot = a.cand ? a.cand + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) : nullptr;
-        double R = -1.0;   // radius of the cached search; < 0: nothing cached
-        int ncand = 0;
-        bool cache_ok = !COUNT && a.cand != nullptr;
-        auto evaluate = [&](double hh) {
-            if (cache_ok && !(R >= hh)) {
-                const double rad = (R < 0 ? kCacheFirst : kCacheGrow) * hh;
-                ncand = cache_fill(a, r0, r1, px, py, pz, rad, slot, a.n_threads);
-                if (ncand < 0) cache_ok = false;  // too many candidates: search directly from now on
-                else R = rad;
-            }
-            if (cache_ok) cache_eval(a, slot, a.n_threads, ncand, px, py, pz, hh, s);
-            else dens_eval<COUNT>(a, r0, r1, px, py, pz, hh, s, tl, kept);
-        };
         for (; iter < 100; ++iter) {
-            evaluate(h);
-            if (COUNT) ++calls;
+            dens_eval<true>(a, r0, r1, px, py, pz, h, s, tl, kept);
+            ++calls;
             if (dens_newton(newton_params(a), p, s, iter, h, h_lo, h_hi)) { converged = true; break; }
         }
         if (!converged) {  // rho of the final h (hydro.cc:281-293)
-            evaluate(h);
-            if (COUNT) ++calls;
+            dens_eval<true>(a, r0, r1, px, py, pz, h, s, tl, kept);
+            ++calls;
         }
-        if (COUNT) ++hist[min(converged ? iter + 1 : 100, 8) - 1];
+        ++hist[min(converged ? iter + 1 : 100, 8) - 1];
         a.h[t] = h;
         a.rho[t] = s.rho;
         a.nngb[t] = s.inside;
         a.iters[t] = iter;
     }
-    if (COUNT) {
-        warp_flush(calls, a.tally + 0);
-        warp_flush(tl.nodes, a.tally + 1);
-        warp_flush(tl.examined, a.tally + 2);
-        warp_flush(kept, a.tally + 3);
-        warp_flush(tl.pad, a.tally + 4);
-        for (int k = 0; k < 8; ++k) warp_flush(hist[k], a.tally + 5 + k);
+    warp_flush(calls, a.tally + 0);
+    warp_flush(tl.nodes, a.tally + 1);
+    warp_flush(tl.examined, a.tally + 2);
+    warp_flush(kept, a.tally + 3);
+    warp_flush(tl.pad, a.tally + 4);
+    for (int k = 0; k < 8; ++k) warp_flush(hist[k], a.tally + 5 + k);
+}
+
+// The solve: a lane per target, refilled as targets finish.
+//
+// The targets of a warp take between 1 and 10 iterations, three on average, so with a target per
+// thread for good most lanes waited for the slowest: 6 of 32 were active.  Here a warp takes kRun
+// consecutive targets at a time and its lanes are a pool: a lane whose target is done takes the next
+// one.  The loop's two phases each run for as many lanes at once as can be gathered: the search that
+// fills a lane's candidate cache (a new target, or an h that outgrew the cache) waits until
+// kGather lanes want it or nobody can do anything else, and an evaluation with its Newton step runs
+// for every lane that holds candidates.  Each target's own sequence of searches, sums and steps is
+// that of the counting solve's thread, so its results are the same bits whichever lane it gets.
+// ONE_ROOT: a single-system tree, whose one root (node 0) the compiler then knows.
+constexpr int kGather = 16;
+template <bool ONE_ROOT>
+__global__ void __launch_bounds__(kBlk, 6) density_kernel(const DensArgs a) {
+    const int lane = threadIdx.x & 31;
+    uint32_t* __restrict__ slot = a.cand + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    unsigned next = 0, end = 0;  // the warp's run of targets still to take
+    bool more = true;            // targets are left beyond it
+    int t = -1, iter = 0, ncand = 0, r0 = 0, r1 = 1;
+    bool direct = false;         // too many candidates and no room to hand over: search at every evaluation
+    bool ready_now = false;      // searched for this h (also where h is not a number), or direct
+    double px = 0, py = 0, pz = 0, h = 0, h_lo = 0, h_hi = 0, R = -1.0;
+    for (;;) {
+        // idle lanes take targets
+        const unsigned idle = __ballot_sync(0xffffffffu, t < 0);
+        if (__popc(idle) >= kGather && (more || next < end)) {
+            if (next >= end) {
+                if (lane == 0) next = atomicAdd(a.heavy_ctr + 2, (unsigned)a.run);
+                next = __shfl_sync(0xffffffffu, next, 0);
+                end = (unsigned)min((int64_t)next + a.run, a.nt);
+                more = (int64_t)next + a.run < a.nt;
+            }
+            const unsigned mine = next + __popc(idle & ((1u << lane) - 1u));
+            if (t < 0 && mine < end) {
+                t = (int)mine;
+                const uint32_t p = a.targets[t];
+                const uint32_t sp = a.rank[p];
+                px = a.g.src[sp].x; py = a.g.src[sp].y; pz = a.g.src[sp].z;
+                if (!ONE_ROOT) {
+                    r1 = a.g.n_roots;
+                    if (a.g.in_off) {
+                        r0 = system_of(a.g.in_off, a.g.n_systems, (int64_t)p);
+                        r1 = r0 + 1;
+                    }
+                }
+                h = a.h_start ? a.h_start[t] : (a.h_default_sys ? a.h_default_sys[r0] : a.h_default);
+                h_lo = h_hi = 0.0;
+                R = -1.0;
+                iter = 0;
+                direct = ready_now = false;
+            }
+            next = min(end, next + (unsigned)__popc(idle));
+            continue;
+        }
+        const bool have = t >= 0, want = have && !ready_now && !(R >= h);
+        const unsigned wants = __ballot_sync(0xffffffffu, want), ready = __ballot_sync(0xffffffffu, have && !want);
+        if ((wants | ready) == 0u) break;
+        if (__popc(wants) >= kGather || ready == 0u) {
+            if (want) {
+                const double rad = (R < 0 ? kCacheFirst : kCacheGrow) * h;
+                ncand = cache_fill(a, r0, r1, px, py, pz, rad, slot, a.n_threads);
+                R = rad;
+                ready_now = true;
+                if (ncand < 0) {
+                    // more candidates than the cache holds: to a warp of density_heavy_kernel
+                    const unsigned at = atomicAdd(a.heavy_ctr, 1u);
+                    if (at < (unsigned)a.heavy_cap) {
+                        a.heavy[at] = DensHeavy{h, h_lo, h_hi, t, iter};
+                        t = -1;
+                    } else {
+                        direct = true;
+                    }
+                }
+            }
+            __syncwarp();
+            continue;
+        }
+        if (have && !want) {
+            DensSums s;
+            if (direct) {
+                NgbTally none;
+                unsigned long long kept = 0;
+                dens_eval<false>(a, r0, r1, px, py, pz, h, s, none, kept);
+            } else {
+                cache_eval(a, slot, a.n_threads, ncand, px, py, pz, h, s);
+            }
+            // after 100 steps, the sums of the final h (hydro.cc:281-293)
+            if (iter == 100 || dens_newton(newton_params(a), a.targets[t], s, iter, h, h_lo, h_hi)) {
+                a.h[t] = h;
+                a.rho[t] = s.rho;
+                a.nngb[t] = s.inside;
+                a.iters[t] = iter;
+                t = -1;
+            } else {
+                ++iter;
+                ready_now = direct;
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// The targets that a thread handed over, a warp each.  A Newton step from a poor guess can ask for an
+// h that holds tens of thousands of neighbours; in one thread such an evaluation took 28 ms, the time
+// of the whole solve of 86,000 targets.  Here the lanes test 32 consecutive particles at a time and
+// compute their terms, and twelve lanes, one per sum, add the 32 terms in order from shared memory:
+// the sums are those of the thread's loop to the last bit.  The traversal is the thread's, in all
+// lanes alike, and stops at nodes of up to kWarpLeaf particles, whose consecutive range is tested
+// whole: the particle test alone decides, so the neighbours and their order are the same.
+constexpr int kHeavyWarps = 4;
+constexpr int kWarpLeaf = 64;
+constexpr int kWarpCand = 2048;  // cached candidates per warp; a larger search is repeated instead
+
+// The particles within `radius` in tree order, 32 at a time: use(s, keep) in every lane.
+template <typename F>
+__device__ __forceinline__ void warp_search(const SearchGeom& g, int r0, int r1, double px, double py, double pz,
+                                            double radius, F&& use) {
+    const int lane = threadIdx.x & 31;
+    const double r2max = radius * radius;
+    for (int root = r0; root < r1; ++root)
+        for (int node = root; node >= 0;) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(g.sn + node));
+            const int4 b = __ldg(reinterpret_cast<const int4*>(g.sn + node) + 1);
+            double dist = radius + (double)a.w;
+            if (g.xpad) dist += (double)__ldg(g.xpad + node);
+            if (g.elapsed > 0 && g.vmax) dist += (double)__ldg(g.vmax + node) * g.elapsed;
+            const double dx = min_image((double)a.x - px, g.box), dy = min_image((double)a.y - py, g.box),
+                         dz = min_image((double)a.z - pz, g.box);
+            const double ball = dist + 0.7320508075688772 * (double)a.w;
+            if (fabs(dx) > dist || fabs(dy) > dist || fabs(dz) > dist || dx * dx + dy * dy + dz * dz > ball * ball) {
+                node = b.y;
+            } else if (b.x < 0 || b.w - b.z <= kWarpLeaf) {
+                for (int s0 = b.z; s0 < b.w; s0 += 32) {
+                    const int s = s0 + lane;
+                    uint32_t j = 0;
+                    const bool keep = s < b.w && is_neighbour<false>(g, s, px, py, pz, r2max, nullptr, 0, j);
+                    use(s, keep);
+                }
+                node = b.y;
+            } else {
+                node = b.x;
+            }
+        }
+}
+
+__global__ void __launch_bounds__(kHeavyWarps * 32) density_heavy_kernel(const DensArgs a) {
+    // terms of 32 particles: the factors of each sum's fused multiply-add
+    __shared__ double term[kHeavyWarps][12][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double(*T)[32] = term[w];
+    uint32_t* __restrict__ list = a.warp_cand + (int64_t)(blockIdx.x * kHeavyWarps + w) * kWarpCand;
+    const unsigned n_heavy = min(a.heavy_ctr[0], (unsigned)a.heavy_cap);
+    // lane c < 12 keeps sum c = sum of T[fa] * T[fb] (wsum and dwdh: of T[fb])
+    const int fb = lane == 1 ? 1 : 0, fa = lane == 2 ? 2 : lane < 9 ? lane + 3 : lane - 6;
+    for (;;) {
+        unsigned i = 0;
+        if (lane == 0) i = atomicAdd(a.heavy_ctr + 1, 1u);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= n_heavy) break;
+        const DensHeavy st = a.heavy[i];
+        const uint32_t p = a.targets[st.t];
+        const uint32_t pos = a.rank[p];
+        const double px = a.g.src[pos].x, py = a.g.src[pos].y, pz = a.g.src[pos].z;
+        int r0 = 0, r1 = a.g.n_roots;
+        if (a.g.in_off) {
+            r0 = system_of(a.g.in_off, a.g.n_systems, (int64_t)p);
+            r1 = r0 + 1;
+        }
+        double h = st.h, h_lo = st.h_lo, h_hi = st.h_hi;
+        int iter = st.iter;
+        bool converged = false;
+        double R = -1.0;  // radius of the cached search; < 0: nothing cached
+        int ncand = 0;
+        DensSums s;
+        auto evaluate = [&](double hh) {
+            const DensNorm nrm = dens_norm(hh, a.n_dims);
+            double acc = 0.0;
+            int inside = 0;
+            const double r2max = hh * hh;
+            // 32 particles of the search at hh, in order
+            auto add = [&](int sp, bool keep) {
+                double q[12];
+                for (int c = 0; c < 12; ++c) q[c] = 0.0;
+                bool in = false;
+                if (keep) {
+                    const double2 xy = __ldg(reinterpret_cast<const double2*>(a.g.src + sp));
+                    const double zz = __ldg(reinterpret_cast<const double*>(a.g.src + sp) + 2);
+                    const double dx = min_image(xy.x - px, a.g.box), dy = min_image(xy.y - py, a.g.box),
+                                 dz = min_image(zz - pz, a.g.box);
+                    dens_terms(dx, dy, dz, nrm, q[0], q[1], in);
+                    q[2] = __ldg(a.smass + sp);
+                    q[3] = dx; q[4] = dy; q[5] = dz;
+                    q[6] = __dmul_rn(dx, dx); q[7] = __dmul_rn(dy, dy); q[8] = __dmul_rn(dz, dz);
+                    q[9] = __dmul_rn(dx, dy); q[10] = __dmul_rn(dy, dz); q[11] = __dmul_rn(dx, dz);
+                }
+                inside += __popc(__ballot_sync(0xffffffffu, in));
+#pragma unroll
+                for (int c = 0; c < 12; ++c) T[c][lane] = q[c];
+                __syncwarp();
+                if (lane < 12) {
+#pragma unroll 8
+                    for (int k = 0; k < 32; ++k)
+                        acc = lane < 2 ? __dadd_rn(acc, T[fb][k]) : __fma_rn(T[fa][k], T[fb][k], acc);
+                }
+                __syncwarp();
+            };
+            if (!(R >= hh)) {
+                const double rad = (R < 0 ? kCacheFirst : kCacheGrow) * hh;
+                int k = 0;
+                warp_search(a.g, r0, r1, px, py, pz, rad, [&](int sp, bool keep) {
+                    keep = keep && !(a.stype && __ldg(a.stype + sp) != 0);
+                    const unsigned m = __ballot_sync(0xffffffffu, keep);
+                    const int at = k + __popc(m & ((1u << lane) - 1u));
+                    if (keep && at < kWarpCand) list[at] = (uint32_t)sp;
+                    k += __popc(m);
+                });
+                __syncwarp();
+                ncand = k;
+                R = k <= kWarpCand ? rad : -1.0;
+            }
+            if (R >= hh) {
+                for (int k0 = 0; k0 < ncand; k0 += 32) {
+                    const bool have = k0 + lane < ncand;
+                    const int sp = have ? (int)list[k0 + lane] : 0;
+                    uint32_t j = 0;
+                    add(sp, have && is_neighbour<false>(a.g, sp, px, py, pz, r2max, nullptr, 0, j));
+                }
+            } else {
+                warp_search(a.g, r0, r1, px, py, pz, hh, [&](int sp, bool keep) {
+                    keep = keep && !(a.stype && __ldg(a.stype + sp) != 0);
+                    if (__any_sync(0xffffffffu, keep)) add(sp, keep);
+                });
+            }
+            auto get = [&](int c) { return __shfl_sync(0xffffffffu, acc, c); };
+            s.wsum = get(0); s.dwdh = get(1); s.rho = get(2);
+            for (int c = 0; c < 6; ++c) s.mom[c] = get(3 + c);
+            for (int c = 0; c < 3; ++c) s.face[c] = get(9 + c);
+            s.inside = inside;
+        };
+        for (; iter < 100; ++iter) {
+            evaluate(h);
+            if (dens_newton(newton_params(a), p, s, iter, h, h_lo, h_hi)) { converged = true; break; }
+        }
+        if (!converged) evaluate(h);
+        if (lane == 0) {
+            a.h[st.t] = h;
+            a.rho[st.t] = s.rho;
+            a.nngb[st.t] = s.inside;
+            a.iters[st.t] = iter;
+        }
     }
 }
 
@@ -789,11 +1125,28 @@ void run_density(gt_context* ctx, gt_tree* t, int64_t nt, const uint32_t* target
     a.h = h; a.rho = rho; a.nngb = nngb; a.iters = iters;
     a.tally = tally && nt > 0 ? fresh_tally(ctx) : nullptr;
     a.cand = nullptr;
+    a.heavy = nullptr;
+    a.heavy_ctr = nullptr;
+    a.warp_cand = nullptr;
+    a.heavy_cap = 0;
+    a.run = 32;
+    const int solve_blocks = (int)std::min<int64_t>((nt + kBlk - 1) / kBlk, (int64_t)ctx->num_sms * 6);
+    const int heavy_blocks = (int)std::min<int64_t>((nt + kHeavyWarps - 1) / kHeavyWarps, (int64_t)ctx->num_sms * 6);
     a.cand_cap = kCandCap;
     a.n_threads = 0;
     if (!a.tally && nt > 0) {
-        a.n_threads = (int64_t)grid_of(ctx, nt) * kBlk;
+        a.n_threads = (int64_t)solve_blocks * kBlk;
+        // eight runs per warp, so that the warps end together, of 32 to 256 targets
+        a.run = (int)std::min<int64_t>(256, std::max<int64_t>(32, nt * 32 / (8 * a.n_threads) / 32 * 32));
         a.cand = (uint32_t*)scratch(ctx, kSlotNgb0, (size_t)a.n_threads * kCandCap * sizeof(uint32_t));
+        a.heavy_cap = (int)std::min<int64_t>(nt, kHeavyCap);
+        const int64_t warps = (int64_t)heavy_blocks * kHeavyWarps;
+        char* hb = (char*)scratch(ctx, kSlotNgb3, 64 + (size_t)a.heavy_cap * sizeof(DensHeavy) +
+                                                      (size_t)warps * kWarpCand * sizeof(uint32_t));
+        a.heavy_ctr = (unsigned int*)hb;
+        a.heavy = (DensHeavy*)(hb + 64);
+        a.warp_cand = (uint32_t*)(hb + 64 + (size_t)a.heavy_cap * sizeof(DensHeavy));
+        check_cuda(cudaMemsetAsync(a.heavy_ctr, 0, 12, st), "memset");
     }
     a.h_default = 0.0;
     a.h_default_sys = nullptr;
@@ -843,11 +1196,14 @@ void run_density(gt_context* ctx, gt_tree* t, int64_t nt, const uint32_t* target
         a.h_default = default_h(lo, hi, (double)t->n, des_ngb, n_dims);
     }
     if (nt <= 0) return;
-    const bool one = a.g.n_roots == 1;
-    if (a.tally) density_kernel<true, false><<<grid_of(ctx, nt), kBlk, 0, st>>>(a);
-    else if (one) density_kernel<false, true><<<grid_of(ctx, nt), kBlk, 0, st>>>(a);
-    else density_kernel<false, false><<<grid_of(ctx, nt), kBlk, 0, st>>>(a);
+    if (a.tally) density_count_kernel<<<grid_of(ctx, nt), kBlk, 0, st>>>(a);
+    else if (a.g.n_roots == 1) density_kernel<true><<<solve_blocks, kBlk, 0, st>>>(a);
+    else density_kernel<false><<<solve_blocks, kBlk, 0, st>>>(a);
     check_launch(ctx, "density_kernel");
+    if (!a.tally) {
+        density_heavy_kernel<<<heavy_blocks, kHeavyWarps * 32, 0, st>>>(a);
+        check_launch(ctx, "density_heavy_kernel");
+    }
     if (a.tally) {
         check_cuda(cudaMemcpyAsync(ctx->pinned, a.tally, GT_NGB_COUNTERS * 8, cudaMemcpyDeviceToHost, st), "d2h");
         check_cuda(cudaStreamSynchronize(st), "sync");

@@ -237,3 +237,30 @@ def test_candidate_cache_is_bit_identical(gpu_ctx, golden, ngb_tree, case):
         gpu_ctx.ngb_count(False)
     for k in ("h", "rho", "nngb", "iters"):
         assert np.array_equal(cached[k], direct[k]), k
+
+
+@pytest.mark.parametrize("nt", [1, 15, 16, 17, 33, 300, 3000])
+@pytest.mark.parametrize("guess", ["close", "wide", "whole", "nan"])
+def test_density_lanes_and_warps_match_counting_solve(gpu_ctx, nt, guess):
+    """The solve takes targets into its lanes sixteen or more at a time and hands those with more than
+    160 candidates to a warp, whose own cache holds 2048: target counts around the lanes, and first
+    guesses with tens, hundreds and all 6000 particles inside, on a clump in a sparse box.  h, rho, the
+    neighbour counts and the iterations equal the counting solve's, a thread per target, bit for bit;
+    an h that is not a number ends after 100 iterations there and here."""
+    rng = np.random.default_rng(7)
+    x = np.concatenate([0.02 * rng.normal(size=(3000, 3)), rng.uniform(-1, 1, (3000, 3))])
+    P = {"x": x[:, 0].copy(), "y": x[:, 1].copy(), "z": x[:, 2].copy(), "m": rng.uniform(0.5, 1.5, 6000)}
+    T = gpu_ctx.build(P, key_mode=g.GT_KEY_MORTON)
+    tg = rng.choice(6000, nt, replace=False).astype(np.uint32)
+    h = {"close": np.where(tg < 3000, 0.01, 0.3), "wide": np.full(nt, 0.1), "whole": np.full(nt, 5.0),
+         "nan": np.full(nt, np.nan)}[guess]
+    if guess == "nan":
+        tg, h = tg[:33], h[:33]
+    got = gpu_ctx.density(T, tg, h_start=h)
+    gpu_ctx.ngb_count(True)
+    try:
+        want = gpu_ctx.density(T, tg, h_start=h)
+    finally:
+        gpu_ctx.ngb_count(False)
+    for k in ("h", "rho", "nngb", "iters"):
+        assert np.array_equal(got[k], want[k], equal_nan=k in ("h", "rho")), k
