@@ -1113,7 +1113,7 @@ int gt_plan_destroy(gt_plan* p) {
     if (p->ctx->stream) cudaStreamSynchronize(p->ctx->stream);
     if (p->exec) cudaGraphExecDestroy(p->exec);
     if (p->graph) cudaGraphDestroy(p->graph);
-    for (void* q : {(void*)p->bufs.stack, (void*)p->bufs.ctr, (void*)p->bufs.model})
+    for (void* q : {(void*)p->bufs.stack, (void*)p->bufs.ctr, (void*)p->bufs.model, (void*)p->bufs.mac_l2, p->bufs.hand})
         if (q) cudaFree(q);
     cudaGetLastError();
     if (prev >= 0) cudaSetDevice(prev);

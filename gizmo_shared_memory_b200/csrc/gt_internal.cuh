@@ -209,6 +209,7 @@ enum Slot {
     kSlotOut0, kSlotOut1, kSlotOut2, kSlotOut3, kSlotOut4, kSlotOut5,
     kSlotStack, kSlotCounters, kSlotDirect, kSlotGroupRoot, kSlotMacL2,
     kSlotNgb0, kSlotNgb1, kSlotNgb2, kSlotNgb3,
+    kSlotHand, kSlotHand2,  // records of long windows (second: chunks on the second compute stream)
     kSlotStack2,  // traversal stacks of the second compute stream (chunked walks)
     kSlotGroupCount,  // device-side group and chunk counts of an explicit-target walk
     kSlotLevels,      // device-side level offsets and counts of the build's structure stage
@@ -259,6 +260,8 @@ void* host_stage(gt_context* ctx, size_t bytes);
 struct WalkBuffers {
     int* stack = nullptr;
     size_t stack_bytes = 0;
+    void* hand = nullptr;
+    size_t hand_bytes = 0;
     unsigned long long* ctr = nullptr;
     size_t ctr_bytes = 0;
     float* model = nullptr;  // device copy of the learned criterion's network

@@ -27,6 +27,7 @@
 //     Kahan-compensated totals (acceleration) and an FP64 total (potential); the final sums and
 //     the factor G are FP64.
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <type_traits>
 
@@ -90,6 +91,40 @@ struct WalkArgs {
     const double* smass;
     const uint32_t* nsink;
     double sink_r;
+    // long windows (walk_pair_kernel, see Handover): iterations after which a pair hands the rest of
+    // its traversal over, the records, and the counters: [0] records asked for, [1] shares taken
+    int budget;
+    int hand_cap;
+    int hand_size;  // subtrees of at most this many particles are not broken up further
+    struct Handover* hand;
+    unsigned int* hand_ctr;
+};
+
+// A window that spans a large volume (the outskirts of a halo, a jump of the curve) walks many times
+// the average number of nodes in its one warp, while the rest of the GPU has nothing left to do: in a
+// Plummer sphere of 65,536 particles the longest pair of windows takes 1,800 iterations against a mean
+// of 60, and the walk took as long as that pair.  A pair that has used up its budget of iterations
+// therefore breaks up the large subtrees on its stack (a depth-first stack has a few that hold most of
+// what is left at its bottom), writes its state here and leaves it: a second launch walks every record in kShares shares, each with every
+// kShares-th stack entry, and the share that finishes last adds the parts in a fixed order.  What is
+// handed over and how it is shared out depends on the particles alone, so results do not change
+// from run to run.  When more pairs ask for a record than there are, every pair is finished by one
+// warp: those without a record at once, those with one from the saved state, as if it had not
+// been interrupted.
+constexpr int kShares = 16;
+constexpr int kHandStack = 2048;   // entries of a record
+constexpr int kHandSteps = 96;     // at most this many steps break up the stack
+constexpr int kHandLeast = 4 * kShares;  // a shorter stack is not worth a record
+struct HandSum {
+    float2 x, y, z;  // Kahan sum and compensation
+    double pot;
+};
+struct Handover {
+    int pair, n;
+    unsigned int done, pad;
+    int stack[kHandStack];
+    HandSum sum[2][32];                 // per window and lane, at the hand-over
+    double part[kShares][4][2][32];     // each share's sums: x, y, z, potential
 };
 
 __device__ __forceinline__ int warp_incl_scan_i(int v) {
@@ -1048,7 +1083,8 @@ __host__ __device__ constexpr int pair_smem_bytes(int pn_cap, int pp_cap) {
     return ((int)sizeof(PairHdr) + 2 * pair_list_bytes(pn_cap, pp_cap) + 15) & ~15;
 }
 
-template <bool WANT_POT, bool COUNT, int MAC>
+// HAND: pairs with more iterations than A.budget hand over; SHARE: walks the records' shares.
+template <bool WANT_POT, bool COUNT, int MAC, bool HAND, bool SHARE>
 __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const WalkArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1064,7 +1100,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
     auto pp_of = [&](int v) { return pn_of(v) + A.pn_cap; };
     auto ph_of = [&](int v) { return reinterpret_cast<float*>(pp_of(v) + A.pp_cap); };
     const int n_groups = A.n_groups_dev ? (int)*A.n_groups_dev : A.n_groups;
-    const int n_pairs = (n_groups + 1) >> 1;
+    // SHARE: the units are the records' shares, or whole records when more were asked for than there are
+    const int n_hand = SHARE ? (int)A.hand_ctr[0] : 0;
+    const bool whole = SHARE && n_hand > A.hand_cap;
+    const int n_units = SHARE ? (whole ? A.hand_cap : n_hand * kShares) : (n_groups + 1) >> 1;
     // SHMEM_COUNT_WALK: per window, as walk_kernel counts them (node tests, monopoles and
     // particles times the window's targets, r = 0 pairs), so a paired walk counts what the two
     // one-window walks count
@@ -1072,10 +1111,12 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
     int c_maxtop = 0;
 
     for (;;) {
-        int pr = 0;
-        if (lane == 0) pr = (int)atomicAdd(A.next_group, 1u);
-        pr = __shfl_sync(kFull, pr, 0);
-        if (pr >= n_pairs) break;
+        int unit = 0;
+        if (lane == 0) unit = (int)atomicAdd(SHARE ? A.hand_ctr + 1 : A.next_group, 1u);
+        unit = __shfl_sync(kFull, unit, 0);
+        if (unit >= n_units) break;
+        Handover* rec = SHARE ? A.hand + (whole ? unit : unit / kShares) : nullptr;
+        const int pr = SHARE ? rec->pair : unit;
         int t0[2], nt[2];
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
@@ -1246,8 +1287,18 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
         // fetch, not arithmetic, limited the first version with a flush at every append site).
         // the root of each window: node 0, or in a forest its system's root; windows of one
         // system share a root entry, windows of two systems start from one entry each
-        int top = 1;
-        {
+        int top = 1, bot = 0;  // the stack's entries: [bot, top), bot > 0 only after breadth-first steps
+        if (SHARE) {
+            // every kShares-th entry of the saved stack, or all of it with the sums so far
+            const int first = whole ? 0 : unit % kShares, every = whole ? 1 : kShares, n = rec->n;
+            top = n > first ? (n - first + every - 1) / every : 0;
+            for (int i = lane; i < top; i += 32) stk[i] = rec->stack[first + i * every];
+            if (whole) {
+                const HandSum a = rec->sum[0][lane], b = rec->sum[1][lane];
+                sx0 = a.x.x; cx0 = a.x.y; sy0 = a.y.x; cy0 = a.y.y; sz0 = a.z.x; cz0 = a.z.y; pot0 = a.pot;
+                sx1 = b.x.x; cx1 = b.x.y; sy1 = b.y.x; cy1 = b.y.y; sz1 = b.z.x; cz1 = b.z.y; pot1 = b.pot;
+            }
+        } else {
             const int ra = A.group_root ? A.group_root[2 * pr] : 0;
             const int rb = (A.group_root && nt[1] > 0) ? A.group_root[2 * pr + 1] : ra;
             if (ra == rb) {
@@ -1261,21 +1312,30 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
         int npn0 = 0, npn1 = 0, npp0 = 0, npp1 = 0;
         int base = 0, tot2 = 0;  // the expanded leaves' particles still to place: [base, tot2)
         bool overflow = false;
+        int left = HAND ? A.budget : 0;  // iterations of the budget; below 0, the stack is broken up
+        int quiet = 0;                   // entries seen since one was broken up
+        int slot = -1;                   // >= 0: the record asked for -- flush the lists, then save
         for (;;) {
-            const bool done = top == 0 && base >= tot2;
+            const bool done = base >= tot2 && (top == bot || (HAND && slot >= 0));
+            if (done || max(npn0, npn1) > A.pn_cap - 32 || max(npp0, npp1) > A.pp_cap - 32) {
 #pragma unroll 1
-            for (int v = 0; v < 2; ++v) {
-                const int n1 = v ? npn1 : npn0, n2 = v ? npp1 : npp0;
-                if (n1 > 0 && (done || n1 > A.pn_cap - 32)) {
-                    flush_pn(v, n1);
-                    if (v) npn1 = 0; else npn0 = 0;
+                for (int v = 0; v < 2; ++v) {
+                    const int n1 = v ? npn1 : npn0, n2 = v ? npp1 : npp0;
+                    if (n1 > 0 && (done || n1 > A.pn_cap - 32)) {
+                        flush_pn(v, n1);
+                        if (v) npn1 = 0; else npn0 = 0;
+                    }
+                    if (n2 > 0 && (done || n2 > A.pp_cap - 32)) {
+                        flush_pp(v, n2);
+                        if (v) npp1 = 0; else npp0 = 0;
+                    }
                 }
-                if (n2 > 0 && (done || n2 > A.pp_cap - 32)) {
-                    flush_pp(v, n2);
-                    if (v) npp1 = 0; else npp0 = 0;
+                if (done) {
+                    if (!HAND || slot < A.hand_cap) break;
+                    slot = -1;  // no record left: this warp goes on from the same state
+                    left = INT_MAX;
                 }
             }
-            if (done) break;
 
             if (base < tot2) {
                 // 32 expanded-leaf particles, one per lane, to the windows that opened their leaf:
@@ -1325,19 +1385,52 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                     npp += __popc(nm);
                 }
                 base += 32;
+                if (HAND) --left;
                 __syncwarp();
                 continue;
             }
 
             // one traversal step: pop up to 32 nodes, test each against its windows
-            const int npop = min(top, 32);
-            top -= npop;
-            const int ent = lane < npop ? stk[top + lane] : -1;
+            bool fifo = false;
+            if (HAND && --left < 0) {
+                const bool over = left < -kHandSteps || quiet >= top - bot || top - bot > kHandStack - 256;
+                if (over || top + 256 > A.stack_cap) {  // the stack back to its start
+                    top -= bot;
+                    for (int i = 0; i < top; i += 32) {
+                        const int q = i + lane < top ? stk[bot + i + lane] : 0;
+                        __syncwarp();
+                        if (i + lane < top) stk[i + lane] = q;
+                        __syncwarp();
+                    }
+                    bot = 0;
+                }
+                if (over) {
+                    left = INT_MAX;
+                    if (top >= kHandLeast && top <= kHandStack) {
+                        if (lane == 0) slot = (int)atomicAdd(A.hand_ctr, 1u);
+                        slot = __shfl_sync(kFull, slot, 0);
+                        continue;
+                    }
+                } else {
+                    fifo = true;
+                }
+            }
+            const int npop = min(top - bot, 32);
+            if (!fifo) top -= npop;
+            const int from = fifo ? bot : top;
+            if (fifo) bot += npop;
+            const int ent = lane < npop ? stk[from + lane] : -1;
             int node = ent >= 0 ? (ent >> 2) : -1;
             if (node >= 0 && !GT_IN_BOUNDS(node, A.n_nodes)) node = -1;
-            const int mk = node >= 0 ? (ent & 3) : 0;
+            int mk = node >= 0 ? (ent & 3) : 0;
             __syncwarp();
             const NodeV nd = load_node(A.nodes + (node >= 0 ? node : 0));
+            // a subtree small enough for one share goes back to the stack as it is
+            const bool keep = HAND && fifo && node >= 0 && nd.phi - nd.plo <= A.hand_size;
+            if (HAND && fifo) {
+                if (keep) mk = 0;
+                quiet = __any_sync(kFull, node >= 0 && !keep) ? 0 : quiet + npop;
+            }
             const bool leaf = nd.first < 0;
             if (COUNT) {
                 const unsigned tests = __reduce_add_sync(kFull, (unsigned)__popc(mk));
@@ -1366,7 +1459,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
 
             // children of opened interior nodes, with the windows that opened them; one scan for
             // the children's stack slots and the expanded leaves' particle slots (walk_kernel)
-            const int nch = push ? nd.nchild : 0;
+            const int nch = keep ? 1 : push ? nd.nchild : 0;
             const int cnt = expand ? nd.phi - nd.plo : 0;
             int incl, inc2;
             if (!__any_sync(kFull, cnt >= (1 << 16))) {
@@ -1383,7 +1476,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                 int* dst = stk + (top + incl - nch);
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
-                    if (c < nch) dst[c] = ((nd.first + c) << 2) | pm;
+                    if (c < nch) dst[c] = keep ? ent : ((nd.first + c) << 2) | pm;
             }
             top += tot;
             if (COUNT) c_maxtop = max(c_maxtop, top);
@@ -1415,6 +1508,47 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
             continue;
         }
 
+        if (HAND && slot >= 0) {
+            Handover* q = A.hand + slot;
+            if (lane == 0) { q->pair = pr; q->n = top; q->done = 0u; }
+            for (int i = lane; i < top; i += 32) q->stack[i] = stk[i];
+            q->sum[0][lane] = HandSum{make_float2(sx0, cx0), make_float2(sy0, cy0), make_float2(sz0, cz0), pot0};
+            q->sum[1][lane] = HandSum{make_float2(sx1, cx1), make_float2(sy1, cy1), make_float2(sz1, cz1), pot1};
+            continue;
+        }
+        double more[2][4] = {};  // SHARE: what is added to this share's sums, per window
+        if (SHARE && !whole) {
+            const int share = unit % kShares;
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                rec->part[share][0][v][lane] = (double)(v ? sx1 : sx0) - (double)(v ? cx1 : cx0);
+                rec->part[share][1][v][lane] = (double)(v ? sy1 : sy0) - (double)(v ? cy1 : cy0);
+                rec->part[share][2][v][lane] = (double)(v ? sz1 : sz0) - (double)(v ? cz1 : cz0);
+                if (WANT_POT) rec->part[share][3][v][lane] = v ? pot1 : pot0;
+            }
+            __threadfence();
+            __syncwarp();
+            unsigned int before = 0;
+            if (lane == 0) before = atomicAdd(&rec->done, 1u);
+            before = __shfl_sync(kFull, before, 0);
+            if (before != kShares - 1) continue;
+            __threadfence();
+            // the last share: the sums at the hand-over, then all shares in order (its own too)
+            sx0 = sy0 = sz0 = cx0 = cy0 = cz0 = sx1 = sy1 = sz1 = cx1 = cy1 = cz1 = 0.0f;
+            pot0 = pot1 = 0.0;
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const HandSum a = rec->sum[v][lane];
+                more[v][0] = (double)a.x.x - (double)a.x.y;
+                more[v][1] = (double)a.y.x - (double)a.y.y;
+                more[v][2] = (double)a.z.x - (double)a.z.y;
+                more[v][3] = a.pot;
+                for (int q = 0; q < kShares; ++q)
+#pragma unroll
+                    for (int c = 0; c < (WANT_POT ? 4 : 3); ++c) more[v][c] += __ldcg(&rec->part[q][c][v][lane]);
+            }
+        }
+
         // ---- write --------------------------------------------------------------------------
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
@@ -1425,11 +1559,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                 const float sx = v ? sx1 : sx0, sy = v ? sy1 : sy0, sz = v ? sz1 : sz0;
                 const float cx = v ? cx1 : cx0, cy = v ? cy1 : cy0, cz = v ? cz1 : cz0;
                 if (A.ax) {
-                    A.ax[o] = A.G * ((double)sx - (double)cx);
-                    A.ay[o] = A.G * ((double)sy - (double)cy);
-                    A.az[o] = A.G * ((double)sz - (double)cz);
+                    A.ax[o] = A.G * (SHARE ? (double)sx - (double)cx + more[v][0] : (double)sx - (double)cx);
+                    A.ay[o] = A.G * (SHARE ? (double)sy - (double)cy + more[v][1] : (double)sy - (double)cy);
+                    A.az[o] = A.G * (SHARE ? (double)sz - (double)cz + more[v][2] : (double)sz - (double)cz);
                 }
-                if (WANT_POT && A.phi) A.phi[o] = A.G * (v ? pot1 : pot0);
+                if (WANT_POT && A.phi) A.phi[o] = A.G * (SHARE ? (v ? pot1 : pot0) + more[v][3] : v ? pot1 : pot0);
             }
         }
     }
@@ -1850,33 +1984,51 @@ constexpr int kPairCapDefault = 160;
 
 size_t pair_smem(int warps, int pn_cap) { return (size_t)warps * pair_smem_bytes(pn_cap, pn_cap / 2); }
 
-template <bool POT, bool CNT, int MAC>
+constexpr int kHandRecords = 2048;  // 90 MB
+
+template <bool POT, bool CNT, int MAC, bool HAND, bool SHARE>
 void prepare_pair() {
     static bool done = false;
     if (done) return;
-    check_cuda(cudaFuncSetAttribute(walk_pair_kernel<POT, CNT, MAC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)pair_smem(kMaxWarps, kPairCapMax)),
+    check_cuda(cudaFuncSetAttribute(walk_pair_kernel<POT, CNT, MAC, HAND, SHARE>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem(kMaxWarps, kPairCapMax)),
                "cudaFuncSetAttribute");
-    check_cuda(cudaFuncSetAttribute(walk_pair_kernel<POT, CNT, MAC>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    100),
+    check_cuda(cudaFuncSetAttribute(walk_pair_kernel<POT, CNT, MAC, HAND, SHARE>,
+                                    cudaFuncAttributePreferredSharedMemoryCarveout, 100),
                "cudaFuncSetAttribute");
     done = true;
 }
 
 template <bool POT, bool CNT, int MAC>
 int pair_occupancy(int warps, int pn_cap) {
-    prepare_pair<POT, CNT, MAC>();
+    prepare_pair<POT, CNT, MAC, false, false>();
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, walk_pair_kernel<POT, CNT, MAC>, warps * 32,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, walk_pair_kernel<POT, CNT, MAC, false, false>, warps * 32,
                                                   pair_smem(warps, pn_cap));
     return std::max(1, nb);
 }
 
+// Blocks of the launch that walks the records' shares, their number known on the device only.
+int share_grid(gt_context* ctx, int records, int warps) {
+    const int64_t units = (int64_t)records * kShares;
+    return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * 3, (units + warps - 1) / warps));
+}
+
+template <bool POT, bool CNT, int MAC, bool HAND, bool SHARE>
+void launch_pair_kernel(gt_context* ctx, const WalkArgs& a, int blocks, int warps) {
+    prepare_pair<POT, CNT, MAC, HAND, SHARE>();
+    walk_pair_kernel<POT, CNT, MAC, HAND, SHARE><<<blocks, warps * 32, pair_smem(warps, a.pn_cap), ctx->stream>>>(a);
+    check_launch(ctx, "walk_pair_kernel");
+}
+
 template <bool POT, bool CNT, int MAC>
 void launch_pair(gt_context* ctx, const WalkArgs& a, int blocks, int warps) {
-    prepare_pair<POT, CNT, MAC>();
-    walk_pair_kernel<POT, CNT, MAC><<<blocks, warps * 32, pair_smem(warps, a.pn_cap), ctx->stream>>>(a);
-    check_launch(ctx, "walk_pair_kernel");
+    if (a.budget <= 0) {
+        launch_pair_kernel<POT, CNT, MAC, false, false>(ctx, a, blocks, warps);
+    } else {
+        launch_pair_kernel<POT, CNT, MAC, true, false>(ctx, a, blocks, warps);
+        launch_pair_kernel<POT, CNT, MAC, false, true>(ctx, a, share_grid(ctx, a.hand_cap, warps), warps);
+    }
 }
 
 template <bool POT, bool CNT>
@@ -1900,6 +2052,12 @@ void dispatch_pair(gt_context* ctx, const WalkArgs& a, int blocks, int warps, bo
 // little of the results' download is left when the last kernel ends; the chunks between are large
 // enough that each one's download hides under the next one's walk.
 constexpr int kChunks = 5;
+// The counter block of a walk, in words of 8 bytes: statistics, group counter and error up to 10, then
+// the chunks' group counters, from 16 the chunk bounds, from kCtrHand the record counters of each
+// chunk's hand-overs.
+constexpr int kCtrHand = 24;
+constexpr size_t kCtrBytes = 256;
+static_assert((kCtrHand + kChunks) * 8 <= (int)kCtrBytes && 16 * 8 + (kChunks + 1) * 8 <= kCtrHand * 8, "counter block");
 struct ChunkEdges {
     int pct[kChunks + 1];
 };
@@ -2118,9 +2276,25 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         per_sm = mac ? occupancy_blocks<4, true, false, false, 1>(warps, pn_cap)
                : macn ? occupancy_blocks<4, true, false, false, 2>(warps, pn_cap)
                       : occupancy_blocks<4, true, false, false, 0>(warps, pn_cap);
+    // Long windows hand over (Handover) where a walk of the whole tree lasts about as long as its longest
+    // pair: fewer than two pairs per resident warp.  The budget is 96 iterations, half as much again as
+    // a pair's mean, where the records suffice for every pair of the tree, and 192 beyond, which a few
+    // per cent of the pairs reach.  A Plummer sphere of 65,536: 4.6 -> 0.8 ms, of 300,000: 1.01 -> 0.71
+    // ms; a galaxy of 100,000: 0.495 -> 0.469 ms.  With more pairs the GPU is busy to the end and the
+    // hand-over only adds work: 5.8 -> 6.3 ms for a galaxy of 2^22 at 256.  The rule reads the tree's
+    // size and not the call's targets, so a slice of the targets is walked as it is in the whole.
+    const int64_t tree_units = paired ? ((t->n_live + param - 1) / param + 1) / 2 : 0;
+    const int64_t units = ((all || t->n_systems > 1 ? ng : (nt + param - 1) / std::max(1, param)) + 1) / 2;
+    int budget = 0, hand_cap = 0;
+    if (paired && tree_units < (int64_t)2 * 24 * ctx->num_sms) {
+        hand_cap = (int)std::min<int64_t>(units, kHandRecords);
+        budget = tree_units <= kHandRecords ? 96 : 192;
+    }
     const int64_t want_blocks = ((paired ? (ng + 1) / 2 : ng) + warps - 1) / warps;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want_blocks, (int64_t)per_sm * ctx->num_sms));
+    // a breadth-first stack of a long window lies below the depth-first levels
     int stack_cap = rq.stack_capacity > 0 ? rq.stack_capacity : 256 * std::max(1, t->n_levels) + 32;
+    if (budget > 0) stack_cap += kHandStack;
     stack_cap = (stack_cap + 31) & ~31;
 
     WalkArgs a;
@@ -2142,7 +2316,8 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     a.az = rq.want_acc ? rq.az : nullptr;
     a.phi = rq.phi;
     a.out_map = (all && rq.out_original) ? t->order : nullptr;
-    const int total_warps = blocks * warps;
+    // a warp of either launch needs a traversal stack
+    const int total_warps = std::max(blocks, budget > 0 ? share_grid(ctx, hand_cap, warps) : 0) * warps;
     a.pn_cap = pn_cap;
     a.pp_cap = pn_cap / 2;
     a.warp_bytes = paired ? pair_smem_bytes(a.pn_cap, a.pp_cap) : warp_smem_bytes(a.pn_cap, a.pp_cap, ext);
@@ -2171,10 +2346,24 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     };
     unsigned long long* ctr;
     if (wb) {
-        own((void**)&wb->ctr, wb->ctr_bytes, 256);
+        own((void**)&wb->ctr, wb->ctr_bytes, kCtrBytes);
         ctr = wb->ctr;
     } else {
-        ctr = (unsigned long long*)scratch(ctx, kSlotCounters, 256);
+        ctr = (unsigned long long*)scratch(ctx, kSlotCounters, kCtrBytes);
+    }
+    a.budget = budget;
+    a.hand_cap = hand_cap;
+    a.hand_size = (int)std::max<int64_t>(64, t->n_live / t->n_systems / 256);
+    a.hand_ctr = (unsigned int*)(ctr + kCtrHand);
+    a.hand = nullptr;
+    const size_t hand_bytes = (size_t)hand_cap * sizeof(Handover);
+    if (budget > 0) {
+        if (wb) {
+            own((void**)&wb->hand, wb->hand_bytes, hand_bytes);
+            a.hand = (Handover*)wb->hand;
+        } else {
+            a.hand = (Handover*)scratch(ctx, kSlotHand, hand_bytes);
+        }
     }
     a.next_group = (unsigned int*)(ctr + 8);
     a.stats = ctr;
@@ -2214,7 +2403,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     if (chunked) {
         ensure_copy_stream(ctx);
         int2* bounds = (int2*)(ctr + 16);  // K+1 int2 after the counters
-        check_cuda(cudaMemsetAsync(ctr, 0, 256, st), "memset counters");
+        check_cuda(cudaMemsetAsync(ctr, 0, kCtrBytes, st), "memset counters");
         chunk_bounds_kernel<<<1, 1, 0, st>>>(groups, (int)ng, (int)nt, kChunkEdge, bounds, ng_dev, paired ? 1 : 0);
         check_launch(ctx, "chunk_bounds_kernel");
         int2 hb[kChunks + 1];
@@ -2270,6 +2459,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         const bool two = wb == nullptr;
         cudaStream_t cs[2] = {st, two ? ctx->walk2 : st};
         int* stacks[2] = {a.stack, two ? (int*)scratch(ctx, kSlotStack2, stack_bytes) : a.stack};
+        Handover* hands[2] = {a.hand, two && budget > 0 ? (Handover*)scratch(ctx, kSlotHand2, hand_bytes) : a.hand};
         check_cuda(cudaEventRecord(ctx->ev0, st), "event");
         if (two) {
             check_cuda(cudaEventRecord(ctx->walk2_start, st), "event");
@@ -2289,6 +2479,8 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
                 ctx->stream = s;
                 WalkArgs ac = a;
                 ac.stack = stacks[c & 1];
+                ac.hand = hands[c & 1];
+                ac.hand_ctr = (unsigned int*)(ctr + kCtrHand + c);
                 ac.groups = groups + g0;
                 ac.n_groups = g1 - g0;
                 ac.n_groups_dev = nullptr;
@@ -2348,7 +2540,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
             a.stack = (int*)scratch(ctx, kSlotStack, stack_bytes);
         }
         a.stack_cap = stack_cap;
-        check_cuda(cudaMemsetAsync(ctr, 0, 96, st), "memset counters");
+        check_cuda(cudaMemsetAsync(ctr, 0, kCtrBytes, st), "memset counters");
         if (!rq.capture) check_cuda(cudaEventRecord(ctx->ev0, st), "event");
         if (paired) dispatch_pair(ctx, a, blocks, warps, want_pot, rq.count, rq.mac);
         else if (xt) dispatch_xt(ctx, a, blocks, warps, ext, rq.leaf_accept, want_pot, rq.count);

@@ -317,6 +317,36 @@ def test_interaction_counts_match_oracle(gpu_ctx, plummer_trees):
     assert s["groups"] == len(O.groups(ob, 0)) - 1
 
 
+@pytest.mark.parametrize("n", [33, 2049, 20000, 65536, 150000])
+def test_long_windows_handed_over(gpu_ctx, oracle, n):
+    """Windows of 32 on a Plummer sphere, whose outskirts hold windows that walk most of the tree and
+    hand over to other warps (at most 131,072 particles: every pair may; above: a larger budget),
+    accelerations and potential against the oracle walk.  The same call twice, and through a plan,
+    gives the same bits: what is handed over depends on the particles alone."""
+    import torch
+
+    P = ics.plummer(n=n, seed=n)
+    T, O = gpu_ctx.build(P, key_mode=g.GT_KEY_MORTON), oracle.build(P)
+    kw = dict(theta=0.7, batch=32, group_mode=g.GT_GROUP_BATCH, want_phi=True)
+    ox, oy, oz, _ = O.accel_grouped(T.download(nodes=False)["orderbuf"], 0.7, batch=32)
+    d, s = gpu_ctx.accel_grouped(T, None, **kw), gpu_ctx.accel_grouped(T, None, window_pairs=False, **kw)
+    e = relerr(*d[:3], ox, oy, oz)
+    assert np.median(e) <= MEDIAN_TOL and np.quantile(e, 0.99) <= 2e-3
+    assert np.abs(d[3] / s[3] - 1).max() <= 1e-5  # FP32 sums per list in another order
+    aold = gpu_ctx.form_aold(*d[:3], 0.0025)
+    runs = [gpu_ctx.accel_grouped(T, None, aold=aold, batch=32, group_mode=g.GT_GROUP_BATCH) for _ in range(2)]
+    dev = torch.as_tensor(aold, device="cuda")
+    outs = tuple(torch.empty(n, dtype=torch.float64, device="cuda") for _ in range(3))
+    ctx = g.Context(0, torch_stream=True)
+    ctx.plan(T, dev, outs, batch=32, group_mode=g.GT_GROUP_BATCH).launch()
+    torch.cuda.synchronize()
+    one = gpu_ctx.accel_grouped(T, None, aold=aold, batch=32, group_mode=g.GT_GROUP_BATCH, window_pairs=False)
+    for k in range(3):
+        assert np.array_equal(runs[0][k], runs[1][k]) and np.array_equal(runs[0][k], outs[k].cpu().numpy())
+    e = relerr(*runs[0], *one)  # FP32 sums in another order
+    assert np.median(e) <= 1e-6 and e.max() <= 1e-4
+
+
 # ---- direct sum -----------------------------------------------------------------------------
 
 def test_direct_fp64_and_fp32(gpu_ctx, oracle, plummer):
