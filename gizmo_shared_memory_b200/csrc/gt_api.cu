@@ -191,6 +191,7 @@ void free_tree_arrays(gt_tree* t) {
             else cudaFree(c.groups);
         }
         if (c.roots) cudaFree(c.roots);
+        if (c.packs) cudaFreeAsync(c.packs, 0);
     }
     t->group_cache.clear();
 }

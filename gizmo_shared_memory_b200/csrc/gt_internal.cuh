@@ -185,6 +185,8 @@ struct gt_tree {
         int2* groups = nullptr;
         int* roots = nullptr;  // forest: root node of each group
         int64_t n_groups = 0;
+        int2* packs = nullptr; // runs of consecutive small groups (first, number), from the pool; made on first use
+        int64_t n_packs = 0;
         bool pooled = false;   // groups came from the stream-ordered pool (cudaMallocAsync)
     };
     std::vector<GroupCache> group_cache;

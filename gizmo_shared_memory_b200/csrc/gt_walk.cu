@@ -93,6 +93,9 @@ struct WalkArgs {
     double sink_r;
     // long windows (walk_pair_kernel, see Handover): iterations after which a pair hands the rest of
     // its traversal over, the records, and the counters: [0] records asked for, [1] shares taken
+    // packs of groups (walk_pack_kernel): first group and number of groups
+    const int2* packs;
+    int n_packs;
     int budget;
     int hand_cap;
     int hand_size;  // subtrees of at most this many particles are not broken up further
@@ -1583,6 +1586,425 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
 }
 
 // ---------------------------------------------------------------------------------------------
+// Packs of small groups
+// ---------------------------------------------------------------------------------------------
+// The engine's grouping walks one leaf at a time: five targets on average, whose box is small, so the
+// walk of a leaf visits two thirds of the nodes that a window of 32 does -- for a sixth of the targets.
+// One warp per leaf spent most of its time on that traversal.  A pack is a run of up to eight
+// consecutive groups with at most 32 targets, one per lane, in one traversal: the pop, the node
+// load, the child pushes and the opened leaves' particles are shared, as in walk_pair_kernel, and
+// a popped node is tested for each group whose walk reaches it, so every group makes exactly its own
+// walk's decisions.  Groups adjacent in the tree open mostly the same nodes.
+//   * The stack entry's low eight bits are the groups that opened its parent.
+//   * Monopoles accepted by every group, and farther from the pack's box than its diagonal, go to a
+//     list that is evaluated as a window's is.
+//   * The others carry the groups that accepted them, and a lane takes the mass of an entry that is not
+//     its group's as zero.  Their offsets from the pack's centre are sums of two floats, and so are
+//     those of the softened particle list: a pack's box is larger than a leaf's, and with single
+//     floats the distance of a near entry would be rounded more coarsely than in the leaf's own walk
+//     (3.1e-7 against 9.2e-8 of the acceleration's norm on a galaxy of a million particles).
+//   * An opened leaf's particle that is outside every target's softening is a monopole.
+constexpr int kPackGroups = 8;
+constexpr int kPackAll = 160, kPackSome = 96, kPackNear = 64;  // list capacities per warp
+
+struct alignas(16) PackHdr {
+    int lo[32];
+    int pre[32];
+    int msk[32];
+    PairHdr::Win wb[kPackGroups];
+    PairHdr::Win all;  // the pack's own box
+};
+constexpr int kPackBytes = ((int)sizeof(PackHdr) + 4 * (4 * kPackAll + 8 * kPackSome + 9 * kPackNear) + 15) & ~15;
+static_assert(4 * (4 * kPackAll + 8 * kPackSome + 9 * kPackNear) >= 5 * 32 * 8, "the targets are staged in the lists");
+
+template <bool WANT_POT, int MAC>
+__global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pack_kernel(const WalkArgs A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    int* __restrict__ stk = A.stack + (size_t)(blockIdx.x * (blockDim.x >> 5) + w) * A.stack_cap;
+    unsigned char* wbase = smem_raw + (size_t)w * kPackBytes;
+    PackHdr& S = *reinterpret_cast<PackHdr*>(wbase);
+    float* __restrict__ LA = reinterpret_cast<float*>(wbase + sizeof(PackHdr));  // x, y, z, m
+    float* __restrict__ LS = LA + 4 * kPackAll;   // x, y, z, their low parts, m, groups
+    float* __restrict__ LN = LS + 8 * kPackSome;  // x, y, z, their low parts, m, softening, groups
+    for (;;) {
+        int u = 0;
+        if (lane == 0) u = (int)atomicAdd(A.next_group, 1u);
+        u = __shfl_sync(kFull, u, 0);
+        if (u >= A.n_packs) break;
+        const int2 pk = A.packs[u];
+        const int G = pk.y, t0 = A.groups[pk.x].x, nt = A.groups[pk.x + G - 1].y - t0;
+        const unsigned full = (1u << G) - 1u;
+        // ---- targets: lane l holds target l of the pack; its group's bit --------------------------
+        const int gs = lane < G ? A.groups[pk.x + lane].x - t0 : 0, ge = lane < G ? A.groups[pk.x + lane].y - t0 : 0;
+        const unsigned starts = __reduce_or_sync(kFull, lane < G ? 1u << gs : 0u);
+        const unsigned mine = 1u << (__popc(starts & (lt_mask | (1u << lane))) - 1);
+        double px = 0.0, py = 0.0, pz = 0.0, ps = 0.0;
+        double* __restrict__ st = reinterpret_cast<double*>(LA);  // the lists are empty: stage the targets there
+        if (lane < nt) {
+            float mf, hf;
+            load_src(A.src + t0 + lane, px, py, pz, mf, hf);
+            ps = A.ssoft[t0 + lane];
+            st[lane] = px; st[32 + lane] = py; st[64 + lane] = pz; st[96 + lane] = ps;
+            st[128 + lane] = A.aold ? A.aold[t0 + lane] : 0.0;
+        }
+        __syncwarp();
+        double lx = 1e300, ly = 1e300, lz = 1e300, hx = -1e300, hy = -1e300, hz = -1e300, emax = 0.0;
+        if (lane < G) {
+            double amin = 1e300;
+            for (int i = gs; i < ge; ++i) {
+                const double x = st[i], y = st[32 + i], z = st[64 + i];
+                lx = fmin(lx, x); hx = fmax(hx, x);
+                ly = fmin(ly, y); hy = fmax(hy, y);
+                lz = fmin(lz, z); hz = fmax(hz, z);
+                emax = fmax(emax, st[96 + i]);
+                amin = fmin(amin, st[128 + i]);
+            }
+            PairHdr::Win& q = S.wb[lane];
+            q.c_x = 0.5 * (lx + hx); q.c_y = 0.5 * (ly + hy); q.c_z = 0.5 * (lz + hz);
+            q.w_x = 0.5 * (hx - lx); q.w_y = 0.5 * (hy - ly); q.w_z = 0.5 * (hz - lz);
+            q.emax = emax; q.amin = amin;
+        }
+        lx = wmin(lx); ly = wmin(ly); lz = wmin(lz);
+        hx = wmax(hx); hy = wmax(hy); hz = wmax(hz);
+        emax = wmax(emax);
+        const double cx = 0.5 * (lx + hx), cy = 0.5 * (ly + hy), cz = 0.5 * (lz + hz);
+        if (lane == 0) {
+            S.all.c_x = cx; S.all.c_y = cy; S.all.c_z = cz;
+            S.all.w_x = 0.5 * (hx - lx); S.all.w_y = 0.5 * (hy - ly); S.all.w_z = 0.5 * (hz - lz);
+            S.all.emax = emax;
+            // the square of the box's diagonal
+            S.all.amin = (hx - lx) * (hx - lx) + (hy - ly) * (hy - ly) + (hz - lz) * (hz - lz);
+        }
+        __syncwarp();
+        const float tx = (float)(px - cx), ty = (float)(py - cy), tz = (float)(pz - cz), th = (float)ps;
+        const float ux = (float)(px - cx - (double)tx), uy = (float)(py - cy - (double)ty), uz = (float)(pz - cz - (double)tz);
+        float sx = 0.0f, sy = 0.0f, sz = 0.0f, kx = 0.0f, ky = 0.0f, kz = 0.0f;
+        double pot = 0.0;
+        auto add_partial = [&](float2 ax, float2 ay, float2 az, float2 np) {
+            kahan_add(sx, kx, ax.x + ax.y);
+            kahan_add(sy, ky, ay.x + ay.y);
+            kahan_add(sz, kz, az.x + az.y);
+            if (WANT_POT) pot -= (double)(np.x + np.y);
+        };
+        const float2 ntx = make_float2(-tx, -tx), nty = make_float2(-ty, -ty), ntz = make_float2(-tz, -tz);
+        const float2 r2_floor = make_float2(1e-30f, 1e-30f);
+        const float2 nux = make_float2(-ux, -ux), nuy = make_float2(-uy, -uy), nuz = make_float2(-uz, -uz);
+        // two monopoles at offset d, as walk_pair_kernel evaluates them
+        auto two = [&](float2 dx, float2 dy, float2 dz, float2 M, float2& ax, float2& ay, float2& az, float2& np) {
+            const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, r2_floor)));
+            const float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+            const float2 mri = __fmul2_rn(M, ri);
+            const float2 f = __fmul2_rn(mri, __fmul2_rn(ri, ri));
+            ax = __ffma2_rn(dx, f, ax);
+            ay = __ffma2_rn(dy, f, ay);
+            az = __ffma2_rn(dz, f, az);
+            if (WANT_POT) np = __fadd2_rn(np, mri);
+        };
+        // the offset of two entries along one axis, from the high and low parts of both ends
+        auto diff = [](float2 hi, float2 lo, float2 nt, float2 nu) { return __fadd2_rn(__fadd2_rn(hi, nt), __fadd2_rn(lo, nu)); };
+        const float2 zero2 = make_float2(0.0f, 0.0f);
+        auto flush_all = [&](int n) {
+            if (lane < (-n & 3))
+#pragma unroll
+                for (int c = 0; c < 4; ++c) LA[c * kPackAll + n + lane] = 0.0f;
+            __syncwarp();
+            const float4* __restrict__ L = reinterpret_cast<const float4*>(LA);
+            float2 ax = zero2, ay = zero2, az = zero2, np = zero2;
+            const int nq = (n + 3) >> 2;
+#pragma unroll 4
+            for (int j = 0; j < nq; ++j) {
+                const float4 X = L[j], Y = L[j + kPackAll / 4], Z = L[j + kPackAll / 2], M = L[j + 3 * kPackAll / 4];
+                two(__fadd2_rn(make_float2(X.x, X.y), ntx), __fadd2_rn(make_float2(Y.x, Y.y), nty),
+                    __fadd2_rn(make_float2(Z.x, Z.y), ntz), make_float2(M.x, M.y), ax, ay, az, np);
+                two(__fadd2_rn(make_float2(X.z, X.w), ntx), __fadd2_rn(make_float2(Y.z, Y.w), nty),
+                    __fadd2_rn(make_float2(Z.z, Z.w), ntz), make_float2(M.z, M.w), ax, ay, az, np);
+            }
+            add_partial(ax, ay, az, np);
+            __syncwarp();
+        };
+        auto mass_if = [&](float m, float g) { return (__float_as_uint(g) & mine) ? m : 0.0f; };
+        auto flush_some = [&](int n) {
+            if ((n & 1) && lane < 8) LS[lane * kPackSome + n] = 0.0f;
+            __syncwarp();
+            const float2* __restrict__ L = reinterpret_cast<const float2*>(LS);
+            constexpr int st2 = kPackSome / 2;
+            float2 ax = zero2, ay = zero2, az = zero2, np = zero2;
+            const int n2 = (n + 1) >> 1;
+#pragma unroll 4
+            for (int j = 0; j < n2; ++j) {
+                const float2 M = L[j + 6 * st2], g = L[j + 7 * st2];
+                two(diff(L[j], L[j + 3 * st2], ntx, nux), diff(L[j + st2], L[j + 4 * st2], nty, nuy),
+                    diff(L[j + 2 * st2], L[j + 5 * st2], ntz, nuz), make_float2(mass_if(M.x, g.x), mass_if(M.y, g.y)), ax, ay,
+                    az, np);
+            }
+            add_partial(ax, ay, az, np);
+            __syncwarp();
+        };
+        // particles: walk_pair_kernel's softened pairs on the two-float offsets
+        auto flush_near = [&](int n) {
+            if ((n & 1) && lane == 0) {
+#pragma unroll
+                for (int c = 0; c < 9; ++c) LN[c * kPackNear + n] = c < 3 ? 1e18f : 0.0f;
+            }
+            __syncwarp();
+            const float2* __restrict__ L = reinterpret_cast<const float2*>(LN);
+            constexpr int st2 = kPackNear / 2;
+            float2 ax = zero2, ay = zero2, az = zero2, np = zero2;
+            const int n2 = (n + 1) >> 1;
+            for (int j = 0; j < n2; ++j) {
+                const float2 dx = diff(L[j], L[j + 3 * st2], ntx, nux);
+                const float2 dy = diff(L[j + st2], L[j + 4 * st2], nty, nuy);
+                const float2 dz = diff(L[j + 2 * st2], L[j + 5 * st2], ntz, nuz);
+                const float2 m0 = L[j + 6 * st2], hj = L[j + 7 * st2], g = L[j + 8 * st2];
+                const float2 M = make_float2(mass_if(m0.x, g.x), mass_if(m0.y, g.y));
+                const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                const float2 hh = make_float2(fmaxf(th, hj.x), fmaxf(th, hj.y));
+                const float2 hh2 = __fmul2_rn(hh, hh);
+                const bool z0 = r2.x == 0.0f, z1 = r2.y == 0.0f;
+                float2 f, mp;
+                if ((r2.x >= hh2.x || z0) && (r2.y >= hh2.y || z1)) {
+                    const float2 ri = make_float2(z0 ? 0.0f : rsqrt_ftz(r2.x), z1 ? 0.0f : rsqrt_ftz(r2.y));
+                    mp = __fmul2_rn(M, ri);
+                    f = __fmul2_rn(mp, __fmul2_rn(ri, ri));
+                } else {
+                    const float r2s[2] = {r2.x, r2.y}, hs[2] = {hh.x, hh.y}, ms[2] = {M.x, M.y};
+                    float fs[2], qs[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        if (r2s[e] >= hs[e] * hs[e] && r2s[e] > 0.0f) {
+                            const float ri = rsqrt_ftz(r2s[e]);
+                            const float mri = ms[e] * ri;
+                            fs[e] = mri * (ri * ri);
+                            qs[e] = -mri;
+                        } else {
+                            spline_pair(r2s[e], hs[e], ms[e], fs[e], qs[e]);
+                        }
+                    }
+                    f = make_float2(fs[0], fs[1]);
+                    mp = make_float2(-qs[0], -qs[1]);
+                }
+                ax = __ffma2_rn(dx, f, ax);
+                ay = __ffma2_rn(dy, f, ay);
+                az = __ffma2_rn(dz, f, az);
+                if (WANT_POT) np = __fadd2_rn(np, mp);
+            }
+            add_partial(ax, ay, az, np);
+            __syncwarp();
+        };
+
+        auto some_put = [&](int pos, double x, double y, double z, float m, unsigned groups) {
+            float* o = LS + pos;
+            const float fx = (float)x, fy = (float)y, fz = (float)z;
+            o[0] = fx; o[kPackSome] = fy; o[2 * kPackSome] = fz;
+            o[3 * kPackSome] = (float)(x - (double)fx);
+            o[4 * kPackSome] = (float)(y - (double)fy);
+            o[5 * kPackSome] = (float)(z - (double)fz);
+            o[6 * kPackSome] = m;
+            o[7 * kPackSome] = __uint_as_float(groups);
+        };
+
+        // ---- traversal: walk_pair_kernel's loop -------------------------------------------------
+        int top = 1;
+        if (!A.group_root) {
+            if (lane == 0) stk[0] = (int)full;
+        } else {
+            // in a forest, one entry per root that the pack's groups start from
+            const int r = lane < G ? A.group_root[pk.x + lane] : -1 - lane;
+            const unsigned same = __match_any_sync(kFull, r);
+            const bool lead = lane < G && (same & lt_mask) == 0u;
+            const unsigned lm = __ballot_sync(kFull, lead);
+            if (lead) stk[__popc(lm & lt_mask)] = (int)(((unsigned)r << kPackGroups) | same);
+            top = __popc(lm);
+        }
+        __syncwarp();
+        int na = 0, ns = 0, nn = 0;
+        int base = 0, qtot = 0;  // the opened leaves' particles still to place: [base, qtot)
+        bool overflow = false;
+        for (;;) {
+            const bool done = top == 0 && base >= qtot;
+            if (na > 0 && (done || na > kPackAll - 32)) { flush_all(na); na = 0; }
+            if (ns > 0 && (done || ns > kPackSome - 32)) { flush_some(ns); ns = 0; }
+            if (nn > 0 && (done || nn > kPackNear - 32)) { flush_near(nn); nn = 0; }
+            if (done) break;
+
+            if (base < qtot) {
+                // 32 particles of opened leaves: those farther from the pack's box than max(largest
+                // target softening, their own) are monopoles for the groups that opened their leaf
+                const int q = base + lane;
+                double qx = 0, qy = 0, qz = 0;
+                float qm = 0.0f, qh = 0.0f;
+                unsigned gm = 0;
+                bool far = false;
+                double g2 = 0.0;
+                if (q < qtot) {
+                    int l = 0;
+#pragma unroll
+                    for (int step = 16; step > 0; step >>= 1)
+                        if (S.pre[l + step] <= q) l += step;
+                    int qpos = S.lo[l] + (q - S.pre[l]);
+                    if (!GT_IN_BOUNDS(qpos, A.n_src)) qpos = 0;
+                    load_src(A.src + qpos, qx, qy, qz, qm, qh);
+                    gm = (unsigned)S.msk[l];
+                    const double ex = box_gap(qx, S.all.c_x, S.all.w_x);
+                    const double ey = box_gap(qy, S.all.c_y, S.all.w_y);
+                    const double ez = box_gap(qz, S.all.c_z, S.all.w_z);
+                    const double qhd = (double)qh;
+                    const double reach = S.all.emax > qhd ? S.all.emax : qhd;
+                    g2 = ex * ex + ey * ey + ez * ez;
+                    far = g2 > reach * reach;
+                }
+                const double rx = qx - S.all.c_x, ry = qy - S.all.c_y, rz = qz - S.all.c_z;
+                const float ex = (float)rx, ey = (float)ry, ez = (float)rz;
+                const bool one = far && gm == full && g2 >= S.all.amin;  // one float per axis is enough
+                const unsigned am = __ballot_sync(kFull, one), sm = __ballot_sync(kFull, far && !one);
+                const unsigned nm = __ballot_sync(kFull, gm != 0 && !far);
+                if (one && GT_IN_BOUNDS(na + __popc(am & lt_mask), kPackAll)) {
+                    float* o = LA + na + __popc(am & lt_mask);
+                    o[0] = ex; o[kPackAll] = ey; o[2 * kPackAll] = ez; o[3 * kPackAll] = qm;
+                } else if (far && GT_IN_BOUNDS(ns + __popc(sm & lt_mask), kPackSome)) {
+                    some_put(ns + __popc(sm & lt_mask), rx, ry, rz, qm, gm);
+                } else if (gm != 0 && GT_IN_BOUNDS(nn + __popc(nm & lt_mask), kPackNear)) {
+                    float* o = LN + nn + __popc(nm & lt_mask);
+                    o[0] = ex; o[kPackNear] = ey; o[2 * kPackNear] = ez;
+                    o[3 * kPackNear] = (float)(rx - (double)ex);
+                    o[4 * kPackNear] = (float)(ry - (double)ey);
+                    o[5 * kPackNear] = (float)(rz - (double)ez);
+                    o[6 * kPackNear] = qm; o[7 * kPackNear] = qh; o[8 * kPackNear] = __uint_as_float(gm);
+                }
+                na += __popc(am);
+                ns += __popc(sm);
+                nn += __popc(nm);
+                base += 32;
+                __syncwarp();
+                continue;
+            }
+
+            const int npop = min(top, 32);
+            top -= npop;
+            const unsigned ent = lane < npop ? (unsigned)stk[top + lane] : 0u;
+            int node = (int)(ent >> kPackGroups);
+            unsigned mk = ent & 0xffu;
+            if (!GT_IN_BOUNDS(node, A.n_nodes)) { node = 0; mk = 0; }
+            __syncwarp();
+            const NodeV nd = load_node(A.nodes + node);
+            const bool leaf = nd.first < 0;
+            const double len = (double)nd.len, lim = 0.6 * len;
+            const double ml2 = MAC == 2 ? nd.mass * (double)__ldg(A.mac_l2 + node) : nd.mass * len * len;
+            unsigned om = 0;  // the groups that open this node
+#pragma unroll 1
+            for (int v = 0; v < G; ++v) {
+                if (!((mk >> v) & 1u)) continue;
+                const double dx = box_gap(nd.cx, S.wb[v].c_x, S.wb[v].w_x);
+                const double dy = box_gap(nd.cy, S.wb[v].c_y, S.wb[v].w_y);
+                const double dz = box_gap(nd.cz, S.wb[v].c_z, S.wb[v].w_z);
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                if (open_node(r2, len, nd.s, ml2, (double)nd.soft, S.wb[v].emax, S.wb[v].amin, A.theta2, dx, dy, dz))
+                    om |= 1u << v;
+            }
+            const unsigned acc = mk & ~om;
+            const bool push = om != 0 && !leaf, expand = om != 0 && leaf;
+            const int nch = push ? nd.nchild : 0;
+            const int cnt = expand ? nd.phi - nd.plo : 0;
+            int incl, inc2;
+            if (!__any_sync(kFull, cnt >= (1 << 16))) {
+                const int both = warp_incl_scan_i(nch | (cnt << 10));
+                incl = both & 1023;
+                inc2 = both >> 10;
+            } else {
+                incl = warp_incl_scan_i(nch);
+                inc2 = warp_incl_scan_i(cnt);
+            }
+            const int tot = __shfl_sync(kFull, incl, 31);
+            if (top + tot > A.stack_cap) { overflow = true; break; }
+            {
+                int* dst = stk + (top + incl - nch);
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    if (c < nch) dst[c] = (int)(((unsigned)(nd.first + c) << kPackGroups) | om);
+            }
+            top += tot;
+
+            bool one = acc == full;  // and far enough from the pack for one float per axis
+            if (one) {
+                const double ex = box_gap(nd.cx, S.all.c_x, S.all.w_x);
+                const double ey = box_gap(nd.cy, S.all.c_y, S.all.w_y);
+                const double ez = box_gap(nd.cz, S.all.c_z, S.all.w_z);
+                one = ex * ex + ey * ey + ez * ez >= S.all.amin;
+            }
+            const unsigned am = __ballot_sync(kFull, one), sm = __ballot_sync(kFull, acc != 0 && !one);
+            if (acc != 0) {
+                const double rx = nd.cx - S.all.c_x, ry = nd.cy - S.all.c_y, rz = nd.cz - S.all.c_z;
+                if (one) {
+                    if (GT_IN_BOUNDS(na + __popc(am & lt_mask), kPackAll)) {
+                        float* o = LA + na + __popc(am & lt_mask);
+                        o[0] = (float)rx; o[kPackAll] = (float)ry; o[2 * kPackAll] = (float)rz; o[3 * kPackAll] = (float)nd.mass;
+                    }
+                } else if (GT_IN_BOUNDS(ns + __popc(sm & lt_mask), kPackSome)) {
+                    some_put(ns + __popc(sm & lt_mask), rx, ry, rz, (float)nd.mass, acc);
+                }
+            }
+            na += __popc(am);
+            ns += __popc(sm);
+
+            qtot = __shfl_sync(kFull, inc2, 31);
+            base = 0;
+            if (qtot > 0) {
+                S.lo[lane] = nd.plo;
+                S.pre[lane] = inc2 - cnt;
+                S.msk[lane] = (int)om;
+            }
+            __syncwarp();
+        }
+        if (overflow) {
+            if (lane == 0) atomicExch(A.error, 1);
+            continue;
+        }
+        if (lane < nt) {
+            const int o = A.out_map ? (int)A.out_map[t0 + lane] : t0 + lane;
+            if (!GT_IN_BOUNDS(o, A.n_out)) continue;
+            if (A.ax) {
+                A.ax[o] = A.G * ((double)sx - (double)kx);
+                A.ay[o] = A.G * ((double)sy - (double)ky);
+                A.az[o] = A.G * ((double)sz - (double)kz);
+            }
+            if (WANT_POT && A.phi) A.phi[o] = A.G * pot;
+        }
+    }
+}
+
+// Packs of a group list over consecutive targets, in order: as many groups as fit kPackGroups and 32
+// targets and begin in one cell four leaf sides wide (the grandparent of the first group's first
+// leaf), so that a jump of the curve ends a pack.  One thread forms the packs of kPackRun groups (a
+// run starts a new pack): first the count, then, with the runs' offsets, the packs.
+constexpr int kPackRun = 64;
+__global__ void pack_groups_kernel(const int2* __restrict__ groups, const int* __restrict__ roots, int64_t ng,
+                                   const uint64_t* __restrict__ skey, const int* __restrict__ sleaf,
+                                   const int* __restrict__ level, int max_level, const uint32_t* __restrict__ off,
+                                   uint32_t* __restrict__ count, int2* __restrict__ packs) {
+    const int64_t runs = (ng + kPackRun - 1) / kPackRun;
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < runs; r += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t g1 = (r + 1) * kPackRun < ng ? (r + 1) * kPackRun : ng;
+        uint32_t n = 0;
+        for (int64_t g = r * kPackRun; g < g1;) {
+            const int t0 = groups[g].x;
+            const int shift = 3 * (max_level - max(level[sleaf[t0]] - 2, 0));
+            const uint64_t cell = skey[t0] >> shift;
+            int k = 1;
+            for (; k < kPackGroups && g + k < g1; ++k) {
+                const int2 q = groups[g + k];
+                if (q.y - t0 > 32 || skey[q.x] >> shift != cell || (roots && roots[g + k] != roots[g])) break;
+            }
+            if (packs) packs[off[r] + n] = make_int2((int)g, k);
+            ++n;
+            g += k;
+        }
+        if (count) count[r] = n;
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
 // Groups
 // ---------------------------------------------------------------------------------------------
 
@@ -2065,21 +2487,23 @@ constexpr ChunkEdges kChunkEdge{{0, 10, 45, 80, 93, 100}};
 
 // Chunk boundaries of a group list for the copy-overlapped walk: chunk c starts at the first group
 // whose first target is at or after nt * edges.pct[c] / 100 (rounded down to an even group when
-// the walk pairs windows, so that no pair straddles two chunks).  out: kChunks+1 pairs (group
+// the walk pairs windows, so that no pair straddles two chunks; with packs, in packs).  out: kChunks+1 pairs (group
 // index, first target).
 __global__ void chunk_bounds_kernel(const int2* __restrict__ groups, int ng, int nt, ChunkEdges edges,
-                                    int2* __restrict__ out, const uint32_t* __restrict__ ng_dev, int even) {
+                                    int2* __restrict__ out, const uint32_t* __restrict__ ng_dev, int even,
+                                    const int2* __restrict__ packs) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     if (ng_dev) ng = min(ng, (int)*ng_dev);
+    auto first = [&](int g) { return packs ? groups[packs[g].x].x : groups[g].x; };
     for (int c = 0; c <= kChunks; ++c) {
         const int64_t want = (int64_t)nt * edges.pct[c] / 100;
         int lo = 0, hi = ng;  // first g with groups[g].x >= want
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (groups[mid].x < want) lo = mid + 1; else hi = mid;
+            if (first(mid) < want) lo = mid + 1; else hi = mid;
         }
         if (even && c > 0 && c < kChunks) lo &= ~1;
-        out[c] = make_int2(lo, lo < ng ? groups[lo].x : nt);
+        out[c] = make_int2(lo, lo < ng ? first(lo) : nt);
     }
 }
 
@@ -2090,6 +2514,70 @@ int occupancy_blocks(int warps, int pn_cap) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, walk_kernel<TPL, LA, POT, CNT, MAC, XT>, warps * 32,
                                                   walk_smem(warps, MAC == 1, pn_cap, XT));
     return std::max(1, nb);
+}
+
+template <bool POT, int MAC>
+void prepare_pack() {
+    static bool done = false;
+    if (done) return;
+    check_cuda(cudaFuncSetAttribute(walk_pack_kernel<POT, MAC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kMaxWarps * kPackBytes),
+               "cudaFuncSetAttribute");
+    check_cuda(cudaFuncSetAttribute(walk_pack_kernel<POT, MAC>, cudaFuncAttributePreferredSharedMemoryCarveout, 100),
+               "cudaFuncSetAttribute");
+    done = true;
+}
+
+int pack_occupancy(int warps) {
+    prepare_pack<false, 0>();
+    int nb = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, walk_pack_kernel<false, 0>, warps * 32, (size_t)warps * kPackBytes);
+    return std::max(1, nb);
+}
+
+template <bool POT, int MAC>
+void launch_pack(gt_context* ctx, const WalkArgs& a, int blocks, int warps) {
+    prepare_pack<POT, MAC>();
+    walk_pack_kernel<POT, MAC><<<blocks, warps * 32, (size_t)warps * kPackBytes, ctx->stream>>>(a);
+    check_launch(ctx, "walk_pack_kernel");
+}
+
+void dispatch_pack(gt_context* ctx, const WalkArgs& a, int blocks, int warps, bool pot, int mac) {
+    if (mac == GT_MAC_NODE) {
+        if (pot) launch_pack<true, 2>(ctx, a, blocks, warps);
+        else launch_pack<false, 2>(ctx, a, blocks, warps);
+    } else {
+        if (pot) launch_pack<true, 0>(ctx, a, blocks, warps);
+        else launch_pack<false, 0>(ctx, a, blocks, warps);
+    }
+}
+
+// The packs of a tree's cached group list, made on the first walk that uses them (under the tree's
+// lock, complete on the device before they are published).
+void make_packs(gt_context* ctx, const gt_tree* t, gt_tree::GroupCache& c) {
+    cudaStream_t st = ctx->stream;
+    const int64_t runs = (c.n_groups + kPackRun - 1) / kPackRun;
+    uint32_t* cnt = (uint32_t*)scratch(ctx, kSlotNodeTmp1, (size_t)runs * 4);
+    uint32_t* off = (uint32_t*)scratch(ctx, kSlotNodeTmp2, (size_t)runs * 4);
+    uint32_t* total = (uint32_t*)scratch(ctx, kSlotCounters, kCtrBytes);
+    const int grid = grid1d(ctx, runs * 4);
+    auto form = [&](const uint32_t* o, uint32_t* n, int2* packs) {
+        pack_groups_kernel<<<grid, 64, 0, st>>>(c.groups, c.roots, c.n_groups, t->skey, t->sleaf, t->level,
+                                                t->opt.max_level, o, n, packs);
+        check_launch(ctx, "pack_groups_kernel");
+    };
+    form(nullptr, cnt, nullptr);
+    scan_exclusive_u32(ctx, cnt, off, runs, total);
+    const int64_t n = read_u32(ctx, total);
+    void* p = nullptr;
+    if (cudaMallocAsync(&p, (size_t)std::max<int64_t>(n, 1) * sizeof(int2), st) != cudaSuccess) {
+        cudaGetLastError();
+        throw Fail{GT_ERR_NOMEM, "cudaMallocAsync for the packs failed"};
+    }
+    form(off, nullptr, (int2*)p);
+    check_cuda(cudaStreamSynchronize(st), "sync");
+    c.packs = (int2*)p;
+    c.n_packs = n;
 }
 
 struct OutputCopy {
@@ -2132,6 +2620,14 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     int64_t ng = 0;
     const uint32_t* tpos = nullptr;
     const uint32_t* ng_dev = nullptr;  // explicit targets: the group count stays on the device
+    // Small groups over all live targets (the engine's leaves, windows of at most 16): packs of them
+    // share one traversal.  A list of explicit targets may hold groups far from one another, which
+    // share nothing and keep a warp each.
+    bool packed = all && rq.pair_windows && !xt && tpl == 1 && rq.leaf_accept && rq.mac != GT_MAC_LEARNED &&
+                  !rq.count && t->n_nodes < (1 << 24) && rq.list_capacity == 0 &&
+                  (mode == GT_GROUP_LEAF || (mode == GT_GROUP_BATCH && param <= 16));
+    int2* packs = nullptr;
+    int64_t n_packs = 0;
     if (all) {
         // the cache is shared by every context that walks this tree: look up and fill it under
         // the tree's lock, and publish a new list only once it is complete on the device
@@ -2193,6 +2689,16 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
             c.mode = mode; c.param = param; c.kmax = kmax; c.groups = groups; c.roots = roots; c.n_groups = ng;
             t->group_cache.push_back(c);
         }
+        // a pack's walk takes about twice as long as a leaf's, and there are six times fewer: with fewer
+        // than eight groups per resident warp the groups finish sooner side by side
+        packed = packed && ng >= (int64_t)8 * 24 * ctx->num_sms;
+        if (packed)
+            for (auto& c : t->group_cache)
+                if (c.mode == mode && c.param == param && c.kmax == kmax) {
+                    if (!c.packs) make_packs(ctx, t, c);
+                    packs = c.packs;
+                    n_packs = c.n_packs;
+                }
     } else {
         uint32_t* tp = (uint32_t*)scratch(ctx, kSlotGroupKey, (size_t)nt * 4);
         uint32_t* flag = (uint32_t*)scratch(ctx, kSlotTargets, (size_t)nt * 4);
@@ -2254,10 +2760,12 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
                         rq.leaf_accept && !mac && t->n_nodes < (1 << 29) && pn_cap <= kPairCapMax;
     if (paired && rq.list_capacity == 0) pn_cap = kPairCapDefault;
     // the largest lists leave room for fewer warps in a block's shared memory
-    if (!paired)
+    if (!paired && !packed)
         while (warps > 1 && walk_smem(warps, mac, pn_cap, ext) > kMaxSmem) --warps;
     int per_sm;
-    if (paired)
+    if (packed)
+        per_sm = pack_occupancy(warps);
+    else if (paired)
         per_sm = macn ? pair_occupancy<false, false, 2>(warps, pn_cap) : pair_occupancy<false, false, 0>(warps, pn_cap);
     else if (ext == 1)
         per_sm = occupancy_blocks<1, true, false, false, 0, 1>(warps, pn_cap);
@@ -2290,7 +2798,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         hand_cap = (int)std::min<int64_t>(units, kHandRecords);
         budget = tree_units <= kHandRecords ? 96 : 192;
     }
-    const int64_t want_blocks = ((paired ? (ng + 1) / 2 : ng) + warps - 1) / warps;
+    const int64_t want_blocks = ((paired ? (ng + 1) / 2 : packed ? n_packs : ng) + warps - 1) / warps;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want_blocks, (int64_t)per_sm * ctx->num_sms));
     // a breadth-first stack of a long window lies below the depth-first levels
     int stack_cap = rq.stack_capacity > 0 ? rq.stack_capacity : 256 * std::max(1, t->n_levels) + 32;
@@ -2351,6 +2859,8 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     } else {
         ctr = (unsigned long long*)scratch(ctx, kSlotCounters, kCtrBytes);
     }
+    a.packs = packs;
+    a.n_packs = (int)n_packs;
     a.budget = budget;
     a.hand_cap = hand_cap;
     a.hand_size = (int)std::max<int64_t>(64, t->n_live / t->n_systems / 256);
@@ -2404,7 +2914,8 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         ensure_copy_stream(ctx);
         int2* bounds = (int2*)(ctr + 16);  // K+1 int2 after the counters
         check_cuda(cudaMemsetAsync(ctr, 0, kCtrBytes, st), "memset counters");
-        chunk_bounds_kernel<<<1, 1, 0, st>>>(groups, (int)ng, (int)nt, kChunkEdge, bounds, ng_dev, paired ? 1 : 0);
+        chunk_bounds_kernel<<<1, 1, 0, st>>>(groups, (int)(packed ? n_packs : ng), (int)nt, kChunkEdge, bounds, ng_dev,
+                                             paired ? 1 : 0, packs);
         check_launch(ctx, "chunk_bounds_kernel");
         int2 hb[kChunks + 1];
         check_cuda(cudaMemcpyAsync(ctx->pinned, bounds, sizeof(hb), cudaMemcpyDeviceToHost, st), "d2h");
@@ -2481,14 +2992,20 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
                 ac.stack = stacks[c & 1];
                 ac.hand = hands[c & 1];
                 ac.hand_ctr = (unsigned int*)(ctr + kCtrHand + c);
-                ac.groups = groups + g0;
-                ac.n_groups = g1 - g0;
-                ac.n_groups_dev = nullptr;
-                ac.group_root = roots ? roots + g0 : nullptr;
+                if (packed) {
+                    ac.packs = packs + g0;
+                    ac.n_packs = g1 - g0;
+                } else {
+                    ac.groups = groups + g0;
+                    ac.n_groups = g1 - g0;
+                    ac.n_groups_dev = nullptr;
+                    ac.group_root = roots ? roots + g0 : nullptr;
+                }
                 ac.next_group = (unsigned int*)(ctr + 10) + c;
                 const int64_t units = paired ? ((int64_t)(g1 - g0) + 1) / 2 : (int64_t)(g1 - g0);
                 const int cb = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (units + warps - 1) / warps));
                 if (paired) dispatch_pair(ctx, ac, cb, warps, want_pot, false, rq.mac);
+                else if (packed) dispatch_pack(ctx, ac, cb, warps, want_pot, rq.mac);
                 else if (xt) dispatch_xt(ctx, ac, cb, warps, ext, rq.leaf_accept, want_pot, false);
                 else if (tpl == 1) dispatch<1>(ctx, ac, cb, warps, rq.leaf_accept, want_pot, false, rq.mac);
                 else if (tpl == 2) dispatch<2>(ctx, ac, cb, warps, rq.leaf_accept, want_pot, false, rq.mac);
@@ -2543,6 +3060,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         check_cuda(cudaMemsetAsync(ctr, 0, kCtrBytes, st), "memset counters");
         if (!rq.capture) check_cuda(cudaEventRecord(ctx->ev0, st), "event");
         if (paired) dispatch_pair(ctx, a, blocks, warps, want_pot, rq.count, rq.mac);
+        else if (packed) dispatch_pack(ctx, a, blocks, warps, want_pot, rq.mac);
         else if (xt) dispatch_xt(ctx, a, blocks, warps, ext, rq.leaf_accept, want_pot, rq.count);
         else if (tpl == 1) dispatch<1>(ctx, a, blocks, warps, rq.leaf_accept, want_pot, rq.count, rq.mac);
         else if (tpl == 2) dispatch<2>(ctx, a, blocks, warps, rq.leaf_accept, want_pot, rq.count, rq.mac);

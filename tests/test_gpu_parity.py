@@ -347,6 +347,42 @@ def test_long_windows_handed_over(gpu_ctx, oracle, n):
     assert np.median(e) <= 1e-6 and e.max() <= 1e-4
 
 
+@pytest.mark.parametrize("ics_kind", ["plummer", "clumps", "collocated"])
+@pytest.mark.parametrize("batch", [0, 5, 8, 16])
+def test_packs_match_single_groups(gpu_ctx, ics_kind, batch):
+    """Leaf groups and small windows over all particles share traversals in packs of up to eight groups
+    and 32 targets where there are enough of them (200,000 particles here): the same walk with one
+    group per warp (window_pairs=False) agrees to FP32 summation, accelerations and potential, in both
+    output orders, with clumps and jumps of the Morton curve between them, and with 40 particles in one
+    place, whose level-20 leaf is longer than a pack.  1e-6 is some ten roundings of 6e-8."""
+    rng = np.random.default_rng(batch + 1)
+    P = ics.plummer(n=200000, seed=batch + 3)
+    if ics_kind == "clumps":
+        for k in ("x", "y", "z"):
+            P[k] = 0.01 * P[k] + rng.integers(0, 4, 200000) * 2.0
+    if ics_kind == "collocated":
+        for k in ("x", "y", "z"):
+            P[k][1000:1040] = P[k][1000]
+    T = gpu_ctx.build(P, key_mode=g.GT_KEY_MORTON)
+    kw = dict(theta=0.7, batch=batch, group_mode=g.GT_GROUP_BATCH if batch else g.GT_GROUP_LEAF, want_phi=True)
+    a = gpu_ctx.accel_grouped(T, None, **kw)
+    b = gpu_ctx.accel_grouped(T, None, window_pairs=False, **kw)
+    aold = gpu_ctx.form_aold(*b[:3], 0.0025)
+    kw["theta"] = 0.0
+    c = gpu_ctx.accel_grouped(T, None, aold=aold, **kw)
+    d = gpu_ctx.accel_grouped(T, None, aold=aold, window_pairs=False, **kw)
+    o = gpu_ctx.accel_grouped(T, None, aold=aold, out_order=g.GT_OUT_ORIGINAL, **kw)
+    ob = T.download(nodes=False)["orderbuf"]
+    for p, q in ((a, b), (c, d)):
+        e = relerr(*p[:3], *q[:3])
+        assert np.median(e) <= 3e-7 and np.quantile(e, 0.999) <= 1e-4
+        n = np.sqrt(sum((x - y) ** 2 for x, y in zip(p[:3], q[:3])).sum() / sum(y ** 2 for y in q[:3]).sum())
+        assert n <= 1e-6
+        assert np.median(np.abs(p[3] / q[3] - 1)) <= 1e-6
+    for k in range(4):
+        assert np.array_equal(o[k][ob], c[k])
+
+
 # ---- direct sum -----------------------------------------------------------------------------
 
 def test_direct_fp64_and_fp32(gpu_ctx, oracle, plummer):
