@@ -128,22 +128,25 @@ __device__ __forceinline__ bool is_neighbour(const SearchGeom& g, int s, double 
 
 // One traversal for one centre in the reference's node order, from roots r0 .. r1-1 in turn.
 // REVERSE: gas particles j < n_gas with radius <= r < h[j] (ngb_search_reverse); otherwise
-// r < radius (ngb_search).  emit(s) receives the tree position; false ends the search.
+// r < radius (ngb_search).  emit(s) receives the tree position; false ends the search.  Every lane of
+// mask calls it, each for its own centre.
 //
 // A thread follows the threading alone, so what bounds the search is how many of a warp's lanes do
 // the same thing at once.  Opening each leaf where the traversal meets it kept 5.5 of 32 lanes
 // active: the lanes reach their leaves at different steps, and every leaf held up the whole warp.
 // Here the traversal only notes the leaves it opens (kLeafBuf of them, in thread-local memory, which
 // the hardware interleaves across the warp); then every lane runs through the particles of its own
-// leaves in one flat loop, a particle an iteration, and the traversal goes on.  Both loops keep
-// nearly all lanes busy, because neighbouring targets visit nearly as many nodes and particles.
+// leaves in one flat loop, a particle an iteration, and the traversal goes on.  The lanes are brought
+// together after each loop: left to themselves they go on from their own last iteration, and two in
+// 32 were active by the time the neighbours' sums were formed.
 // The prune is the reference's box and circumsphere test in FP32, widened by the rounding of the
 // centre, the distances and the squares, so it never drops a node that the FP64 test keeps; the
 // particle test decides in FP64, so the lists are the same, in the same order.
 constexpr int kLeafBuf = 32;
 template <bool REVERSE, typename F>
 __device__ __forceinline__ void search(const SearchGeom& g, int r0, int r1, double px, double py, double pz,
-                                       double radius, const double* __restrict__ h, int64_t n_gas, F&& emit) {
+                                       double radius, const double* __restrict__ h, int64_t n_gas, unsigned mask,
+                                       F&& emit) {
     const double r2max = radius * radius;
     const float fx = (float)px, fy = (float)py, fz = (float)pz;
     const float fbox = (float)g.box, fhalf = 0.5f * fbox;
@@ -160,43 +163,47 @@ __device__ __forceinline__ void search(const SearchGeom& g, int r0, int r1, doub
         return s;
     };
     int2 leaf[kLeafBuf];
-    for (int root = r0; root < r1; ++root) {
-        int node = root;
-        while (node >= 0) {
-            int nl = 0;
-            while (node >= 0 && nl < kLeafBuf) {
-                const float4 a = __ldg(reinterpret_cast<const float4*>(g.sn + node));
-                const int4 b = __ldg(reinterpret_cast<const int4*>(g.sn + node) + 1);
-                float dist = reach + a.w;
-                bool keep = true;
-                if (REVERSE) {
-                    const float hm = __ldg(g.hmax + node);
-                    keep = !((double)hm <= radius);
-                    dist += hm;
-                }
-                if (g.xpad) dist += __ldg(g.xpad + node);
-                if (moving) dist = fmaf(__ldg(g.vmax + node), felapsed, dist);
-                dist *= 1.000002f;
-                const float dx = image(a.x - fx), dy = image(a.y - fy), dz = image(a.z - fz);
-                const float ball = fmaf(0.73205090f, a.w, dist) * 1.000002f;
-                keep = keep && !(fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz))) > dist) &&
-                       !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > ball * ball);
-                if (keep && b.x < 0) leaf[nl++] = make_int2(b.z, b.w);
-                node = keep && b.x >= 0 ? b.x : b.y;
+    int root = r0, node = r0 < r1 ? r0 : -1;
+    while (__any_sync(mask, node >= 0)) {
+        int nl = 0;
+        while (node >= 0 && nl < kLeafBuf) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(g.sn + node));
+            const int4 b = __ldg(reinterpret_cast<const int4*>(g.sn + node) + 1);
+            float dist = reach + a.w;
+            bool keep = true;
+            if (REVERSE) {
+                const float hm = __ldg(g.hmax + node);
+                keep = !((double)hm <= radius);
+                dist += hm;
             }
-            int s = 0, e = 0, li = 0;
-            for (;;) {
-                while (s >= e && li < nl) {
-                    s = leaf[li].x;
-                    e = leaf[li].y;
-                    ++li;
-                }
-                if (s >= e) break;
-                uint32_t j = 0;
-                if (is_neighbour<REVERSE>(g, s, px, py, pz, r2max, h, n_gas, j) && !emit(s)) return;
-                ++s;
-            }
+            if (g.xpad) dist += __ldg(g.xpad + node);
+            if (moving) dist = fmaf(__ldg(g.vmax + node), felapsed, dist);
+            dist *= 1.000002f;
+            const float dx = image(a.x - fx), dy = image(a.y - fy), dz = image(a.z - fz);
+            const float ball = fmaf(0.73205090f, a.w, dist) * 1.000002f;
+            keep = keep && !(fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz))) > dist) &&
+                   !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > ball * ball);
+            if (keep && b.x < 0) leaf[nl++] = make_int2(b.z, b.w);
+            node = keep && b.x >= 0 ? b.x : b.y;
+            if (node < 0 && ++root < r1) node = root;  // the next root, where there is one
         }
+        __syncwarp(mask);
+        int s = 0, e = 0, li = 0;
+        for (;;) {
+            while (s >= e && li < nl) {
+                s = leaf[li].x;
+                e = leaf[li].y;
+                ++li;
+            }
+            if (s >= e) break;
+            uint32_t j = 0;
+            if (is_neighbour<REVERSE>(g, s, px, py, pz, r2max, h, n_gas, j) && !emit(s)) {
+                node = -1;  // ended by the caller
+                break;
+            }
+            ++s;
+        }
+        __syncwarp(mask);
     }
 }
 
@@ -288,11 +295,16 @@ template <bool FILL, bool COUNT>
 __global__ void __launch_bounds__(kBlk) ngb_kernel(const NgbArgs a) {
     unsigned long long mine = 0, calls = 0, kept = 0, over = 0;
     NgbTally tl;
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); c0 < a.n; c0 += step) {
+        const int64_t c = c0 + (threadIdx.x & 31);
+        // lists within the cache's room are copied from there
+        const bool have = c < a.n && !(FILL && a.kcache > 0 && a.count[c] <= (uint32_t)a.kcache);
+        const unsigned mask = __ballot_sync(0xffffffffu, have);
+        if (!have) continue;
         const double px = a.cx[c], py = a.cy[c], pz = a.cz[c], r = a.radius[c];
         int r0, r1;
         roots_of(a.g, a.systems, c, r0, r1, FILL ? nullptr : a.total + 1);
-        if (FILL && a.kcache > 0 && a.count[c] <= (uint32_t)a.kcache) continue;  // copied from the cache
         int64_t k = FILL ? a.start[c] : 0;
         auto emit = [&](int s) {
             if (FILL) a.found[k] = __ldg(a.g.order + s);
@@ -302,19 +314,21 @@ __global__ void __launch_bounds__(kBlk) ngb_kernel(const NgbArgs a) {
         };
         if (a.mode != GT_NGB_REVERSE) {
             if (COUNT) search_counted(a.g, r0, r1, px, py, pz, r, emit, &tl);
-            else search<false>(a.g, r0, r1, px, py, pz, r, nullptr, 0, emit);
+            else search<false>(a.g, r0, r1, px, py, pz, r, nullptr, 0, mask, emit);
             if (COUNT) {
                 ++calls;
                 kept += (unsigned long long)k;
             }
         }
-        if (a.mode != GT_NGB_GATHER) search<true>(a.g, r0, r1, px, py, pz, r, a.h, a.n_gas, emit);
+        if (COUNT) __syncwarp(mask);
+        if (a.mode != GT_NGB_GATHER) search<true>(a.g, r0, r1, px, py, pz, r, a.h, a.n_gas, mask, emit);
         if (!FILL) {
             a.count[c] = (uint32_t)k;
             mine += (unsigned long long)k;
             over += k > a.kcache ? 1ull : 0ull;
         }
     }
+    __syncwarp();
     if (!FILL) {
         warp_flush(mine, a.total);
         warp_flush(over, a.total + 2);
@@ -411,37 +425,51 @@ __device__ __forceinline__ void dens_zero(DensSums& s) {
 // weight w and dW/dh.  Every rounding is spelled out, so that the solve's forms -- a thread per target
 // and a warp per target -- add the same terms in the same order and agree to the last bit.
 struct DensNorm {
-    double h, norm, dnorm;  // dnorm: -dim / h of the kernel's norm
+    double h, hinv, norm, dnorm;  // dnorm: -dim / h of the kernel's norm
+    bool plain;                   // h is far from the ends of the FP64 range
 };
 __device__ __forceinline__ DensNorm dens_norm(double h, int dim) {
     const double norm = kernel_norm(h, dim);
-    return DensNorm{h, norm, __dmul_rn(-((double)dim / h), norm)};
+    return DensNorm{h, 1.0 / h, norm, __dmul_rn(-((double)dim / h), norm), h > 1e-100 && h < 1e100};
 }
+
+// x / h from the rounded reciprocal of h: the quotient's remainder is exact in one fused operation and
+// corrects it (Markstein's division), three instructions where a division takes a dozen and a branch.
+__device__ __forceinline__ double over_h(double x, const DensNorm& n) {
+    if (!n.plain) return x / n.h;
+    const double q = __dmul_rn(x, n.hinv);
+    return __fma_rn(__fma_rn(-n.h, q, x), n.hinv, q);
+}
+
+// The square root of r2 from its reciprocal square root: y by the approximation and one step of the
+// binomial series (gt_direct.cu, rsqrt_d), then s = r2 y corrected by the exact remainder r2 - s^2.
+__device__ __forceinline__ double root_of(double r2) {
+    if (!(r2 > 1e-280 && r2 < 1e280)) return r2 == 0.0 ? 0.0 : sqrt(r2);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+    const double e = __fma_rn(-r2, __dmul_rn(y, y), 1.0);
+    y = __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
+    const double s = __dmul_rn(r2, y);
+    return __fma_rn(__fma_rn(-s, s, r2), __dmul_rn(0.5, y), s);
+}
+
 __device__ __forceinline__ void dens_terms(double dx, double dy, double dz, const DensNorm& n, double& w, double& dh,
                                            bool& inside) {
-    const double r = sqrt(__fma_rn(dz, dz, __fma_rn(dx, dx, __dmul_rn(dy, dy))));
-    const double q = r / n.h;
-    w = dh = 0.0;
-    if (q < 1.0) {
-        double f, fp;  // the spline and its derivative
-        if (q < 0.5) {
-            const double q6 = __dmul_rn(6.0, q), q66 = __dmul_rn(q6, q);
-            f = __fma_rn(q66, q, __dadd_rn(1.0, -q66));
-            fp = __fma_rn(__dmul_rn(18.0, q), q, __dmul_rn(-12.0, q));
-        } else {
-            const double u = __dadd_rn(1.0, -q);
-            f = __dmul_rn(__dmul_rn(__dmul_rn(2.0, u), u), u);
-            fp = __dmul_rn(__dmul_rn(-6.0, u), u);
-        }
-        w = __dmul_rn(n.norm, f);
-        dh = __fma_rn(-__dmul_rn(q / n.h, n.norm), fp, __dmul_rn(n.dnorm, f));
-    }
+    const double r = root_of(__fma_rn(dz, dz, __fma_rn(dx, dx, __dmul_rn(dy, dy))));
+    const double q = over_h(r, n);
+    // the spline and its derivative on either side of q = 1/2, without a branch
+    const double q6 = __dmul_rn(6.0, q), q66 = __dmul_rn(q6, q);
+    const double u = __dadd_rn(1.0, -q);
+    const bool low = q < 0.5;
+    const double f = low ? __fma_rn(q66, q, __dadd_rn(1.0, -q66)) : __dmul_rn(__dmul_rn(__dmul_rn(2.0, u), u), u);
+    const double fp = low ? __fma_rn(__dmul_rn(18.0, q), q, __dmul_rn(-12.0, q)) : __dmul_rn(__dmul_rn(-6.0, u), u);
+    const bool some = q < 1.0;
+    w = some ? __dmul_rn(n.norm, f) : 0.0;
+    dh = some ? __fma_rn(-__dmul_rn(over_h(q, n), n.norm), fp, __dmul_rn(n.dnorm, f)) : 0.0;
     inside = r < n.h;
 }
-__device__ __forceinline__ void dens_add(double dx, double dy, double dz, double m, const DensNorm& n, DensSums& s) {
-    double w, dh;
-    bool inside;
-    dens_terms(dx, dy, dz, n, w, dh, inside);
+__device__ __forceinline__ void dens_sum(double dx, double dy, double dz, double m, double w, double dh, bool inside,
+                                         DensSums& s) {
     s.wsum = __dadd_rn(s.wsum, w);
     s.dwdh = __dadd_rn(s.dwdh, dh);
     s.rho = __fma_rn(m, w, s.rho);
@@ -455,6 +483,12 @@ __device__ __forceinline__ void dens_add(double dx, double dy, double dz, double
     s.face[1] = __fma_rn(dy, w, s.face[1]);
     s.face[2] = __fma_rn(dz, w, s.face[2]);
     if (inside) ++s.inside;
+}
+__device__ __forceinline__ void dens_add(double dx, double dy, double dz, double m, const DensNorm& n, DensSums& s) {
+    double w, dh;
+    bool inside;
+    dens_terms(dx, dy, dz, n, w, dh, inside);
+    dens_sum(dx, dy, dz, m, w, dh, inside, s);
 }
 
 // One evaluation at h: the sums over the GAS neighbours inside h, in tree order (hydro.cc:205-222).
@@ -470,7 +504,7 @@ constexpr double kCacheGrow = 1.4;
 
 template <bool COUNT>
 __device__ __noinline__ void dens_eval(const DensArgs& a, int r0, int r1, double px, double py, double pz, double h, DensSums& s,
-                          NgbTally& tl, unsigned long long& kept) {
+                          NgbTally& tl, unsigned long long& kept, unsigned mask) {
     dens_zero(s);
     const DensNorm nrm = dens_norm(h, a.n_dims);
     int buf[kDensBuf];
@@ -493,7 +527,7 @@ __device__ __noinline__ void dens_eval(const DensArgs& a, int r0, int r1, double
         return true;
     };
     if (COUNT) search_counted(a.g, r0, r1, px, py, pz, h, found, &tl);
-    else search<false>(a.g, r0, r1, px, py, pz, h, nullptr, 0, found);
+    else search<false>(a.g, r0, r1, px, py, pz, h, nullptr, 0, mask, found);
     drain();
 }
 
@@ -505,10 +539,10 @@ __device__ __noinline__ void dens_eval(const DensArgs& a, int r0, int r1, double
 // and an iteration that shrinks h costs a scan of a few dozen candidates instead of a traversal.
 // A search that finds more than cand_cap gas particles ends there and returns -1.
 __device__ __forceinline__ int cache_fill(const DensArgs& a, int r0, int r1, double px, double py, double pz,
-                                          double R, uint32_t* __restrict__ slot, int64_t stride) {
+                                          double R, uint32_t* __restrict__ slot, int64_t stride, unsigned mask) {
     int k = 0;
     const int cap = a.cand_cap;
-    search<false>(a.g, r0, r1, px, py, pz, R, nullptr, 0, [&](int sp) {
+    search<false>(a.g, r0, r1, px, py, pz, R, nullptr, 0, mask, [&](int sp) {
         if (a.stype && __ldg(a.stype + sp) != 0) return true;
         if (k < cap) slot[(int64_t)k * stride] = (uint32_t)sp;
         return ++k <= cap;
@@ -516,19 +550,44 @@ __device__ __forceinline__ int cache_fill(const DensArgs& a, int r0, int r1, dou
     return k <= cap ? k : -1;
 }
 
+// Two candidates at a time, the next two's positions on their way: what bounds the evaluation is the
+// latency of its loads and of the FP64 chains to the weights, which two independent candidates
+// overlap.  The sums take the kept ones in order.
 __device__ __forceinline__ void cache_eval(const DensArgs& a, const uint32_t* __restrict__ slot, int64_t stride, int n,
                                            double px, double py, double pz, double h, DensSums& s) {
     dens_zero(s);
     const DensNorm nrm = dens_norm(h, a.n_dims);
     const double r2max = h * h;
-    for (int k = 0; k < n; ++k) {
-        const int sp = (int)slot[(int64_t)k * stride];
+    auto at = [&](int k) { return (int)slot[(int64_t)min(k, n - 1) * stride]; };
+    auto load = [&](int sp, double& x, double& y, double& z) {
         const double2 xy = __ldg(reinterpret_cast<const double2*>(a.g.src + sp));
-        const double zz = __ldg(reinterpret_cast<const double*>(a.g.src + sp) + 2);
-        const double ox = min_image(xy.x - px, a.g.box), oy = min_image(xy.y - py, a.g.box),
-                     oz = min_image(zz - pz, a.g.box);
-        const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(ox, ox), __dmul_rn(oy, oy)), __dmul_rn(oz, oz));
-        if (r2 < r2max) dens_add(ox, oy, oz, __ldg(a.smass + sp), nrm, s);
+        x = xy.x; y = xy.y;
+        z = __ldg(reinterpret_cast<const double*>(a.g.src + sp) + 2);
+    };
+    if (n <= 0) return;
+    int s0 = at(0), s1 = at(1), s2 = at(2), s3 = at(3);
+    double x0, y0, z0, x1, y1, z1;
+    load(s0, x0, y0, z0);
+    load(s1, x1, y1, z1);
+    for (int k = 0; k < n; k += 2) {
+        const double m0 = __ldg(a.smass + s0), m1 = __ldg(a.smass + s1);
+        const double dx0 = min_image(x0 - px, a.g.box), dy0 = min_image(y0 - py, a.g.box), dz0 = min_image(z0 - pz, a.g.box);
+        const double dx1 = min_image(x1 - px, a.g.box), dy1 = min_image(y1 - py, a.g.box), dz1 = min_image(z1 - pz, a.g.box);
+        s0 = s2; s1 = s3;
+        s2 = at(k + 4); s3 = at(k + 5);
+        load(s0, x0, y0, z0);
+        load(s1, x1, y1, z1);
+        const double r0 = __dadd_rn(__dadd_rn(__dmul_rn(dx0, dx0), __dmul_rn(dy0, dy0)), __dmul_rn(dz0, dz0));
+        const double r1 = __dadd_rn(__dadd_rn(__dmul_rn(dx1, dx1), __dmul_rn(dy1, dy1)), __dmul_rn(dz1, dz1));
+        const bool keep0 = r0 < r2max, keep1 = k + 1 < n && r1 < r2max;
+        if (keep0 || keep1) {
+            double w0, e0, w1, e1;
+            bool in0, in1;
+            dens_terms(dx0, dy0, dz0, nrm, w0, e0, in0);
+            dens_terms(dx1, dy1, dz1, nrm, w1, e1, in1);
+            if (keep0) dens_sum(dx0, dy0, dz0, m0, w0, e0, in0, s);
+            if (keep1) dens_sum(dx1, dy1, dz1, m1, w1, e1, in1, s);
+        }
     }
 }
 
@@ -639,12 +698,12 @@ __global__ void __launch_bounds__(kBlk, 6) density_count_kernel(const DensArgs a
         bool converged = false;
         DensSums s;
         for (; iter < 100; ++iter) {
-            dens_eval<true>(a, r0, r1, px, py, pz, h, s, tl, kept);
+            dens_eval<true>(a, r0, r1, px, py, pz, h, s, tl, kept, 0u);
             ++calls;
             if (dens_newton(newton_params(a), p, s, iter, h, h_lo, h_hi)) { converged = true; break; }
         }
         if (!converged) {  // rho of the final h (hydro.cc:281-293)
-            dens_eval<true>(a, r0, r1, px, py, pz, h, s, tl, kept);
+            dens_eval<true>(a, r0, r1, px, py, pz, h, s, tl, kept, 0u);
             ++calls;
         }
         ++hist[min(converged ? iter + 1 : 100, 8) - 1];
@@ -664,17 +723,20 @@ __global__ void __launch_bounds__(kBlk, 6) density_count_kernel(const DensArgs a
 // The solve: a lane per target, refilled as targets finish.
 //
 // The targets of a warp take between 1 and 10 iterations, three on average, so with a target per
-// thread for good most lanes waited for the slowest: 6 of 32 were active.  Here a warp takes kRun
-// consecutive targets at a time and its lanes are a pool: a lane whose target is done takes the next
-// one.  The loop's two phases each run for as many lanes at once as can be gathered: the search that
-// fills a lane's candidate cache (a new target, or an h that outgrew the cache) waits until
-// kGather lanes want it or nobody can do anything else, and an evaluation with its Newton step runs
-// for every lane that holds candidates.  Each target's own sequence of searches, sums and steps is
-// that of the counting solve's thread, so its results are the same bits whichever lane it gets.
+// thread for good most lanes waited for the slowest.  Here a warp takes a run of consecutive targets
+// at a time and its lanes are a pool: a lane whose target is done takes the next one.  The loop's two
+// phases each run for as many lanes at once as can be gathered: the search that fills a lane's
+// candidate cache (a new target, or an h that outgrew the cache) waits until kGather lanes are idle or
+// want it, or nobody can do anything else, and an evaluation with its Newton step runs for every lane
+// that holds candidates.  Each target's own sequence of searches, sums and steps is that of the
+// counting solve's thread, so its results are the same bits whichever lane it gets.  Warm solve of a
+// 2^20 galaxy, lengths 5 % off: 26.0 ms before leaves were collected (search) and crowded targets
+// went to warps, 14.2 then, 13.2 with the square root and quotients of dens_terms, 12.2 with two
+// candidates at a time and the four blocks per SM whose registers that needs (six spill: 13.5).
 // ONE_ROOT: a single-system tree, whose one root (node 0) the compiler then knows.
 constexpr int kGather = 16;
 template <bool ONE_ROOT>
-__global__ void __launch_bounds__(kBlk, 6) density_kernel(const DensArgs a) {
+__global__ void __launch_bounds__(kBlk, 4) density_kernel(const DensArgs a) {
     const int lane = threadIdx.x & 31;
     uint32_t* __restrict__ slot = a.cand + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
     unsigned next = 0, end = 0;  // the warp's run of targets still to take
@@ -686,7 +748,8 @@ __global__ void __launch_bounds__(kBlk, 6) density_kernel(const DensArgs a) {
     for (;;) {
         // idle lanes take targets
         const unsigned idle = __ballot_sync(0xffffffffu, t < 0);
-        if (__popc(idle) >= kGather && (more || next < end)) {
+        const unsigned out = __ballot_sync(0xffffffffu, t < 0 || (!ready_now && !(R >= h)));  // idle or to search
+        if (idle != 0u && __popc(out) >= kGather && (more || next < end)) {
             if (next >= end) {
                 if (lane == 0) next = atomicAdd(a.heavy_ctr + 2, (unsigned)a.run);
                 next = __shfl_sync(0xffffffffu, next, 0);
@@ -721,7 +784,7 @@ __global__ void __launch_bounds__(kBlk, 6) density_kernel(const DensArgs a) {
         if (__popc(wants) >= kGather || ready == 0u) {
             if (want) {
                 const double rad = (R < 0 ? kCacheFirst : kCacheGrow) * h;
-                ncand = cache_fill(a, r0, r1, px, py, pz, rad, slot, a.n_threads);
+                ncand = cache_fill(a, r0, r1, px, py, pz, rad, slot, a.n_threads, wants);
                 R = rad;
                 ready_now = true;
                 if (ncand < 0) {
@@ -740,13 +803,16 @@ __global__ void __launch_bounds__(kBlk, 6) density_kernel(const DensArgs a) {
         }
         if (have && !want) {
             DensSums s;
+            // (no lane searches directly unless the hand-over list is full)
+            const unsigned straight = __ballot_sync(ready, direct);
             if (direct) {
                 NgbTally none;
                 unsigned long long kept = 0;
-                dens_eval<false>(a, r0, r1, px, py, pz, h, s, none, kept);
+                dens_eval<false>(a, r0, r1, px, py, pz, h, s, none, kept, straight);
             } else {
                 cache_eval(a, slot, a.n_threads, ncand, px, py, pz, h, s);
             }
+            __syncwarp(ready);
             // after 100 steps, the sums of the final h (hydro.cc:281-293)
             if (iter == 100 || dens_newton(newton_params(a), a.targets[t], s, iter, h, h_lo, h_hi)) {
                 a.h[t] = h;
@@ -1130,7 +1196,7 @@ void run_density(gt_context* ctx, gt_tree* t, int64_t nt, const uint32_t* target
     a.warp_cand = nullptr;
     a.heavy_cap = 0;
     a.run = 32;
-    const int solve_blocks = (int)std::min<int64_t>((nt + kBlk - 1) / kBlk, (int64_t)ctx->num_sms * 6);
+    const int solve_blocks = (int)std::min<int64_t>((nt + kBlk - 1) / kBlk, (int64_t)ctx->num_sms * 4);
     const int heavy_blocks = (int)std::min<int64_t>((nt + kHeavyWarps - 1) / kHeavyWarps, (int64_t)ctx->num_sms * 6);
     a.cand_cap = kCandCap;
     a.n_threads = 0;
