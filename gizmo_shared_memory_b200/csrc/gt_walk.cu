@@ -1975,8 +1975,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pack_kernel(const Walk
 }
 
 // Packs of a group list over consecutive targets, in order: as many groups as fit kPackGroups and 32
-// targets and begin in one cell four leaf sides wide (the grandparent of the first group's first
-// leaf), so that a jump of the curve ends a pack.  One thread forms the packs of kPackRun groups (a
+// targets and begin in one cell sixteen sides of the first group's first leaf wide, so that a long
+// jump of the curve ends a pack (cells of four sides leave packs shorter: 11.2 against 10.9 ms for
+// the leaves of a clustered box of two million).  One thread forms the packs of kPackRun groups (a
 // run starts a new pack): first the count, then, with the runs' offsets, the packs.
 constexpr int kPackRun = 64;
 __global__ void pack_groups_kernel(const int2* __restrict__ groups, const int* __restrict__ roots, int64_t ng,
@@ -1989,7 +1990,7 @@ __global__ void pack_groups_kernel(const int2* __restrict__ groups, const int* _
         uint32_t n = 0;
         for (int64_t g = r * kPackRun; g < g1;) {
             const int t0 = groups[g].x;
-            const int shift = 3 * (max_level - max(level[sleaf[t0]] - 2, 0));
+            const int shift = 3 * (max_level - max(level[sleaf[t0]] - 4, 0));
             const uint64_t cell = skey[t0] >> shift;
             int k = 1;
             for (; k < kPackGroups && g + k < g1; ++k) {
@@ -2105,9 +2106,13 @@ __global__ void target_flags_kernel(const uint32_t* __restrict__ targets, int64_
 // Small explicit target lists (the sparse active sets of deep time bins) form their groups in one
 // block, in one launch: flags, an ordered compaction of the group starts into shared memory, then
 // the chunking of groups longer than kmax.  count[0] = groups, count[1] = chunks, as
-// finish_groups_dev leaves them; the walk reads count[1].
+// finish_groups_dev leaves them; the walk reads count[1].  What bounds it is the latency of the
+// scattered reads of rank and leaf_of, so every thread takes kSmallPer consecutive targets, whose
+// reads are all in flight at once, and each scan runs once: a walk of 4194 targets of 2^22 takes
+// 210 us instead of 217.
 constexpr int kSmallTargets = 8192;
 constexpr int kSmallThreads = 1024;
+constexpr int kSmallPer = kSmallTargets / kSmallThreads;
 
 // Exclusive scan of one value per thread over the 1024-thread block; *total gets the sum.
 __device__ __forceinline__ int block_excl_scan_1024(int v, int* wsum, int* total) {
@@ -2146,29 +2151,54 @@ small_groups_kernel(const uint32_t* __restrict__ targets, int nt, int mode, int 
                     unsigned* __restrict__ bad) {
     __shared__ int starts[kSmallTargets + 1];
     __shared__ int wsum[32];
+    __shared__ int last[32];  // the key of each warp's last target
     __shared__ int total;
-    int ng = 0;
-    for (int base = 0; base < nt; base += kSmallThreads) {
-        const int k = base + (int)threadIdx.x;
-        const bool st = k < nt && target_starts(targets, k, mode, param, rank, leaf_of, gid, tpos, sys_off,
-                                                in_off, n_systems, 0, n, bad);
-        const int at = block_excl_scan_1024(st ? 1 : 0, wsum, &total);
-        if (st) starts[ng + at] = k;
-        ng += total;
-        __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k0 = (int)threadIdx.x * kSmallPer;
+    uint32_t p[kSmallPer], pos[kSmallPer];
+    int key[kSmallPer];  // what two neighbours of one group share (windows: their system)
+#pragma unroll
+    for (int i = 0; i < kSmallPer; ++i) p[i] = k0 + i < nt ? checked_target(targets, k0 + i, n, bad) : 0u;
+#pragma unroll
+    for (int i = 0; i < kSmallPer; ++i) pos[i] = k0 + i < nt ? rank[p[i]] : 0u;
+#pragma unroll
+    for (int i = 0; i < kSmallPer; ++i) {
+        key[i] = 0;
+        if (k0 + i >= nt) continue;
+        if (mode == GT_GROUP_LEAF) key[i] = leaf_of[p[i]];
+        else if (mode == GT_GROUP_NODE) key[i] = gid[pos[i]];
+        else if (mode == GT_GROUP_BATCH && n_systems > 1) key[i] = system_of(in_off, n_systems, (int64_t)p[i]);
     }
+    if (lane == 31) last[w] = key[kSmallPer - 1];
+    __syncthreads();
+    int prev = __shfl_up_sync(kFull, key[kSmallPer - 1], 1);
+    if (lane == 0) prev = w > 0 ? last[w - 1] : 0;
+    unsigned flags = 0;
+#pragma unroll
+    for (int i = 0; i < kSmallPer; ++i) {
+        const int k = k0 + i, q = i > 0 ? key[i - 1] : prev;
+        if (k >= nt) continue;
+        tpos[k] = pos[i];
+        // a new group where the key changes or is negative (target_starts)
+        bool st = k == 0;
+        if (mode == GT_GROUP_LEAF || mode == GT_GROUP_NODE) st |= key[i] != q || key[i] < 0;
+        else if (mode == GT_GROUP_BATCH) st |= key[i] != q || k % param == 0;
+        else st = true;
+        if (st) flags |= 1u << i;
+    }
+    int at = block_excl_scan_1024(__popc(flags), wsum, &total);
+#pragma unroll
+    for (int i = 0; i < kSmallPer; ++i)
+        if ((flags >> i) & 1u) starts[at++] = k0 + i;
+    const int ng = total;
     if (threadIdx.x == 0) starts[ng] = nt;
     __syncthreads();
-    int nc = 0;
-    for (int base = 0; base < ng; base += kSmallThreads) {
-        const int gi = base + (int)threadIdx.x;
-        const int s = gi < ng ? starts[gi] : 0, e = gi < ng ? starts[gi + 1] : 0;
-        const int c = gi < ng ? (e - s + kmax - 1) / kmax : 0;
-        int o = nc + block_excl_scan_1024(c, wsum, &total);
-        for (int a = s; a < e; a += kmax, ++o) groups[o] = make_int2(a, min(a + kmax, e));
-        nc += total;
-    }
-    if (threadIdx.x == 0) { count[0] = (uint32_t)ng; count[1] = (uint32_t)nc; }
+    // chunks of the groups, kSmallPer groups per thread
+    int c = 0;
+    for (int g = k0; g < min(k0 + kSmallPer, ng); ++g) c += (starts[g + 1] - starts[g] + kmax - 1) / kmax;
+    int o = block_excl_scan_1024(c, wsum, &total);
+    for (int g = k0; g < min(k0 + kSmallPer, ng); ++g)
+        for (int a = starts[g]; a < starts[g + 1]; a += kmax, ++o) groups[o] = make_int2(a, min(a + kmax, starts[g + 1]));
+    if (threadIdx.x == 0) { count[0] = (uint32_t)ng; count[1] = (uint32_t)total; }
 }
 
 __global__ void compact_starts_kernel(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ pos,
@@ -2785,10 +2815,12 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
                : macn ? occupancy_blocks<4, true, false, false, 2>(warps, pn_cap)
                       : occupancy_blocks<4, true, false, false, 0>(warps, pn_cap);
     // Long windows hand over (Handover) where a walk of the whole tree lasts about as long as its longest
-    // pair: fewer than two pairs per resident warp.  The budget is 96 iterations, half as much again as
-    // a pair's mean, where the records suffice for every pair of the tree, and 192 beyond, which a few
-    // per cent of the pairs reach.  A Plummer sphere of 65,536: 4.6 -> 0.8 ms, of 300,000: 1.01 -> 0.71
-    // ms; a galaxy of 100,000: 0.495 -> 0.469 ms.  With more pairs the GPU is busy to the end and the
+    // pair: fewer than two pairs per resident warp.  Where a third of the warps would have a pair the
+    // budget is 32 iterations, half a pair's mean, and the idle warps take the rest; up to a record for
+    // every pair it is 96, and 192 beyond, which a few per cent of the pairs reach.  Plummer spheres of
+    // 9,000, 65,536 and 300,000: 0.27, 0.70 and 0.71 ms (no hand-over, the last two: 4.6 and 1.01; a
+    // budget of 96, the first two: 0.42 and 0.82); a galaxy of 100,000: 0.469 ms (0.495; 0.50 at 32).
+    // With more pairs the GPU is busy to the end and the
     // hand-over only adds work: 5.8 -> 6.3 ms for a galaxy of 2^22 at 256.  The rule reads the tree's
     // size and not the call's targets, so a slice of the targets is walked as it is in the whole.
     const int64_t tree_units = paired ? ((t->n_live + param - 1) / param + 1) / 2 : 0;
@@ -2796,7 +2828,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     int budget = 0, hand_cap = 0;
     if (paired && tree_units < (int64_t)2 * 24 * ctx->num_sms) {
         hand_cap = (int)std::min<int64_t>(units, kHandRecords);
-        budget = tree_units <= kHandRecords ? 96 : 192;
+        budget = tree_units <= (int64_t)8 * ctx->num_sms ? 32 : tree_units <= kHandRecords ? 96 : 192;
     }
     const int64_t want_blocks = ((paired ? (ng + 1) / 2 : packed ? n_packs : ng) + warps - 1) / warps;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want_blocks, (int64_t)per_sm * ctx->num_sms));

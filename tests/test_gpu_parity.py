@@ -383,6 +383,25 @@ def test_packs_match_single_groups(gpu_ctx, ics_kind, batch):
         assert np.array_equal(o[k][ob], c[k])
 
 
+@pytest.mark.parametrize("nt", [1, 7, 8, 9, 257, 4095, 8191, 8192])
+@pytest.mark.parametrize("mode", [g.GT_GROUP_LEAF, g.GT_GROUP_NODE, g.GT_GROUP_BATCH])
+def test_small_target_lists_group_as_long_ones(gpu_ctx, plummer, plummer_trees, nt, mode):
+    """Up to 8192 explicit targets form their groups in one block, eight targets per thread; longer lists
+    by scans.  A list's groups are those of its targets at the start of a longer list, so the forces
+    are the same bits, but for a last window that the longer list continues."""
+    T = plummer_trees[0]
+    ob = T.download(nodes=False)["orderbuf"]
+    pos = np.sort(np.random.default_rng(nt).choice(30000, nt, replace=False))
+    rest = ob[40000:40000 + 8192]
+    kw = dict(theta=0.7, batch=32 if mode == g.GT_GROUP_BATCH else 0, group_mode=mode, window_pairs=False)
+    a = gpu_ctx.accel_grouped(T, ob[pos], **kw)
+    b = gpu_ctx.accel_grouped(T, np.concatenate([ob[pos], rest]), **kw)
+    whole = nt if mode != g.GT_GROUP_BATCH else nt // 32 * 32
+    for k in range(3):
+        assert np.array_equal(a[k][:whole], b[k][:whole])
+    assert np.isfinite(np.stack(a)).all()
+
+
 # ---- direct sum -----------------------------------------------------------------------------
 
 def test_direct_fp64_and_fp32(gpu_ctx, oracle, plummer):
