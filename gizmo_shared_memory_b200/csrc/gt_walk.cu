@@ -571,8 +571,10 @@ walk_kernel(const WalkArgs A) {
                         for (int c = 0; c < 10; ++c) xq2[XT == 1 ? k : 0][c] = make_float2(0.0f, 0.0f);
                 }
                 // 8 pairs in flight per lane (unroll 2 and 4 measured 1.9 % and 0.6 % slower); the
-                // tidal and jerk body is three times longer, and unrolled it outgrows instruction fetch
-#pragma unroll (XT == 1 ? 1 : 8)
+                // tidal and jerk body is three times longer and outgrows instruction fetch when it is
+                // unrolled far: 4.13 ms for a galaxy of 2^20 not unrolled, 3.90 by 2, 3.87 by 3, 3.96
+                // by 4; a clustered box 2.23, 2.04, 2.06, 2.07
+#pragma unroll (XT == 1 ? 2 : 8)
                 for (int jp = slice; jp < np; jp += NS) {
                     const float4 A = pn[2 * jp], B = pn[2 * jp + 1];
                     const float2 X = make_float2(A.x, A.y), Y = make_float2(A.z, A.w);
