@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 
 #include "gt_internal.cuh"
 
@@ -100,6 +101,43 @@ void* host_stage(gt_context* ctx, size_t bytes) {
     return p;
 }
 
+void host_copy(const HostPiece* pieces, int n) {
+    constexpr size_t kSplit = (size_t)2 << 20;  // bytes worth a thread of their own (it costs 20 us)
+    constexpr size_t kThreads = 4;              // 32 MB into fresh pages: 4.3 ms by one, 1.9 by 4, 1.5 by 8
+    size_t total = 0;
+    for (int i = 0; i < n; ++i) total += pieces[i].bytes;
+    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+    const size_t parts = std::max<size_t>(1, std::min({kThreads, cores, total / kSplit}));
+    const size_t share = (total / parts + 4096) & ~(size_t)4095;
+    // bytes [share * k, share * (k + 1)) of the pieces laid end to end
+    auto copy = [&](size_t k) {
+        const size_t a = share * k, b = k + 1 == parts ? total : std::min(total, share * (k + 1));
+        size_t at = 0;
+        for (int i = 0; i < n; ++i) {
+            const size_t lo = std::max(a, at), hi = std::min(b, at + pieces[i].bytes);
+            if (lo < hi)
+                std::memcpy((char*)pieces[i].dst + (lo - at), (const char*)pieces[i].src + (lo - at), hi - lo);
+            at += pieces[i].bytes;
+        }
+    };
+    std::thread th[kThreads];
+    size_t made = 0;
+    try {
+        for (; made + 1 < parts; ++made) th[made] = std::thread(copy, made);
+    } catch (...) {
+        // no thread to be had: this one copies the rest
+    }
+    for (size_t k = made; k < parts; ++k) copy(k);
+    for (size_t k = 0; k < made; ++k) th[k].join();
+}
+
+bool is_pageable(const void* host) {
+    cudaPointerAttributes at;
+    const bool p = cudaPointerGetAttributes(&at, host) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return p;
+}
+
 }  // namespace gt
 
 using namespace gt;
@@ -166,9 +204,35 @@ T* out_buf(gt_context* ctx, Slot s, T* p, int64_t n, int mem) {
     return (T*)scratch(ctx, s, (size_t)std::max<int64_t>(n, 1) * sizeof(T));
 }
 
+// A large pageable destination is filled through the pinned staging buffer, a ring of four pieces: the
+// next pieces cross the bus while host_copy moves the one that has landed.  The driver's own copy to
+// pageable memory runs in one thread: 7.5 ms for 32 MB into fresh pages, 2 ms this way.
+constexpr size_t kRingPiece = (size_t)8 << 20;
+constexpr int kRing = 4;
+
 template <typename T>
 void copy_out(gt_context* ctx, T* host, const T* dev, int64_t n, int mem) {
     if (!host || mem == GT_MEM_DEVICE || n <= 0) return;
+    const size_t bytes = (size_t)n * sizeof(T);
+    if (bytes >= kRingPiece && is_pageable(host)) {
+        ensure_copy_stream(ctx);  // the events
+        char* stage = (char*)host_stage(ctx, kRing * kRingPiece);
+        const int64_t pieces = (int64_t)((bytes + kRingPiece - 1) / kRingPiece);
+        auto size = [&](int64_t k) { return std::min(kRingPiece, bytes - (size_t)k * kRingPiece); };
+        auto send = [&](int64_t k) {
+            check_cuda(cudaMemcpyAsync(stage + (k % kRing) * kRingPiece, (const char*)dev + (size_t)k * kRingPiece, size(k),
+                                       cudaMemcpyDeviceToHost, ctx->stream), "D2H");
+            check_cuda(cudaEventRecord(ctx->down_ev[k % kRing], ctx->stream), "event");
+        };
+        for (int64_t k = 0; k < std::min<int64_t>(pieces, kRing); ++k) send(k);
+        for (int64_t k = 0; k < pieces; ++k) {
+            check_cuda(cudaEventSynchronize(ctx->down_ev[k % kRing]), "sync");
+            const HostPiece p{(char*)host + (size_t)k * kRingPiece, stage + (k % kRing) * kRingPiece, size(k)};
+            host_copy(&p, 1);
+            if (k + kRing < pieces) send(k + kRing);
+        }
+        return;
+    }
     check_cuda(cudaMemcpyAsync(host, dev, (size_t)n * sizeof(T), cudaMemcpyDeviceToHost, ctx->stream), "D2H");
 }
 

@@ -257,6 +257,16 @@ void ensure_copy_stream(gt_context* ctx);
 // The context's pinned staging buffer of at least `bytes` (grow-only; throws Fail).
 void* host_stage(gt_context* ctx, size_t bytes);
 
+// Copies between host arrays.  One thread moves 7 GB/s into fresh pages, whose first touch is most of
+// the cost, so a large copy is split over a few threads that live as long as it does.
+struct HostPiece {
+    void* dst;
+    const void* src;
+    size_t bytes;
+};
+void host_copy(const HostPiece* pieces, int n);
+bool is_pageable(const void* host);
+
 // Walk (gt_walk.cu)
 // Stack and counters owned by a walk plan (a captured graph must not point into the workspace).
 struct WalkBuffers {

@@ -2974,11 +2974,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         size_t stage_need = 0;
         for (int i = 0; i < 6; ++i) {
             if (!outs[i].dev || !outs[i].host) continue;
-            cudaPointerAttributes at;
-            const bool pageable = cudaPointerGetAttributes(&at, outs[i].host) != cudaSuccess ||
-                                  at.type == cudaMemoryTypeUnregistered;
-            cudaGetLastError();
-            if (!pageable) continue;
+            if (!is_pageable(outs[i].host)) continue;
             staged[i] = true;
             stage_off[i] = stage_need;
             stage_need += (size_t)nt * outs[i].stride * sizeof(double);
@@ -3065,11 +3061,14 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
                 const int64_t t0 = hb[c].y, t1 = hb[c + 1].y;
                 if (t1 <= t0) continue;
                 check_cuda(cudaEventSynchronize(ctx->down_ev[c]), "sync");
+                HostPiece pieces[6];
+                int np = 0;
                 for (int i = 0; i < 6; ++i)
                     if (staged[i])
-                        std::memcpy(outs[i].host + t0 * outs[i].stride,
-                                    reinterpret_cast<const double*>(stage + stage_off[i]) + t0 * outs[i].stride,
-                                    (size_t)(t1 - t0) * outs[i].stride * sizeof(double));
+                        pieces[np++] = HostPiece{outs[i].host + t0 * outs[i].stride,
+                                                 reinterpret_cast<const double*>(stage + stage_off[i]) + t0 * outs[i].stride,
+                                                 (size_t)(t1 - t0) * outs[i].stride * sizeof(double)};
+                host_copy(pieces, np);
             }
         }
         if (two) {

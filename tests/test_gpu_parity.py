@@ -623,6 +623,17 @@ def test_host_outputs_copied_in_chunks_are_identical(gpu_ctx):
         assert np.array_equal(d.cpu().numpy(), h)
 
 
+@pytest.mark.parametrize("n", [2 ** 20 - 1, 2 ** 20, 2 ** 20 + 1, 2 ** 22, 5 * 2 ** 20 + 3])
+def test_large_host_outputs_cross_the_ring_unchanged(gpu_ctx, n):
+    """Outputs of 8 MB (2^20 doubles) and more reach pageable memory through a ring of four pinned pieces:
+    the same bits as in device memory, below one piece, at its edge and past the ring."""
+    import torch
+
+    v = np.random.default_rng(n).normal(size=(3, n))
+    dev = gpu_ctx.form_aold(*(torch.as_tensor(x, device="cuda") for x in v), 0.005, G=2.0)
+    assert np.array_equal(gpu_ctx.form_aold(*v, 0.005, G=2.0), dev.cpu().numpy())
+
+
 def test_host_aold_uploaded_in_chunks_is_identical(gpu_ctx):
     """A walk given a host aold and host outputs uploads aold piece by piece on the copy stream,
     each chunk waiting only for its own targets' piece, and downloads each chunk's results while the
