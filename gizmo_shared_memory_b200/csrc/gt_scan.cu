@@ -46,10 +46,7 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total)
     return res;
 }
 
-// n_dev (optional): the number of items, on the device, at most n (the launch is sized by n).
-__global__ void tile_sum_kernel(const uint32_t* __restrict__ in, int64_t n, uint32_t* __restrict__ sums,
-                                const int64_t* __restrict__ n_dev) {
-    if (n_dev) n = min(n, *n_dev);
+__global__ void tile_sum_kernel(const uint32_t* __restrict__ in, int64_t n, uint32_t* __restrict__ sums) {
     const int64_t base = (int64_t)blockIdx.x * kScanTile;
     uint32_t s = 0;
 #pragma unroll
@@ -63,9 +60,7 @@ __global__ void tile_sum_kernel(const uint32_t* __restrict__ in, int64_t n, uint
 }
 
 // One block scans all tile totals in place (exclusive); total to total_out.
-__global__ void scan_sums_kernel(uint32_t* __restrict__ sums, int nb, uint32_t* __restrict__ total_out,
-                                 const int64_t* __restrict__ n_dev) {
-    if (n_dev) nb = (int)min((int64_t)nb, (*n_dev + kScanTile - 1) / kScanTile);
+__global__ void scan_sums_kernel(uint32_t* __restrict__ sums, int nb, uint32_t* __restrict__ total_out) {
     const int per = (nb + blockDim.x - 1) / blockDim.x;
     const int lo = threadIdx.x * per, hi = min(nb, lo + per);
     uint32_t s = 0;
@@ -83,9 +78,7 @@ __global__ void scan_sums_kernel(uint32_t* __restrict__ sums, int nb, uint32_t* 
 // Blocked arrangement inside the tile: thread t owns items [t*8, t*8+8) so the scan order is the
 // index order.
 __global__ void tile_scan_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int64_t n,
-                                 const uint32_t* __restrict__ sums, const int64_t* __restrict__ n_dev) {
-    if (n_dev) n = min(n, *n_dev);
-    if ((int64_t)blockIdx.x * kScanTile >= n) return;  // the whole block lies past the items
+                                 const uint32_t* __restrict__ sums) {
     const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
     uint32_t s = 0;
@@ -130,6 +123,35 @@ __global__ void radix_hist_kernel(const uint64_t* __restrict__ keys, int64_t n, 
     hist[(int64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
+// A block per digit: its counts become exclusive sums over the tiles, its total goes to totals.  The
+// sums over the digits are left to the scatter, whose blocks each scan the 256 totals, so a pass is
+// three launches, where a scan of the whole table, as scan_exclusive_u32 runs it, made it five: a
+// dozen microseconds a pass at any size, most of them launches of a few blocks.
+__global__ void __launch_bounds__(kScanThreads)
+radix_rows_kernel(uint32_t* __restrict__ hist, int nblocks, uint32_t* __restrict__ totals) {
+    uint32_t* row = hist + (int64_t)blockIdx.x * nblocks;
+    uint32_t run = 0;
+    for (int tile = 0; tile < nblocks; tile += kScanTile) {
+        const int base = tile + (int)threadIdx.x * kScanItems;
+        uint32_t v[kScanItems];
+        uint32_t s = 0;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            v[k] = base + k < nblocks ? row[base + k] : 0u;
+            s += v[k];
+        }
+        uint32_t tot;
+        uint32_t at = run + block_excl_scan(s, &tot);
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            if (base + k < nblocks) row[base + k] = at;
+            at += v[k];
+        }
+        run += tot;
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = run;
+}
+
 // Stable scatter of one 8-bit digit.  Warp w owns keys [w*256, w*256+256) of the tile and walks
 // them 32 at a time in index order; lanes with equal digits are ranked with __match_any_sync, so
 // the destination order equals the source order within every digit.  The tile is first reordered
@@ -139,7 +161,7 @@ __global__ void radix_hist_kernel(const uint64_t* __restrict__ keys, int64_t n, 
 __global__ void __launch_bounds__(kSortThreads)
 radix_scatter_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                      uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n, int shift,
-                     const uint32_t* __restrict__ offsets, int nblocks) {
+                     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ totals, int nblocks) {
     __shared__ uint32_t wh[kSortWarps][kRadix];
     __shared__ uint32_t boff[kRadix];
     __shared__ uint32_t bstart[kRadix];   // first tile position of each digit
@@ -148,8 +170,14 @@ radix_scatter_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restric
     __shared__ uint32_t tval[kSortTile];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int d = threadIdx.x; d < kSortWarps * kRadix; d += kSortThreads) (&wh[0][0])[d] = 0;
-    boff[threadIdx.x] = offsets[(int64_t)threadIdx.x * nblocks + blockIdx.x];
-    __syncthreads();
+    {   // where this block's run of each digit goes: all keys of smaller digits, then those of earlier tiles
+        const uint32_t c = totals[threadIdx.x], inc = warp_incl_scan(c);
+        if (lane == 31) wsum[w] = inc;
+        __syncthreads();
+        uint32_t at = inc - c + offsets[(int64_t)threadIdx.x * nblocks + blockIdx.x];
+        for (int ww = 0; ww < w; ++ww) at += wsum[ww];
+        boff[threadIdx.x] = at;
+    }
     const int64_t tile0 = (int64_t)blockIdx.x * kSortTile;
     const int64_t base = tile0 + (int64_t)w * kWarpSpan;
     const uint32_t lt = (1u << lane) - 1u;
@@ -182,12 +210,7 @@ radix_scatter_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restric
         }
     }
     {   // exclusive scan over digits of the block's counts: where each digit's run starts in the tile
-        uint32_t v = total;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += t;
-        }
+        const uint32_t v = warp_incl_scan(total);
         if (lane == 31) wsum[w] = v;
         __syncthreads();
         uint32_t before = 0;
@@ -217,18 +240,18 @@ radix_scatter_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restric
 }  // namespace
 
 void scan_exclusive_u32(gt_context* ctx, const uint32_t* in, uint32_t* out, int64_t n,
-                        uint32_t* total_dev, const int64_t* n_dev) {
+                        uint32_t* total_dev) {
     if (n <= 0) {
         if (total_dev) check_cuda(cudaMemsetAsync(total_dev, 0, 4, ctx->stream), "memset");
         return;
     }
     const int nb = div_up(n, kScanTile);
     uint32_t* sums = (uint32_t*)scratch(ctx, kSlotScanB, (size_t)nb * 4);
-    tile_sum_kernel<<<nb, kScanThreads, 0, ctx->stream>>>(in, n, sums, n_dev);
+    tile_sum_kernel<<<nb, kScanThreads, 0, ctx->stream>>>(in, n, sums);
     check_launch(ctx, "tile_sum_kernel");
-    scan_sums_kernel<<<1, 1024, 0, ctx->stream>>>(sums, nb, total_dev, n_dev);
+    scan_sums_kernel<<<1, 1024, 0, ctx->stream>>>(sums, nb, total_dev);
     check_launch(ctx, "scan_sums_kernel");
-    tile_scan_kernel<<<nb, kScanThreads, 0, ctx->stream>>>(in, out, n, sums, n_dev);
+    tile_scan_kernel<<<nb, kScanThreads, 0, ctx->stream>>>(in, out, n, sums);
     check_launch(ctx, "tile_scan_kernel");
 }
 
@@ -237,7 +260,8 @@ void radix_sort_pairs(gt_context* ctx, uint64_t* keys, uint32_t* vals, int64_t n
     const int nb = div_up(n, kSortTile);
     uint64_t* kb = (uint64_t*)scratch(ctx, kSlotKeysB, (size_t)n * 8);
     uint32_t* vb = (uint32_t*)scratch(ctx, kSlotValsB, (size_t)n * 4);
-    uint32_t* hist = (uint32_t*)scratch(ctx, kSlotHist, (size_t)kRadix * nb * 4);
+    uint32_t* hist = (uint32_t*)scratch(ctx, kSlotHist, ((size_t)nb + 1) * kRadix * 4);
+    uint32_t* totals = hist + (size_t)kRadix * nb;
     uint64_t* ka = keys;
     uint32_t* va = vals;
     const int passes = (bits + 7) / 8;
@@ -245,8 +269,9 @@ void radix_sort_pairs(gt_context* ctx, uint64_t* keys, uint32_t* vals, int64_t n
         const int shift = 8 * p;
         radix_hist_kernel<<<nb, kSortThreads, 0, ctx->stream>>>(ka, n, shift, hist, nb);
         check_launch(ctx, "radix_hist_kernel");
-        scan_exclusive_u32(ctx, hist, hist, (int64_t)kRadix * nb, nullptr);
-        radix_scatter_kernel<<<nb, kSortThreads, 0, ctx->stream>>>(ka, va, kb, vb, n, shift, hist, nb);
+        radix_rows_kernel<<<kRadix, kScanThreads, 0, ctx->stream>>>(hist, nb, totals);
+        check_launch(ctx, "radix_rows_kernel");
+        radix_scatter_kernel<<<nb, kSortThreads, 0, ctx->stream>>>(ka, va, kb, vb, n, shift, hist, totals, nb);
         check_launch(ctx, "radix_scatter_kernel");
         uint64_t* tk = ka; ka = kb; kb = tk;
         uint32_t* tv = va; va = vb; vb = tv;

@@ -150,6 +150,48 @@ def test_tree_threading_audit(gpu_ctx, plummer):
     assert np.all(seen == 1)
 
 
+@pytest.mark.parametrize("ics_kind,n", [("clumps", 17000), ("uniform", 2047), ("uniform", 2048), ("uniform", 2049),
+                                        ("uniform", 2048 * 2048 + 1), ("one", 1), ("massless", 100)])
+def test_tree_structure_at_the_edges_of_its_kernels(gpu_ctx, ics_kind, n):
+    """The sort's tiles hold 2048 keys and its rows 2048 tiles per step; a level's nodes are shared out
+    among the blocks, 256 at a time; clumps of 17 close particles make more nodes than the arrays first
+    hold, so the levels run again in larger ones.  Keys sorted, equal ones in index order, every node's
+    children contiguous in particles and in nodes, and every leaf at its limit."""
+    rng = np.random.default_rng(n)
+    x = rng.uniform(0, 1, (3, n))
+    if ics_kind == "clumps":
+        x = np.repeat(x[:, ::17], 17, axis=1)[:, rng.permutation(n)] + rng.uniform(0, 1e-7, (3, n))
+    P = dict(zip("xyz", x), m=np.full(n, 0.0 if ics_kind == "massless" else 1.0), soft=np.full(n, 1e-3))
+    T = gpu_ctx.build(P, key_mode=g.GT_KEY_MORTON)
+    d, key = T.download(), T.keys()
+    live = 0 if ics_kind == "massless" else n
+    ob, first, plo, phi, lev = d["orderbuf"], d["first"], d["plo"], d["phi"], d["level"]
+    assert np.array_equal(np.sort(ob), np.arange(live)) and np.array_equal(d["rank"][ob], np.arange(live))
+    assert np.all((key[1:] > key[:-1]) | ((key[1:] == key[:-1]) & (ob[1:] > ob[:-1])))
+    inner = np.nonzero(first >= 0)[0]
+    leaf = first < 0
+    assert np.all((phi - plo)[leaf & (lev < 20)] <= 16) and np.all((phi - plo)[inner] > 16)
+    if len(inner) == 0:
+        assert len(first) == 1
+        return
+    end = np.append(first[inner][1:], len(first))  # children of successive inner nodes follow one another
+    assert first[inner][0] == 1
+    assert np.array_equal(plo[first[inner]], plo[inner]) and np.array_equal(phi[end - 1], phi[inner])
+    cell = np.repeat(np.arange(len(inner)), end - first[inner])
+    assert np.array_equal(d["parent"][1:], inner[cell]) and np.array_equal(lev[1:], lev[inner][cell] + 1)
+    same = cell[1:] == cell[:-1]
+    assert np.array_equal(plo[2:][same], phi[1:-1][same])
+    last = np.append(~same, True)
+    child = np.arange(1, len(first))
+    assert np.array_equal(d["next"][1:], np.where(last, d["next"][inner[cell]], child + 1))
+    shift = np.uint64(3) * (20 - lev[1:]).astype(np.uint64)
+    k0, k1 = key[plo[1:]] >> shift, key[phi[1:] - 1] >> shift
+    assert np.array_equal(k0, k1) and np.all(k0[1:][same] > k0[:-1][same])
+    if ics_kind == "clumps":
+        assert len(first) > 2 * n // 16 * 3 + 1024 + 1  # the first arrays
+    gpu_ctx.accel_grouped(T, None, theta=0.7)
+
+
 # ---- walks ----------------------------------------------------------------------------------
 
 def check(a, b, tol=MEDIAN_TOL, p99=2e-3):
