@@ -214,9 +214,16 @@ template <typename T>
 void copy_out(gt_context* ctx, T* host, const T* dev, int64_t n, int mem) {
     if (!host || mem == GT_MEM_DEVICE || n <= 0) return;
     const size_t bytes = (size_t)n * sizeof(T);
+    char* stage = nullptr;
     if (bytes >= kRingPiece && is_pageable(host)) {
         ensure_copy_stream(ctx);  // the events
-        char* stage = (char*)host_stage(ctx, kRing * kRingPiece);
+        try {
+            stage = (char*)host_stage(ctx, kRing * kRingPiece);
+        } catch (const Fail&) {
+            // no pinned memory to be had: the driver's copy
+        }
+    }
+    if (stage) {
         const int64_t pieces = (int64_t)((bytes + kRingPiece - 1) / kRingPiece);
         auto size = [&](int64_t k) { return std::min(kRingPiece, bytes - (size_t)k * kRingPiece); };
         auto send = [&](int64_t k) {
