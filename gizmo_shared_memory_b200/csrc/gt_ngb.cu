@@ -7,8 +7,10 @@
 // root side plus four float ulps of the largest centre coordinate, tree.cc:490-505), with the
 // reference's threading (first child / next).  One thread follows the threading for one centre,
 // as the reference's loop does, so every list comes out in tree order -- the reference's order --
-// and the density sums accumulate in the reference's order too.  Neighbouring centres (tree-ordered
-// targets) follow nearly the same path, so a warp's threads mostly read the same nodes.
+// and the density sums accumulate in the reference's order too.  The leaves a thread reaches wait in
+// a small buffer, and their particles are tested in a run, where the lanes of a warp meet again.  In
+// the density solve a lane whose target is done takes another, and targets with very many candidates
+// go to a warp each, which sums in the same order.
 //
 // Lists are CSR: a counting pass, an exclusive scan, and a filling pass over the same traversal.
 //

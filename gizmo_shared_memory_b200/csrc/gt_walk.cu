@@ -23,6 +23,9 @@
 //     both lists in pairs of entries and evaluate two entries per sm_100 packed FP32 instruction.
 //     Groups of <= 16 targets split the list across the idle lanes (lane = slice * NT + target)
 //     and reduce the slices at the end.
+//   * Windows of 17-32 share a traversal in pairs (walk_pair_kernel), and where a small tree leaves
+//     warps idle a long pair hands the rest of its traversal to them (Handover).  Walks of all targets
+//     in smaller groups share one among up to eight groups (walk_pack_kernel).
 //   * Accumulation: each list evaluation sums into FP32 partials, which are added into FP32
 //     Kahan-compensated totals (acceleration) and an FP64 total (potential); the final sums and
 //     the factor G are FP64.
