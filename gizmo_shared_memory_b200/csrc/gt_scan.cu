@@ -125,8 +125,9 @@ __global__ void radix_hist_kernel(const uint64_t* __restrict__ keys, int64_t n, 
 
 // A block per digit: its counts become exclusive sums over the tiles, its total goes to totals.  The
 // sums over the digits are left to the scatter, whose blocks each scan the 256 totals, so a pass is
-// three launches, where a scan of the whole table, as scan_exclusive_u32 runs it, made it five: a
-// dozen microseconds a pass at any size, most of them launches of a few blocks.
+// three launches, where a scan of the whole table, as scan_exclusive_u32 runs it, made it five:
+// 65,536 keys in 0.142 ms instead of 0.211, 2^20 in 0.214 instead of 0.267, 2^24 in 1.77 instead of
+// 1.71.
 __global__ void __launch_bounds__(kScanThreads)
 radix_rows_kernel(uint32_t* __restrict__ hist, int nblocks, uint32_t* __restrict__ totals) {
     uint32_t* row = hist + (int64_t)blockIdx.x * nblocks;
