@@ -25,7 +25,7 @@
 //     and reduce the slices at the end.
 //   * Windows of 17-32 share a traversal in pairs (walk_pair_kernel), and where a small tree leaves
 //     warps idle a long pair hands the rest of its traversal to them (Handover).  Walks of all targets
-//     in smaller groups share one among up to eight groups (walk_pack_kernel).
+//     by leaves share one among up to eight leaves (walk_pack_kernel).
 //   * Accumulation: each list evaluation sums into FP32 partials, which are added into FP32
 //     Kahan-compensated totals (acceleration) and an FP64 total (potential); the final sums and
 //     the factor G are FP64.
@@ -2655,12 +2655,13 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     int64_t ng = 0;
     const uint32_t* tpos = nullptr;
     const uint32_t* ng_dev = nullptr;  // explicit targets: the group count stays on the device
-    // Small groups over all live targets (the engine's leaves, windows of at most 16): packs of them
-    // share one traversal.  A list of explicit targets may hold groups far from one another, which
-    // share nothing and keep a warp each.
+    // The leaves of all live targets (the engine's grouping): packs of them share one traversal.  A list
+    // of explicit targets may hold groups far from one another, which share nothing and keep a warp
+    // each; so do small windows, whose boxes span the jumps of the curve (a clustered box is suspected
+    // of 4.05 -> 7.06 ms when packed, and was not measured apart).
     bool packed = all && rq.pair_windows && !xt && tpl == 1 && rq.leaf_accept && rq.mac != GT_MAC_LEARNED &&
                   !rq.count && t->n_nodes < (1 << 24) && rq.list_capacity == 0 &&
-                  (mode == GT_GROUP_LEAF || (mode == GT_GROUP_BATCH && param <= 16));
+                  mode == GT_GROUP_LEAF;
     int2* packs = nullptr;
     int64_t n_packs = 0;
     if (all) {

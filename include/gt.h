@@ -132,8 +132,7 @@ typedef struct {
      * for bit: the list order can differ).  Forests and counting walks included; not for
      * GT_MAC_LEARNED, the tidal tensor, the jerk or the gas rules.  Likewise by default: a long
      * window of a small tree hands part of its traversal to other warps, and in walks of all
-     * targets several leaf groups (or windows of up to 16) share one traversal, each again with its
-     * own decisions.  1: none of these, one warp per group. */
+     * targets several leaf groups share one traversal, each again with its own decisions.  1: none of these, one warp per group. */
     int no_window_pairs;
 } gt_walk_options;
 
