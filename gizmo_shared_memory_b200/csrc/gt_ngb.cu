@@ -308,7 +308,9 @@ __global__ void __launch_bounds__(kBlk) ngb_kernel(const NgbArgs a) {
         int r0, r1;
         roots_of(a.g, a.systems, c, r0, r1, FILL ? nullptr : a.total + 1);
         int64_t k = FILL ? a.start[c] : 0;
+        const int64_t end = FILL ? a.start[c + 1] : 0;
         auto emit = [&](int s) {
+            if (FILL && k >= end) return false;  // never past the centre's own entries
             if (FILL) a.found[k] = __ldg(a.g.order + s);
             else if (k < a.kcache) a.cache[k * a.n + c] = __ldg(a.g.order + s);
             ++k;
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(kBlk) ngb_kernel(const NgbArgs a) {
         warp_flush(mine, a.total);
         warp_flush(over, a.total + 2);
     }
-    if (COUNT) {
+    if (COUNT && !FILL) {
         warp_flush(calls, a.tally + 0);
         warp_flush(tl.nodes, a.tally + 1);
         warp_flush(tl.examined, a.tally + 2);
@@ -1154,8 +1156,10 @@ int64_t run_ngb(gt_context* ctx, gt_tree* t, int64_t n, const double* cx, const 
         if (!a.kcache || total[2] > 0) {  // the centres the cache did not hold whole
             a.start = start;
             a.found = dst;
-            a.tally = nullptr;
-            ngb_kernel<true, false><<<grid_of(ctx, n), kBlk, 0, st>>>(a);
+            // by the traversal that counted them: on a tree whose boxes do not cover its moved
+            // particles the two prunes need not find the same
+            if (a.tally) ngb_kernel<true, true><<<grid_of(ctx, n), kBlk, 0, st>>>(a);
+            else ngb_kernel<true, false><<<grid_of(ctx, n), kBlk, 0, st>>>(a);
             check_launch(ctx, "ngb_kernel");
         }
     }

@@ -264,3 +264,60 @@ def test_density_lanes_and_warps_match_counting_solve(gpu_ctx, nt, guess):
         gpu_ctx.ngb_count(False)
     for k in ("h", "rho", "nngb", "iters"):
         assert np.array_equal(got[k], want[k], equal_nan=k in ("h", "rho")), k
+
+
+def search64(d, root, P, cen, rad):
+    """The reference's gather search over downloaded nodes and the particles' present positions, its
+    prune in FP64 on float boxes (hydro.cc:51-106): the lists of the centres."""
+    f32 = np.float32
+    box = np.stack([d[k].astype(f32) for k in ("gcx", "gcy", "gcz")], 1).astype(float)
+    top = np.max(np.abs(np.stack([d[k] for k in ("gcx", "gcy", "gcz")], 1)), axis=1)
+    half = (0.5 * d["size"] + 1e-6 * root + 4.0 * np.finfo(f32).eps * top).astype(f32).astype(float)
+    X = np.stack([P[k] for k in "xyz"], 1)[d["orderbuf"]]
+    lists = []
+    for c, r in zip(np.stack(cen, 1), rad):
+        node, found = 0, []
+        while node >= 0:
+            o, dist = np.abs(box[node] - c), r + half[node]
+            if (o > dist).any() or (o * o).sum() > (dist + 0.7320508075688772 * half[node]) ** 2:
+                node = d["next"][node]
+            elif d["first"][node] < 0:
+                s = np.arange(d["plo"][node], d["phi"][node])
+                found.append(d["orderbuf"][s[((X[s] - c) ** 2).sum(1) < r * r]])
+                node = d["next"][node]
+            else:
+                node = d["first"][node]
+        lists.append(np.concatenate(found))
+    return lists
+
+
+def test_counted_lists_of_moved_particles(gpu_ctx):
+    """Lists longer than the counting pass keeps are found again, by the same prune: on a tree whose
+    particles moved out of their boxes with no pad for it, a leaf that the counted search's FP64 prune
+    leaves out by four parts in 10^7 belongs to the wider FP32 prune of the plain search, and entries
+    found by one pass and not by the other would end up in the next centre's list."""
+    rng = np.random.default_rng(3)
+    x = np.concatenate([0.02 * rng.normal(size=(1200, 3)), [0.7, 1e-3, 1e-3] + 1e-4 * rng.normal(size=(10, 3)),
+                        rng.uniform(-1, 1, (800, 3))])
+    P = {k: x[:, i].copy() for i, k in enumerate("xyz")}
+    P["m"] = np.ones(len(x))
+    T = gpu_ctx.build(P, key_mode=g.GT_KEY_MORTON)
+    d = T.download()
+    leaf = d["leaf_of"][1200]
+    gone = np.nonzero(d["leaf_of"] == leaf)[0]
+    for k in "xyz":
+        P[k][gone] = 0.01 * rng.normal(size=len(gone))
+    gpu_ctx.tree_particles(T, *(P[k] for k in "xyz"))
+    cen = [np.linspace(-0.05, 0.05, 40), np.full(40, d["gcy"][leaf]), np.full(40, d["gcz"][leaf])]
+    half = 0.5 * d["size"][leaf] + 1e-6 * d["size"][0] + 4.0 * np.finfo(np.float32).eps * d["gcx"][leaf]
+    rad = (np.float64(np.float32(d["gcx"][leaf])) - cen[0] - half) * (1.0 - 4e-7)
+    plain = np.diff(gpu_ctx.ngb_search(T, *cen, rad)[0])
+    gpu_ctx.ngb_count(True)
+    try:
+        st, f = gpu_ctx.ngb_search(T, *cen, rad)
+    finally:
+        gpu_ctx.ngb_count(False)
+    want = search64(d, d["size"][0], P, cen, rad)
+    assert min(len(w) for w in want) > 64  # past what the counting pass keeps
+    assert (plain > np.diff(st)).any()     # the two prunes differ here
+    assert np.array_equal(np.diff(st), [len(w) for w in want]) and np.array_equal(f, np.concatenate(want))
