@@ -214,11 +214,15 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
                 if (!FP64) shm[q] = 0.0f;
                 continue;
             }
-            sh[q] = DirSrc{x[j], y[j], z[j], m[j]};
+            // a mass that is no number times the 0 of a pair left out would be none either: such a
+            // source weighs nothing on the short path and takes all its pairs off it
+            const double mj = m[j];
+            const bool fin = isfinite(FP64 ? mj : (double)(float)mj);
+            sh[q] = DirSrc{x[j], y[j], z[j], fin ? mj : 0.0};
             const double s = soft ? soft[j] : 0.0;
             shs[q] = s;
-            shlim[q] = limit(s);
-            if (!FP64) shm[q] = (float)m[j];
+            shlim[q] = fin ? limit(s) : INT_MAX;
+            if (!FP64) shm[q] = fin ? (float)mj : 0.0f;
             if (GAS) {
                 shzeta[q] = zeta ? zeta[j] : 0.0;
                 shgas[q] = (!type || type[j] == 0) ? 1 : 0;
@@ -273,16 +277,17 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
                         if (!((slow >> (i * kDirPer + k)) & 1u) || q >= nq || base + q == self[k]) continue;
                         const DirSrc s = sh[q];
                         const double ox = s.x - px[k], oy = s.y - py[k], oz = s.z - pz[k];
+                        const double mj = __ldg(m + base + q);  // as it was given
                         if (FP64) {
                             double mf, mp;
-                            pair_d<GAS>(ox, oy, oz, ps[k], shs[q], s.m, gas[GAS ? k : 0], GAS ? shzeta[q] : 0.0,
+                            pair_d<GAS>(ox, oy, oz, ps[k], shs[q], mj, gas[GAS ? k : 0], GAS ? shzeta[q] : 0.0,
                                         GAS && shgas[q], mf, mp);
                             ax[k] += ox * mf; ay[k] += oy * mf; az[k] += oz * mf;
                             ap[k] += mp;
                         } else {
                             const float dx = (float)ox, dy = (float)oy, dz = (float)oz;
                             float mf, mp;
-                            pair_f(dx, dy, dz, (float)ps[k], (float)shs[q], shm[q], mf, mp);
+                            pair_f(dx, dy, dz, (float)ps[k], (float)shs[q], (float)mj, mf, mp);
                             fx[k] += dx * mf; fy[k] += dy * mf; fz[k] += dz * mf;
                             fp[k] += mp;
                         }

@@ -490,6 +490,25 @@ def test_direct_edges_of_tiles(gpu_ctx, oracle, n, soft):
         assert (np.abs(phi - op) <= tol * pscale)[seen].all()
 
 
+@pytest.mark.parametrize("mass,precision", [(np.inf, g.GT_DIRECT_FP64), (np.nan, g.GT_DIRECT_FP64),
+                                            (np.inf, g.GT_DIRECT_FP32), (np.nan, g.GT_DIRECT_FP32),
+                                            (1e39, g.GT_DIRECT_FP32)])
+def test_direct_with_a_mass_that_is_no_number(gpu_ctx, mass, precision):
+    """A particle's own mass is no part of its own sum, nor of that of a particle in the same place: both
+    stay what they are when it weighs nothing, to the last bit, and everybody else's is no number."""
+    P = ics.plummer(n=300, seed=5)
+    for k in ("x", "y", "z"):
+        P[k][6] = P[k][5]
+    tg = np.arange(300, dtype=np.uint32)
+    P["m"][5] = 0.0
+    want = gpu_ctx.direct(P, tg, precision=precision)
+    P["m"][5] = mass
+    got = gpu_ctx.direct(P, tg, precision=precision)
+    for a, b in zip(got, want):
+        assert np.isfinite(b).all() and np.array_equal(a[5:7], b[5:7])
+        assert not np.isfinite(np.delete(a, [5, 6])).any()
+
+
 # ---- edge cases -----------------------------------------------------------------------------
 
 def test_empty_single_and_pair(gpu_ctx, oracle):
