@@ -111,16 +111,17 @@ struct WalkArgs {
 // Plummer sphere of 65,536 particles the longest pair of windows takes 1,800 iterations against a mean
 // of 60, and the walk took as long as that pair.  A pair that has used up its budget of iterations
 // therefore breaks up the large subtrees on its stack (a depth-first stack has a few that hold most of
-// what is left at its bottom), writes its state here and leaves it: a second launch walks every record in kShares shares, each with every
-// kShares-th stack entry, and the share that finishes last adds the parts in a fixed order.  What is
-// handed over and how it is shared out depends on the particles alone, so results do not change
-// from run to run.  When more pairs ask for a record than there are, every pair is finished by one
-// warp: those without a record at once, those with one from the saved state, as if it had not
-// been interrupted.
+// what is left at its bottom), writes its state here and leaves it: a second launch walks every record
+// in kShares shares, each with every kShares-th stack entry, and the share that finishes last adds the
+// parts in a fixed order.  A pair that finds no record left walks the same shares itself, one after
+// another, and adds their sums in the same order.  So what is handed over, how it is shared out and
+// how it is summed depend on the pair's own particles alone: not on which pairs got the records, on
+// how many asked in the same launch, or on how many there are.
 constexpr int kShares = 16;
 constexpr int kHandStack = 2048;   // entries of a record
 constexpr int kHandSteps = 96;     // at most this many steps break up the stack
 constexpr int kHandLeast = 4 * kShares;  // a shorter stack is not worth a record
+constexpr int kHandSums = 2 * 4 * 32 * 2;  // stack entries that hold a pair's sums while it walks its own shares
 struct HandSum {
     float2 x, y, z;  // Kahan sum and compensation
     double pot;
@@ -1108,10 +1109,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
     auto pp_of = [&](int v) { return pn_of(v) + A.pn_cap; };
     auto ph_of = [&](int v) { return reinterpret_cast<float*>(pp_of(v) + A.pp_cap); };
     const int n_groups = A.n_groups_dev ? (int)*A.n_groups_dev : A.n_groups;
-    // SHARE: the units are the records' shares, or whole records when more were asked for than there are
-    const int n_hand = SHARE ? (int)A.hand_ctr[0] : 0;
-    const bool whole = SHARE && n_hand > A.hand_cap;
-    const int n_units = SHARE ? (whole ? A.hand_cap : n_hand * kShares) : (n_groups + 1) >> 1;
+    // SHARE: the units are the records' shares
+    const int n_units = SHARE ? min((int)A.hand_ctr[0], A.hand_cap) * kShares : (n_groups + 1) >> 1;
+    // HAND: past the traversal's entries, the sums of a pair that walks its own shares
+    const int stack_cap = HAND ? A.stack_cap - kHandSums : A.stack_cap;
+    double* __restrict__ own = reinterpret_cast<double*>(stk + stack_cap) + lane;
     // SHMEM_COUNT_WALK: per window, as walk_kernel counts them (node tests, monopoles and
     // particles times the window's targets, r = 0 pairs), so a paired walk counts what the two
     // one-window walks count
@@ -1123,7 +1125,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
         if (lane == 0) unit = (int)atomicAdd(SHARE ? A.hand_ctr + 1 : A.next_group, 1u);
         unit = __shfl_sync(kFull, unit, 0);
         if (unit >= n_units) break;
-        Handover* rec = SHARE ? A.hand + (whole ? unit : unit / kShares) : nullptr;
+        Handover* rec = SHARE ? A.hand + unit / kShares : nullptr;
         const int pr = SHARE ? rec->pair : unit;
         int t0[2], nt[2];
 #pragma unroll
@@ -1295,17 +1297,12 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
         // fetch, not arithmetic, limited the first version with a flush at every append site).
         // the root of each window: node 0, or in a forest its system's root; windows of one
         // system share a root entry, windows of two systems start from one entry each
-        int top = 1, bot = 0;  // the stack's entries: [bot, top), bot > 0 only after breadth-first steps
+        // the stack's entries: [bot, top), bot > 0 after breadth-first steps and above a pair's own shares
+        int top = 1, bot = 0;
         if (SHARE) {
-            // every kShares-th entry of the saved stack, or all of it with the sums so far
-            const int first = whole ? 0 : unit % kShares, every = whole ? 1 : kShares, n = rec->n;
-            top = n > first ? (n - first + every - 1) / every : 0;
-            for (int i = lane; i < top; i += 32) stk[i] = rec->stack[first + i * every];
-            if (whole) {
-                const HandSum a = rec->sum[0][lane], b = rec->sum[1][lane];
-                sx0 = a.x.x; cx0 = a.x.y; sy0 = a.y.x; cy0 = a.y.y; sz0 = a.z.x; cz0 = a.z.y; pot0 = a.pot;
-                sx1 = b.x.x; cx1 = b.x.y; sy1 = b.y.x; cy1 = b.y.y; sz1 = b.z.x; cz1 = b.z.y; pot1 = b.pot;
-            }
+            const int first = unit % kShares, n = rec->n;
+            top = n > first ? (n - first + kShares - 1) / kShares : 0;
+            for (int i = lane; i < top; i += 32) stk[i] = rec->stack[first + i * kShares];
         } else {
             const int ra = A.group_root ? A.group_root[2 * pr] : 0;
             const int rb = (A.group_root && nt[1] > 0) ? A.group_root[2 * pr + 1] : ra;
@@ -1323,6 +1320,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
         int left = HAND ? A.budget : 0;  // iterations of the budget; below 0, the stack is broken up
         int quiet = 0;                   // entries seen since one was broken up
         int slot = -1;                   // >= 0: the record asked for -- flush the lists, then save
+        int share = -1;                  // >= 0: no record was left -- the share of the stack at hand
         for (;;) {
             const bool done = base >= tot2 && (top == bot || (HAND && slot >= 0));
             if (done || max(npn0, npn1) > A.pn_cap - 32 || max(npp0, npp1) > A.pp_cap - 32) {
@@ -1338,10 +1336,27 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                         if (v) npp1 = 0; else npp0 = 0;
                     }
                 }
-                if (done) {
-                    if (!HAND || slot < A.hand_cap) break;
-                    slot = -1;  // no record left: this warp goes on from the same state
-                    left = INT_MAX;
+                if (!HAND && done) break;
+                if constexpr (HAND) if (done) {
+                    if (slot < 0 ? share < 0 : slot < A.hand_cap) break;
+                    // the sums so far are the hand-over's or those of a share: as the last share adds them
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        const double q[4] = {(double)(v ? sx1 : sx0) - (double)(v ? cx1 : cx0),
+                                             (double)(v ? sy1 : sy0) - (double)(v ? cy1 : cy0),
+                                             (double)(v ? sz1 : sz0) - (double)(v ? cz1 : cz0), v ? pot1 : pot0};
+#pragma unroll
+                        for (int c = 0; c < (WANT_POT ? 4 : 3); ++c)
+                            own[(4 * v + c) * 32] = share < 0 ? q[c] : own[(4 * v + c) * 32] + q[c];
+                    }
+                    sx0 = sy0 = sz0 = cx0 = cy0 = cz0 = sx1 = sy1 = sz1 = cx1 = cy1 = cz1 = 0.0f;
+                    pot0 = pot1 = 0.0;
+                    if (share < 0) bot = top;  // the shares are taken from [0, bot)
+                    slot = -1;
+                    if (++share == kShares) break;
+                    top = bot + (bot - share + kShares - 1) / kShares;
+                    for (int i = bot + lane; i < top; i += 32) stk[i] = stk[share + (i - bot) * kShares];
+                    __syncwarp();
                 }
             }
 
@@ -1402,7 +1417,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
             bool fifo = false;
             if (HAND && --left < 0) {
                 const bool over = left < -kHandSteps || quiet >= top - bot || top - bot > kHandStack - 256;
-                if (over || top + 256 > A.stack_cap) {  // the stack back to its start
+                if (over || top + 256 > stack_cap) {  // the stack back to its start
                     top -= bot;
                     for (int i = 0; i < top; i += 32) {
                         const int q = i + lane < top ? stk[bot + i + lane] : 0;
@@ -1479,7 +1494,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                 inc2 = warp_incl_scan_i(cnt);
             }
             const int tot = __shfl_sync(kFull, incl, 31);
-            if (top + tot > A.stack_cap) { overflow = true; break; }
+            if (top + tot > stack_cap) { overflow = true; break; }
             {
                 int* dst = stk + (top + incl - nch);
 #pragma unroll
@@ -1524,15 +1539,21 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
             q->sum[1][lane] = HandSum{make_float2(sx1, cx1), make_float2(sy1, cy1), make_float2(sz1, cz1), pot1};
             continue;
         }
-        double more[2][4] = {};  // SHARE: what is added to this share's sums, per window
-        if (SHARE && !whole) {
-            const int share = unit % kShares;
+        double more[2][4] = {};  // SHARE and HAND: what is added to the sums at hand, per window
+        if (HAND && share >= 0) {
+#pragma unroll
+            for (int v = 0; v < 2; ++v)
+#pragma unroll
+                for (int c = 0; c < (WANT_POT ? 4 : 3); ++c) more[v][c] = own[(4 * v + c) * 32];
+        }
+        if (SHARE) {
+            const int at = unit % kShares;
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
-                rec->part[share][0][v][lane] = (double)(v ? sx1 : sx0) - (double)(v ? cx1 : cx0);
-                rec->part[share][1][v][lane] = (double)(v ? sy1 : sy0) - (double)(v ? cy1 : cy0);
-                rec->part[share][2][v][lane] = (double)(v ? sz1 : sz0) - (double)(v ? cz1 : cz0);
-                if (WANT_POT) rec->part[share][3][v][lane] = v ? pot1 : pot0;
+                rec->part[at][0][v][lane] = (double)(v ? sx1 : sx0) - (double)(v ? cx1 : cx0);
+                rec->part[at][1][v][lane] = (double)(v ? sy1 : sy0) - (double)(v ? cy1 : cy0);
+                rec->part[at][2][v][lane] = (double)(v ? sz1 : sz0) - (double)(v ? cz1 : cz0);
+                if (WANT_POT) rec->part[at][3][v][lane] = v ? pot1 : pot0;
             }
             __threadfence();
             __syncwarp();
@@ -1567,11 +1588,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                 const float sx = v ? sx1 : sx0, sy = v ? sy1 : sy0, sz = v ? sz1 : sz0;
                 const float cx = v ? cx1 : cx0, cy = v ? cy1 : cy0, cz = v ? cz1 : cz0;
                 if (A.ax) {
-                    A.ax[o] = A.G * (SHARE ? (double)sx - (double)cx + more[v][0] : (double)sx - (double)cx);
-                    A.ay[o] = A.G * (SHARE ? (double)sy - (double)cy + more[v][1] : (double)sy - (double)cy);
-                    A.az[o] = A.G * (SHARE ? (double)sz - (double)cz + more[v][2] : (double)sz - (double)cz);
+                    A.ax[o] = A.G * (HAND || SHARE ? (double)sx - (double)cx + more[v][0] : (double)sx - (double)cx);
+                    A.ay[o] = A.G * (HAND || SHARE ? (double)sy - (double)cy + more[v][1] : (double)sy - (double)cy);
+                    A.az[o] = A.G * (HAND || SHARE ? (double)sz - (double)cz + more[v][2] : (double)sz - (double)cz);
                 }
-                if (WANT_POT && A.phi) A.phi[o] = A.G * (SHARE ? (v ? pot1 : pot0) + more[v][3] : v ? pot1 : pot0);
+                if (WANT_POT && A.phi) A.phi[o] = A.G * (HAND || SHARE ? (v ? pot1 : pot0) + more[v][3] : v ? pot1 : pot0);
             }
         }
     }
@@ -2484,7 +2505,8 @@ void launch_pair(gt_context* ctx, const WalkArgs& a, int blocks, int warps) {
         launch_pair_kernel<POT, CNT, MAC, false, false>(ctx, a, blocks, warps);
     } else {
         launch_pair_kernel<POT, CNT, MAC, true, false>(ctx, a, blocks, warps);
-        launch_pair_kernel<POT, CNT, MAC, false, true>(ctx, a, share_grid(ctx, a.hand_cap, warps), warps);
+        if (a.hand_cap > 0)
+            launch_pair_kernel<POT, CNT, MAC, false, true>(ctx, a, share_grid(ctx, a.hand_cap, warps), warps);
     }
 }
 
@@ -2838,9 +2860,9 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     }
     const int64_t want_blocks = ((paired ? (ng + 1) / 2 : packed ? n_packs : ng) + warps - 1) / warps;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want_blocks, (int64_t)per_sm * ctx->num_sms));
-    // a breadth-first stack of a long window lies below the depth-first levels
+    // a breadth-first stack of a long window, and a share taken from it, lie below the depth-first levels
     int stack_cap = rq.stack_capacity > 0 ? rq.stack_capacity : 256 * std::max(1, t->n_levels) + 32;
-    if (budget > 0) stack_cap += kHandStack;
+    if (budget > 0) stack_cap += kHandStack + kHandStack / kShares + kHandSums;
     stack_cap = (stack_cap + 31) & ~31;
 
     WalkArgs a;
@@ -2900,19 +2922,28 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     a.packs = packs;
     a.n_packs = (int)n_packs;
     a.budget = budget;
-    a.hand_cap = hand_cap;
     a.hand_size = (int)std::max<int64_t>(64, t->n_live / t->n_systems / 256);
     a.hand_ctr = (unsigned int*)(ctr + kCtrHand);
-    a.hand = nullptr;
+    // records that the device has no room for are done without: every pair then walks its own shares
     const size_t hand_bytes = (size_t)hand_cap * sizeof(Handover);
-    if (budget > 0) {
-        if (wb) {
-            own((void**)&wb->hand, wb->hand_bytes, hand_bytes);
-            a.hand = (Handover*)wb->hand;
-        } else {
-            a.hand = (Handover*)scratch(ctx, kSlotHand, hand_bytes);
+    auto records = [&](Slot slot, Handover*& p) {
+        p = nullptr;
+        if (hand_cap <= 0) return 0;
+        try {
+            if (!wb) {
+                p = (Handover*)scratch(ctx, slot, hand_bytes);
+            } else {
+                if (rq.capture && wb->hand_bytes < hand_bytes) return 0;  // nor had the walk before
+                own((void**)&wb->hand, wb->hand_bytes, hand_bytes);
+                p = (Handover*)wb->hand;
+            }
+        } catch (const Fail& f) {
+            if (f.status != GT_ERR_NOMEM) throw;
+            return 0;
         }
-    }
+        return hand_cap;
+    };
+    a.hand_cap = records(kSlotHand, a.hand);
     a.next_group = (unsigned int*)(ctr + 8);
     a.stats = ctr;
     a.error = (int*)(ctr + 9);
@@ -3004,7 +3035,9 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         const bool two = wb == nullptr;
         cudaStream_t cs[2] = {st, two ? ctx->walk2 : st};
         int* stacks[2] = {a.stack, two ? (int*)scratch(ctx, kSlotStack2, stack_bytes) : a.stack};
-        Handover* hands[2] = {a.hand, two && budget > 0 ? (Handover*)scratch(ctx, kSlotHand2, hand_bytes) : a.hand};
+        Handover* hands[2] = {a.hand, a.hand};
+        int hand_caps[2] = {a.hand_cap, a.hand_cap};
+        if (two) hand_caps[1] = records(kSlotHand2, hands[1]);
         check_cuda(cudaEventRecord(ctx->ev0, st), "event");
         if (two) {
             check_cuda(cudaEventRecord(ctx->walk2_start, st), "event");
@@ -3025,6 +3058,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
                 WalkArgs ac = a;
                 ac.stack = stacks[c & 1];
                 ac.hand = hands[c & 1];
+                ac.hand_cap = hand_caps[c & 1];
                 ac.hand_ctr = (unsigned int*)(ctr + kCtrHand + c);
                 if (packed) {
                     ac.packs = packs + g0;

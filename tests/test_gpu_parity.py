@@ -389,6 +389,32 @@ def test_long_windows_handed_over(gpu_ctx, oracle, n):
     assert np.median(e) <= 1e-6 and e.max() <= 1e-4
 
 
+def test_handed_over_windows_do_not_depend_on_the_launch(gpu_ctx):
+    """Windows of scattered targets, of which every one outgrows its budget: 4688 pairs ask for 2048 records
+    when the walk is one launch (device arrays), and no launch runs out when it is five (host arrays) or
+    a slice of the targets.  Who gets a record differs from run to run; the bits do not.  Against one
+    window per warp only the order of the FP32 sums differs."""
+    import torch
+
+    n, nt = 400000, 300000
+    T = gpu_ctx.build(ics.plummer(n=n, seed=12), key_mode=g.GT_KEY_MORTON)
+    tg = np.random.default_rng(1).permutation(n)[:nt].astype(np.uint32)
+    kw = dict(batch=32, group_mode=g.GT_GROUP_BATCH, want_phi=True)
+    aold = gpu_ctx.form_aold(*gpu_ctx.accel_grouped(T, None, theta=0.7, batch=32, group_mode=g.GT_GROUP_BATCH,
+                                                    out_order=g.GT_OUT_ORIGINAL), 0.0025)[tg]
+    dt, da = torch.as_tensor(tg.view(np.int32), device="cuda"), torch.as_tensor(aold, device="cuda")
+    host = gpu_ctx.accel_grouped(T, tg, aold=aold, **kw)
+    runs = [[q.cpu().numpy() for q in gpu_ctx.accel_grouped(T, dt, aold=da, **kw)] for _ in range(3)]
+    part = gpu_ctx.accel_grouped(T, tg[64000:96000], aold=aold[64000:96000], **kw)
+    one = [q.cpu().numpy() for q in gpu_ctx.accel_grouped(T, dt, aold=da, window_pairs=False, **kw)]
+    for k in range(4):
+        for r in runs:
+            assert np.array_equal(r[k], host[k])
+        assert np.array_equal(part[k], host[k][64000:96000])
+    e = relerr(*host[:3], *one[:3])
+    assert np.median(e) <= 1e-6 and e.max() <= 1e-4
+
+
 @pytest.mark.parametrize("ics_kind", ["plummer", "clumps", "collocated"])
 @pytest.mark.parametrize("batch", [0, 5, 8, 16])
 def test_packs_match_single_groups(gpu_ctx, ics_kind, batch):
