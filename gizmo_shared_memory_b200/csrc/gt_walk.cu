@@ -94,15 +94,21 @@ struct WalkArgs {
     const double* smass;
     const uint32_t* nsink;
     double sink_r;
-    // long windows (walk_pair_kernel, see Handover): iterations after which a pair hands the rest of
-    // its traversal over, the records, and the counters: [0] records asked for, [1] shares taken
     // packs of groups (walk_pack_kernel): first group and number of groups
     const int2* packs;
     int n_packs;
+    // long windows (walk_pair_kernel, see Handover): iterations after which a pair hands the rest of its
+    // traversal over, the size from which subtrees are broken up first, the least entries of a stack worth
+    // it and of a share, the records (hand_cap of them) and the counters: [0] records asked for, [1]
+    // shares taken
     int budget;
+    int hand_size;
+    int hand_least;
+    int share_least;
+    int shares;       // of a record, at most
     int hand_cap;
-    int hand_size;  // subtrees of at most this many particles are not broken up further
-    struct Handover* hand;
+    char* hand;
+    int hand_stride;  // bytes
     unsigned int* hand_ctr;
 };
 
@@ -110,28 +116,26 @@ struct WalkArgs {
 // the average number of nodes in its one warp, while the rest of the GPU has nothing left to do: in a
 // Plummer sphere of 65,536 particles the longest pair of windows takes 1,800 iterations against a mean
 // of 60, and the walk took as long as that pair.  A pair that has used up its budget of iterations
-// therefore breaks up the large subtrees on its stack (a depth-first stack has a few that hold most of
-// what is left at its bottom), writes its state here and leaves it: a second launch walks every record
-// in kShares shares, each with every kShares-th stack entry, and the share that finishes last adds the
-// parts in a fixed order.  A pair that finds no record left walks the same shares itself, one after
-// another, and adds their sums in the same order.  So what is handed over, how it is shared out and
-// how it is summed depend on the pair's own particles alone: not on which pairs got the records, on
-// how many asked in the same launch, or on how many there are.
-constexpr int kShares = 16;
-constexpr int kHandStack = 2048;   // entries of a record
-constexpr int kHandSteps = 96;     // at most this many steps break up the stack
-constexpr int kHandLeast = 4 * kShares;  // a shorter stack is not worth a record
+// therefore breaks up the large subtrees on its stack, writes its state here and leaves it: a second
+// launch walks every record in up to A.shares shares, each with every so many-th stack entry, and the
+// share that finishes last adds the parts in a fixed order.  A pair that finds no record left walks the same
+// shares itself, one after another, and adds their sums in the same order.  So what is handed over,
+// how it is shared out and how it is summed depend on the pair's own particles and the tree alone: not
+// on which pairs got the records, on how many asked in the same launch, or on how many there are.
+constexpr int kHandStack = 2048;    // entries of a record
+constexpr int kHandSteps = 64;      // at most this many steps break up the stack
+constexpr int kHandShare = 256;     // entries of a share at most: 2048 in eight, or a sixteenth
 constexpr int kHandSums = 2 * 4 * 32 * 2;  // stack entries that hold a pair's sums while it walks its own shares
 struct HandSum {
     float2 x, y, z;  // Kahan sum and compensation
     double pot;
 };
 struct Handover {
-    int pair, n;
-    unsigned int done, pad;
+    int pair, n, shares;
+    unsigned int done;
     int stack[kHandStack];
     HandSum sum[2][32];                 // per window and lane, at the hand-over
-    double part[kShares][4][2][32];     // each share's sums: x, y, z, potential
+    // then each share's sums, double [x, y, z and with it the potential][window][lane]
 };
 
 __device__ __forceinline__ int warp_incl_scan_i(int v) {
@@ -1085,7 +1089,48 @@ struct alignas(16) PairHdr {
     // per window, in one 64-byte record: box centre and half width per axis side by side (one
     // 16-byte shared-memory load per axis of a box gap), largest target softening, smallest aold
     struct alignas(16) Win { double c_x, w_x, c_y, w_y, c_z, w_z, emax, amin; } wb[2];
+    // HAND, kept here since the loop has no registers to spare (six more made it 15 % slower): stack
+    // entries below `from` are small; the share at hand of a pair without a record (-1: none) of the
+    // n entries it set aside
+    int from, share, n, shares;
+    int cap, pad[3];  // of the stack
 };
+
+// Up to 32 interior nodes of more than `size` particles to the top of a stack of `top` entries, the
+// others below them in their order; returns their number.  Entries below *from are known to be small.
+// Every lane of the warp calls it; buf: 32 ints of shared memory.
+__device__ __noinline__ int large_first(const GNode* __restrict__ nodes, int64_t n_nodes, int size, int* stk, int top,
+                                        int* from, int* buf) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    int found = 0, out = *from, seen = out;
+    __syncwarp();
+    for (int i = out; i < top; i += 32) {
+        const bool live = i + lane < top;
+        const int e = live ? stk[i + lane] : 0;
+        bool large = false;
+        if (live && found < 32 && (int64_t)(e >> 2) < n_nodes) {
+            const int4 d = __ldg(reinterpret_cast<const int4*>(nodes + (e >> 2)) + 3);  // first, nchild, plo, phi
+            large = d.x >= 0 && d.w - d.z > size;
+        }
+        const int at = found + __popc(__ballot_sync(kFull, large) & lt_mask);
+        const bool take = large && at < 32;
+        const unsigned keep = __ballot_sync(kFull, live && !take);
+        __syncwarp();  // every lane has read its entry
+        if (take) buf[at] = e;
+        if (live && !take && (found > 0 || keep != kFull)) stk[out + __popc(keep & lt_mask)] = e;
+        __syncwarp();
+        const int before = found;
+        found += __popc(__ballot_sync(kFull, take));
+        out += __popc(keep);
+        if (found < 32) seen = out;
+        else if (before < 32) seen = min(seen, out);
+    }
+    if (lane < found) stk[out + lane] = buf[lane];
+    if (lane == 0) *from = seen;
+    __syncwarp();
+    return found;
+}
 
 __host__ __device__ constexpr int pair_list_bytes(int pn_cap, int pp_cap) { return pn_cap * 16 + pp_cap * 20; }
 __host__ __device__ constexpr int pair_smem_bytes(int pn_cap, int pp_cap) {
@@ -1110,10 +1155,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
     auto ph_of = [&](int v) { return reinterpret_cast<float*>(pp_of(v) + A.pp_cap); };
     const int n_groups = A.n_groups_dev ? (int)*A.n_groups_dev : A.n_groups;
     // SHARE: the units are the records' shares
-    const int n_units = SHARE ? min((int)A.hand_ctr[0], A.hand_cap) * kShares : (n_groups + 1) >> 1;
-    // HAND: past the traversal's entries, the sums of a pair that walks its own shares
-    const int stack_cap = HAND ? A.stack_cap - kHandSums : A.stack_cap;
-    double* __restrict__ own = reinterpret_cast<double*>(stk + stack_cap) + lane;
+    const int n_units = SHARE ? min((int)A.hand_ctr[0], A.hand_cap) * A.shares : (n_groups + 1) >> 1;
+    // HAND: the sums of a pair that walks its own shares lie past the stack, and the entries it took them
+    // from in the stack's last kHandStack entries, which it no longer needs then
+    const int sums = A.stack_cap - kHandSums;
+    auto record = [&](int i) { return reinterpret_cast<Handover*>(A.hand + (size_t)i * A.hand_stride); };
     // SHMEM_COUNT_WALK: per window, as walk_kernel counts them (node tests, monopoles and
     // particles times the window's targets, r = 0 pairs), so a paired walk counts what the two
     // one-window walks count
@@ -1125,8 +1171,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
         if (lane == 0) unit = (int)atomicAdd(SHARE ? A.hand_ctr + 1 : A.next_group, 1u);
         unit = __shfl_sync(kFull, unit, 0);
         if (unit >= n_units) break;
-        Handover* rec = SHARE ? A.hand + unit / kShares : nullptr;
-        const int pr = SHARE ? rec->pair : unit;
+        if (SHARE && unit % A.shares >= record(unit / A.shares)->shares) continue;
+        const int pr = SHARE ? record(unit / A.shares)->pair : unit;
         int t0[2], nt[2];
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
@@ -1297,12 +1343,12 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
         // fetch, not arithmetic, limited the first version with a flush at every append site).
         // the root of each window: node 0, or in a forest its system's root; windows of one
         // system share a root entry, windows of two systems start from one entry each
-        // the stack's entries: [bot, top), bot > 0 after breadth-first steps and above a pair's own shares
-        int top = 1, bot = 0;
+        int top = 1;
         if (SHARE) {
-            const int first = unit % kShares, n = rec->n;
-            top = n > first ? (n - first + kShares - 1) / kShares : 0;
-            for (int i = lane; i < top; i += 32) stk[i] = rec->stack[first + i * kShares];
+            const Handover* rec = record(unit / A.shares);
+            const int first = unit % A.shares, every = rec->shares;
+            top = (rec->n - first + every - 1) / every;
+            for (int i = lane; i < top; i += 32) stk[i] = rec->stack[first + i * every];
         } else {
             const int ra = A.group_root ? A.group_root[2 * pr] : 0;
             const int rb = (A.group_root && nt[1] > 0) ? A.group_root[2 * pr + 1] : ra;
@@ -1313,16 +1359,15 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                 top = 2;
             }
         }
+        if (HAND && lane == 0) { S.from = 0; S.share = -1; S.cap = sums; }
         __syncwarp();
         int npn0 = 0, npn1 = 0, npp0 = 0, npp1 = 0;
         int base = 0, tot2 = 0;  // the expanded leaves' particles still to place: [base, tot2)
         bool overflow = false;
-        int left = HAND ? A.budget : 0;  // iterations of the budget; below 0, the stack is broken up
-        int quiet = 0;                   // entries seen since one was broken up
-        int slot = -1;                   // >= 0: the record asked for -- flush the lists, then save
-        int share = -1;                  // >= 0: no record was left -- the share of the stack at hand
+        // iterations of the budget; below 0 the stack is broken up, at INT_MIN it is handed over
+        int left = HAND ? A.budget : 0;
         for (;;) {
-            const bool done = base >= tot2 && (top == bot || (HAND && slot >= 0));
+            const bool done = base >= tot2 && (top == 0 || (HAND && left == INT_MIN));
             if (done || max(npn0, npn1) > A.pn_cap - 32 || max(npp0, npp1) > A.pp_cap - 32) {
 #pragma unroll 1
                 for (int v = 0; v < 2; ++v) {
@@ -1338,9 +1383,36 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                 }
                 if (!HAND && done) break;
                 if constexpr (HAND) if (done) {
-                    if (slot < 0 ? share < 0 : slot < A.hand_cap) break;
-                    // the sums so far are the hand-over's or those of a share: as the last share adds them
-#pragma unroll
+                    const int share = S.share;
+                    if (left == INT_MIN) {
+                        int slot = 0;
+                        if (lane == 0) slot = (int)atomicAdd(A.hand_ctr, 1u);
+                        slot = __shfl_sync(kFull, slot, 0);
+                        const bool have = slot < A.hand_cap;
+                        const int shares = min(A.shares, top / A.share_least);
+                        int* set = have ? record(slot)->stack : stk + (sums - kHandStack);
+                        for (int i = (top - 1) & ~31; i >= 0; i -= 32) {  // from the end: the two may overlap
+                            const int e = i + lane < top ? stk[i + lane] : 0;
+                            __syncwarp();
+                            if (i + lane < top) set[i + lane] = e;
+                            __syncwarp();
+                        }
+                        if (have) {
+                            Handover* q = record(slot);
+                            if (lane == 0) { q->pair = pr; q->n = top; q->shares = shares; q->done = 0u; }
+                            q->sum[0][lane] = HandSum{make_float2(sx0, cx0), make_float2(sy0, cy0), make_float2(sz0, cz0), pot0};
+                            q->sum[1][lane] = HandSum{make_float2(sx1, cx1), make_float2(sy1, cy1), make_float2(sz1, cz1), pot1};
+                            break;
+                        }
+                        left = INT_MAX;
+                        if (lane == 0) { S.n = top; S.shares = shares; S.cap = sums - kHandStack; }
+                    } else if (share < 0) {
+                        break;
+                    }
+                    // No record was left: the sums so far, the hand-over's and then each share's, are added
+                    // as the share that finishes last adds them.
+                    double* own = reinterpret_cast<double*>(stk + sums) + lane;
+#pragma unroll 1
                     for (int v = 0; v < 2; ++v) {
                         const double q[4] = {(double)(v ? sx1 : sx0) - (double)(v ? cx1 : cx0),
                                              (double)(v ? sy1 : sy0) - (double)(v ? cy1 : cy0),
@@ -1351,11 +1423,12 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                     }
                     sx0 = sy0 = sz0 = cx0 = cy0 = cz0 = sx1 = sy1 = sz1 = cx1 = cy1 = cz1 = 0.0f;
                     pot0 = pot1 = 0.0;
-                    if (share < 0) bot = top;  // the shares are taken from [0, bot)
-                    slot = -1;
-                    if (++share == kShares) break;
-                    top = bot + (bot - share + kShares - 1) / kShares;
-                    for (int i = bot + lane; i < top; i += 32) stk[i] = stk[share + (i - bot) * kShares];
+                    __syncwarp();
+                    if (lane == 0) S.share = share + 1;
+                    const int every = S.shares;
+                    if (share + 1 == every) break;
+                    top = (S.n - (share + 1) + every - 1) / every;
+                    for (int i = lane; i < top; i += 32) stk[i] = stk[sums - kHandStack + share + 1 + i * every];
                     __syncwarp();
                 }
             }
@@ -1414,46 +1487,24 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
             }
 
             // one traversal step: pop up to 32 nodes, test each against its windows
-            bool fifo = false;
+            int npop = min(top, 32);
             if (HAND && --left < 0) {
-                const bool over = left < -kHandSteps || quiet >= top - bot || top - bot > kHandStack - 256;
-                if (over || top + 256 > stack_cap) {  // the stack back to its start
-                    top -= bot;
-                    for (int i = 0; i < top; i += 32) {
-                        const int q = i + lane < top ? stk[bot + i + lane] : 0;
-                        __syncwarp();
-                        if (i + lane < top) stk[i + lane] = q;
-                        __syncwarp();
-                    }
-                    bot = 0;
-                }
-                if (over) {
-                    left = INT_MAX;
-                    if (top >= kHandLeast && top <= kHandStack) {
-                        if (lane == 0) slot = (int)atomicAdd(A.hand_ctr, 1u);
-                        slot = __shfl_sync(kFull, slot, 0);
-                        continue;
-                    }
+                const int n = left >= -kHandSteps && top <= kHandStack - 256
+                                  ? large_first(A.nodes, A.n_nodes, A.hand_size, stk, top, &S.from, S.lo) : 0;
+                if (n > 0) {
+                    npop = n;
                 } else {
-                    fifo = true;
+                    left = top >= A.hand_least && top <= kHandStack ? INT_MIN : INT_MAX;
+                    if (left == INT_MIN) continue;
                 }
             }
-            const int npop = min(top - bot, 32);
-            if (!fifo) top -= npop;
-            const int from = fifo ? bot : top;
-            if (fifo) bot += npop;
-            const int ent = lane < npop ? stk[from + lane] : -1;
+            top -= npop;
+            const int ent = lane < npop ? stk[top + lane] : -1;
             int node = ent >= 0 ? (ent >> 2) : -1;
             if (node >= 0 && !GT_IN_BOUNDS(node, A.n_nodes)) node = -1;
-            int mk = node >= 0 ? (ent & 3) : 0;
+            const int mk = node >= 0 ? (ent & 3) : 0;
             __syncwarp();
             const NodeV nd = load_node(A.nodes + (node >= 0 ? node : 0));
-            // a subtree small enough for one share goes back to the stack as it is
-            const bool keep = HAND && fifo && node >= 0 && nd.phi - nd.plo <= A.hand_size;
-            if (HAND && fifo) {
-                if (keep) mk = 0;
-                quiet = __any_sync(kFull, node >= 0 && !keep) ? 0 : quiet + npop;
-            }
             const bool leaf = nd.first < 0;
             if (COUNT) {
                 const unsigned tests = __reduce_add_sync(kFull, (unsigned)__popc(mk));
@@ -1482,7 +1533,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
 
             // children of opened interior nodes, with the windows that opened them; one scan for
             // the children's stack slots and the expanded leaves' particle slots (walk_kernel)
-            const int nch = keep ? 1 : push ? nd.nchild : 0;
+            const int nch = push ? nd.nchild : 0;
             const int cnt = expand ? nd.phi - nd.plo : 0;
             int incl, inc2;
             if (!__any_sync(kFull, cnt >= (1 << 16))) {
@@ -1494,12 +1545,12 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                 inc2 = warp_incl_scan_i(cnt);
             }
             const int tot = __shfl_sync(kFull, incl, 31);
-            if (top + tot > stack_cap) { overflow = true; break; }
+            if (top + tot > (HAND ? S.cap : A.stack_cap)) { overflow = true; break; }
             {
                 int* dst = stk + (top + incl - nch);
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
-                    if (c < nch) dst[c] = keep ? ent : ((nd.first + c) << 2) | pm;
+                    if (c < nch) dst[c] = ((nd.first + c) << 2) | pm;
             }
             top += tot;
             if (COUNT) c_maxtop = max(c_maxtop, top);
@@ -1531,36 +1582,34 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
             continue;
         }
 
-        if (HAND && slot >= 0) {
-            Handover* q = A.hand + slot;
-            if (lane == 0) { q->pair = pr; q->n = top; q->done = 0u; }
-            for (int i = lane; i < top; i += 32) q->stack[i] = stk[i];
-            q->sum[0][lane] = HandSum{make_float2(sx0, cx0), make_float2(sy0, cy0), make_float2(sz0, cz0), pot0};
-            q->sum[1][lane] = HandSum{make_float2(sx1, cx1), make_float2(sy1, cy1), make_float2(sz1, cz1), pot1};
-            continue;
-        }
+        if (HAND && left == INT_MIN) continue;  // handed over
         double more[2][4] = {};  // SHARE and HAND: what is added to the sums at hand, per window
-        if (HAND && share >= 0) {
+        if (HAND && S.share >= 0) {
+            const double* own = reinterpret_cast<const double*>(stk + sums) + lane;
 #pragma unroll
             for (int v = 0; v < 2; ++v)
 #pragma unroll
                 for (int c = 0; c < (WANT_POT ? 4 : 3); ++c) more[v][c] = own[(4 * v + c) * 32];
         }
         if (SHARE) {
-            const int at = unit % kShares;
+            constexpr int kSums = WANT_POT ? 4 : 3;
+            Handover* rec = record(unit / A.shares);
+            double(*part)[kSums][2][32] = reinterpret_cast<double(*)[kSums][2][32]>(rec + 1);
+            const int shares = rec->shares;
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
-                rec->part[at][0][v][lane] = (double)(v ? sx1 : sx0) - (double)(v ? cx1 : cx0);
-                rec->part[at][1][v][lane] = (double)(v ? sy1 : sy0) - (double)(v ? cy1 : cy0);
-                rec->part[at][2][v][lane] = (double)(v ? sz1 : sz0) - (double)(v ? cz1 : cz0);
-                if (WANT_POT) rec->part[at][3][v][lane] = v ? pot1 : pot0;
+                double(*q)[2][32] = part[unit % A.shares];
+                q[0][v][lane] = (double)(v ? sx1 : sx0) - (double)(v ? cx1 : cx0);
+                q[1][v][lane] = (double)(v ? sy1 : sy0) - (double)(v ? cy1 : cy0);
+                q[2][v][lane] = (double)(v ? sz1 : sz0) - (double)(v ? cz1 : cz0);
+                if (WANT_POT) q[kSums - 1][v][lane] = v ? pot1 : pot0;
             }
             __threadfence();
             __syncwarp();
             unsigned int before = 0;
             if (lane == 0) before = atomicAdd(&rec->done, 1u);
             before = __shfl_sync(kFull, before, 0);
-            if (before != kShares - 1) continue;
+            if ((int)before != shares - 1) continue;
             __threadfence();
             // the last share: the sums at the hand-over, then all shares in order (its own too)
             sx0 = sy0 = sz0 = cx0 = cy0 = cz0 = sx1 = sy1 = sz1 = cx1 = cy1 = cz1 = 0.0f;
@@ -1572,9 +1621,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                 more[v][1] = (double)a.y.x - (double)a.y.y;
                 more[v][2] = (double)a.z.x - (double)a.z.y;
                 more[v][3] = a.pot;
-                for (int q = 0; q < kShares; ++q)
+                for (int q = 0; q < shares; ++q)
 #pragma unroll
-                    for (int c = 0; c < (WANT_POT ? 4 : 3); ++c) more[v][c] += __ldcg(&rec->part[q][c][v][lane]);
+                    for (int c = 0; c < kSums; ++c) more[v][c] += __ldcg(&part[q][c][v][lane]);
             }
         }
 
@@ -2462,7 +2511,6 @@ constexpr int kPairCapDefault = 160;
 
 size_t pair_smem(int warps, int pn_cap) { return (size_t)warps * pair_smem_bytes(pn_cap, pn_cap / 2); }
 
-constexpr int kHandRecords = 2048;  // 90 MB
 
 template <bool POT, bool CNT, int MAC, bool HAND, bool SHARE>
 void prepare_pair() {
@@ -2487,8 +2535,8 @@ int pair_occupancy(int warps, int pn_cap) {
 }
 
 // Blocks of the launch that walks the records' shares, their number known on the device only.
-int share_grid(gt_context* ctx, int records, int warps) {
-    const int64_t units = (int64_t)records * kShares;
+int share_grid(gt_context* ctx, int records, int shares, int warps) {
+    const int64_t units = (int64_t)records * shares;
     return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * 3, (units + warps - 1) / warps));
 }
 
@@ -2506,7 +2554,7 @@ void launch_pair(gt_context* ctx, const WalkArgs& a, int blocks, int warps) {
     } else {
         launch_pair_kernel<POT, CNT, MAC, true, false>(ctx, a, blocks, warps);
         if (a.hand_cap > 0)
-            launch_pair_kernel<POT, CNT, MAC, false, true>(ctx, a, share_grid(ctx, a.hand_cap, warps), warps);
+            launch_pair_kernel<POT, CNT, MAC, false, true>(ctx, a, share_grid(ctx, a.hand_cap, a.shares, warps), warps);
     }
 }
 
@@ -2843,26 +2891,33 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
                : macn ? occupancy_blocks<4, true, false, false, 2>(warps, pn_cap)
                       : occupancy_blocks<4, true, false, false, 0>(warps, pn_cap);
     // Long windows hand over (Handover) where a walk of the whole tree lasts about as long as its longest
-    // pair: fewer than two pairs per resident warp.  Where a third of the warps would have a pair the
-    // budget is 32 iterations, half a pair's mean, and the idle warps take the rest; up to a record for
-    // every pair it is 96, and 192 beyond, which a few per cent of the pairs reach.  Plummer spheres of
-    // 9,000, 65,536 and 300,000: 0.27, 0.70 and 0.71 ms (no hand-over, the last two: 4.6 and 1.01; a
-    // budget of 96, the first two: 0.42 and 0.82); a galaxy of 100,000: 0.469 ms (0.495; 0.50 at 32).
-    // With more pairs the GPU is busy to the end and the
-    // hand-over only adds work: 5.8 -> 6.3 ms for a galaxy of 2^22 at 256.  The rule reads the tree's
-    // size and not the call's targets, so a slice of the targets is walked as it is in the whole.
+    // pair: fewer than two pairs per resident warp.  Trees of fewer than 40 pairs keep theirs: the second
+    // launch's 12 us are a tenth of their walk.  The fewer the pairs, the more warps wait for work, and
+    // the sooner and the finer a pair is split; with more pairs than resident warps a share of fewer than
+    // 64 entries is not worth its ramp-up.  The rule reads the tree's size and not the call's targets, so
+    // a slice of the targets is walked as it is in the whole.  Device time of whole calls without and
+    // with it, ms, at alpha 0.0025 and 0.000025: Plummer spheres of 20,000 particles 1.44 -> 0.32 and
+    // 1.73 -> 0.40, of 65,536 0.84 -> 0.34 and 3.92 -> 0.94, of 150,000 6.16 -> 0.99 and 9.25 -> 2.02, of
+    // 300,000 1.29 -> 0.88 and 10.1 -> 4.4, of 440,000 1.24 -> 1.11 and 10.2 -> 6.0; galaxies of 100,000
+    // 0.64 -> 0.45 and 3.05 -> 1.23, of 300,000 0.76 -> 0.79 and 4.25 -> 3.91; clustered boxes of 150,000
+    // 0.66 -> 0.56 and 3.35 -> 1.85, of 440,000 1.29 -> 1.22 and 7.7 -> 5.5.  At 4 windows per warp
+    // (2^22 particles) the hand-over only adds work.
     const int64_t tree_units = paired ? ((t->n_live + param - 1) / param + 1) / 2 : 0;
     const int64_t units = ((all || t->n_systems > 1 ? ng : (nt + param - 1) / std::max(1, param)) + 1) / 2;
-    int budget = 0, hand_cap = 0;
-    if (paired && tree_units < (int64_t)2 * 24 * ctx->num_sms) {
-        hand_cap = (int)std::min<int64_t>(units, kHandRecords);
-        budget = tree_units <= (int64_t)8 * ctx->num_sms ? 32 : tree_units <= kHandRecords ? 96 : 192;
+    const int64_t resident = (int64_t)24 * ctx->num_sms;
+    int budget = 0, hand_least = 64, share_least = 4, shares = 16;
+    if (paired && tree_units >= 40 && tree_units < 2 * resident) {
+        budget = tree_units <= resident / 3 ? 32 : tree_units <= resident * 3 / 5 ? 96 : 192;
+        if (tree_units > resident) { hand_least = 256; share_least = 64; shares = 8; }
     }
+    // a record for every pair, within reason: a list of targets can name more windows than the tree has
+    const int hand_cap = budget > 0 ? (int)std::min<int64_t>(units, 2 * resident) : 0;
+    const int hand_stride = (int)sizeof(Handover) + shares * (rq.want_phi && rq.phi ? 4 : 3) * 2 * 32 * 8;
     const int64_t want_blocks = ((paired ? (ng + 1) / 2 : packed ? n_packs : ng) + warps - 1) / warps;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want_blocks, (int64_t)per_sm * ctx->num_sms));
-    // a breadth-first stack of a long window, and a share taken from it, lie below the depth-first levels
+    // room to break up a long pair's stack, or for a share and the entries it is taken from; and its sums
     int stack_cap = rq.stack_capacity > 0 ? rq.stack_capacity : 256 * std::max(1, t->n_levels) + 32;
-    if (budget > 0) stack_cap += kHandStack + kHandStack / kShares + kHandSums;
+    if (budget > 0) stack_cap += kHandShare + kHandStack + kHandSums;
     stack_cap = (stack_cap + 31) & ~31;
 
     WalkArgs a;
@@ -2885,7 +2940,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     a.phi = rq.phi;
     a.out_map = (all && rq.out_original) ? t->order : nullptr;
     // a warp of either launch needs a traversal stack
-    const int total_warps = std::max(blocks, budget > 0 ? share_grid(ctx, hand_cap, warps) : 0) * warps;
+    const int total_warps = std::max(blocks, budget > 0 ? share_grid(ctx, hand_cap, shares, warps) : 0) * warps;
     a.pn_cap = pn_cap;
     a.pp_cap = pn_cap / 2;
     a.warp_bytes = paired ? pair_smem_bytes(a.pn_cap, a.pp_cap) : warp_smem_bytes(a.pn_cap, a.pp_cap, ext);
@@ -2922,28 +2977,34 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     a.packs = packs;
     a.n_packs = (int)n_packs;
     a.budget = budget;
+    a.hand_least = hand_least;
+    a.share_least = share_least;
+    a.shares = shares;
+    a.hand_stride = hand_stride;
     a.hand_size = (int)std::max<int64_t>(64, t->n_live / t->n_systems / 256);
     a.hand_ctr = (unsigned int*)(ctr + kCtrHand);
-    // records that the device has no room for are done without: every pair then walks its own shares
-    const size_t hand_bytes = (size_t)hand_cap * sizeof(Handover);
-    auto records = [&](Slot slot, Handover*& p) {
-        p = nullptr;
-        if (hand_cap <= 0) return 0;
+    a.hand_cap = 0;
+    a.hand = nullptr;
+    // the records of one launch; those that the device has no room for are done without, and every pair
+    // then walks its own shares
+    auto records = [&](WalkArgs& w, Slot slot, int want) {
+        w.hand_cap = 0;
+        if (want <= 0) return;
+        const size_t need = (size_t)want * hand_stride;
         try {
             if (!wb) {
-                p = (Handover*)scratch(ctx, slot, hand_bytes);
+                w.hand = (char*)scratch(ctx, slot, need);
             } else {
-                if (rq.capture && wb->hand_bytes < hand_bytes) return 0;  // nor had the walk before
-                own((void**)&wb->hand, wb->hand_bytes, hand_bytes);
-                p = (Handover*)wb->hand;
+                if (rq.capture && wb->hand_bytes < need) return;  // nor had the walk before
+                own((void**)&wb->hand, wb->hand_bytes, need);
+                w.hand = (char*)wb->hand;
             }
         } catch (const Fail& f) {
             if (f.status != GT_ERR_NOMEM) throw;
-            return 0;
+            return;
         }
-        return hand_cap;
+        w.hand_cap = want;
     };
-    a.hand_cap = records(kSlotHand, a.hand);
     a.next_group = (unsigned int*)(ctr + 8);
     a.stats = ctr;
     a.error = (int*)(ctr + 9);
@@ -3035,9 +3096,16 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         const bool two = wb == nullptr;
         cudaStream_t cs[2] = {st, two ? ctx->walk2 : st};
         int* stacks[2] = {a.stack, two ? (int*)scratch(ctx, kSlotStack2, stack_bytes) : a.stack};
-        Handover* hands[2] = {a.hand, a.hand};
-        int hand_caps[2] = {a.hand_cap, a.hand_cap};
-        if (two) hand_caps[1] = records(kSlotHand2, hands[1]);
+        // two chunks in flight need their own records, as many as the longest one's pairs
+        WalkArgs on[2] = {a, a};
+        if (budget > 0) {
+            int most = 0;
+            for (int c = 0; c < kChunks; ++c) most = std::max(most, (hb[c + 1].x - hb[c].x + 1) / 2);
+            most = std::min(most, hand_cap);
+            records(on[0], kSlotHand, most);
+            if (two) records(on[1], kSlotHand2, most);
+            else on[1] = on[0];
+        }
         check_cuda(cudaEventRecord(ctx->ev0, st), "event");
         if (two) {
             check_cuda(cudaEventRecord(ctx->walk2_start, st), "event");
@@ -3053,12 +3121,10 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
                     gt_context* c;
                     cudaStream_t old;
                     ~OnStream() { c->stream = old; }
-                } on{ctx, ctx->stream};
+                } restore{ctx, ctx->stream};
                 ctx->stream = s;
-                WalkArgs ac = a;
+                WalkArgs ac = on[c & 1];
                 ac.stack = stacks[c & 1];
-                ac.hand = hands[c & 1];
-                ac.hand_cap = hand_caps[c & 1];
                 ac.hand_ctr = (unsigned int*)(ctr + kCtrHand + c);
                 if (packed) {
                     ac.packs = packs + g0;
@@ -3119,6 +3185,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         return true;
     }
 
+    records(a, kSlotHand, hand_cap);
     for (int attempt = 0; attempt < 3; ++attempt) {
         const size_t stack_bytes = (size_t)total_warps * stack_cap * 4;
         if (wb) {

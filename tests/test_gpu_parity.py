@@ -390,15 +390,16 @@ def test_long_windows_handed_over(gpu_ctx, oracle, n):
 
 
 def test_handed_over_windows_do_not_depend_on_the_launch(gpu_ctx):
-    """Windows of scattered targets, of which every one outgrows its budget: 4688 pairs ask for 2048 records
-    when the walk is one launch (device arrays), and no launch runs out when it is five (host arrays) or
-    a slice of the targets.  Who gets a record differs from run to run; the bits do not.  Against one
-    window per warp only the order of the FP32 sums differs."""
+    """Windows of scattered targets, of which every one outgrows its budget: 9375 pairs ask for the 7104
+    records that 148 SMs have when the walk is one launch (device arrays), and no launch runs out when it
+    is five (host arrays) or a slice of the targets.  Who gets a record differs from run to run; the bits
+    do not.  Against one window per warp only the order of the FP32 sums differs."""
     import torch
 
-    n, nt = 400000, 300000
+    n, nt = 400000, 600000
     T = gpu_ctx.build(ics.plummer(n=n, seed=12), key_mode=g.GT_KEY_MORTON)
-    tg = np.random.default_rng(1).permutation(n)[:nt].astype(np.uint32)
+    tg = np.random.default_rng(1).permutation(n).astype(np.uint32)
+    tg = np.concatenate([tg, tg[:nt - n]])
     kw = dict(batch=32, group_mode=g.GT_GROUP_BATCH, want_phi=True)
     aold = gpu_ctx.form_aold(*gpu_ctx.accel_grouped(T, None, theta=0.7, batch=32, group_mode=g.GT_GROUP_BATCH,
                                                     out_order=g.GT_OUT_ORIGINAL), 0.0025)[tg]
