@@ -2795,9 +2795,13 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
             c.mode = mode; c.param = param; c.kmax = kmax; c.groups = groups; c.roots = roots; c.n_groups = ng;
             t->group_cache.push_back(c);
         }
-        // a pack's walk takes about twice as long as a leaf's, and there are six times fewer: with fewer
-        // than eight groups per resident warp the groups finish sooner side by side
-        packed = packed && ng >= (int64_t)8 * 24 * ctx->num_sms;
+        // A pack's walk takes about twice as long as a leaf's, there are six times fewer, and the longest one
+        // (the outskirts of a halo) as long as all its leaves': with fewer groups per resident warp it is
+        // what the walk waits for.  Packed against one warp per leaf, aold at 0.0025 and at a tenth:
+        // Plummer spheres 1.11 and 1.15 at 17 groups per warp (300,000 particles), 1.04 and 1.04 at 21,
+        // 0.82 and 0.79 at 24, 0.69 and 0.65 at 29; clustered boxes 1.07 and 1.06 at 13, 0.91 and 0.86 at
+        // 16, 0.84 and 0.79 at 22; galaxies 1.05 and 0.95 at 9, 0.80 and 0.75 at 12, 0.71 and 0.67 at 23.
+        packed = packed && ng >= (int64_t)24 * 24 * ctx->num_sms;
         if (packed)
             for (auto& c : t->group_cache)
                 if (c.mode == mode && c.param == param && c.kmax == kmax) {

@@ -416,40 +416,85 @@ def test_handed_over_windows_do_not_depend_on_the_launch(gpu_ctx):
     assert np.median(e) <= 1e-6 and e.max() <= 1e-4
 
 
+def packed_leaves(gpu_ctx, T, **kw):
+    """A leaf walk of all targets in packs, and the same with one group per warp (window_pairs=False): the
+    tree holds enough leaves for packs (24 per resident warp, 148 SMs of 24), which shows in the bits."""
+    a = gpu_ctx.accel_grouped(T, None, **kw)
+    b = gpu_ctx.accel_grouped(T, None, window_pairs=False, **kw)
+    assert gpu_ctx.stats()["groups"] >= 24 * 24 * 148
+    assert not np.array_equal(a[0], b[0])
+    return a, b
+
+
+def packs_agree(p, q):
+    """To FP32 summation: 1e-6 is some ten roundings of 6e-8."""
+    e = relerr(*p[:3], *q[:3])
+    assert np.median(e) <= 3e-7 and np.quantile(e, 0.999) <= 1e-4
+    n = np.sqrt(sum((x - y) ** 2 for x, y in zip(p[:3], q[:3])).sum() / sum(y ** 2 for y in q[:3]).sum())
+    assert n <= 1e-6
+    if len(p) > 3:
+        assert np.median(np.abs(p[3] / q[3] - 1)) <= 1e-6
+
+
 @pytest.mark.parametrize("ics_kind", ["plummer", "clumps", "collocated"])
-@pytest.mark.parametrize("batch", [0, 5, 8, 16])
-def test_packs_match_single_groups(gpu_ctx, ics_kind, batch):
-    """Leaf groups and small windows over all particles share traversals in packs of up to eight groups
-    and 32 targets where there are enough of them (200,000 particles here): the same walk with one
-    group per warp (window_pairs=False) agrees to FP32 summation, accelerations and potential, in both
-    output orders, with clumps and jumps of the Morton curve between them, and with 40 particles in one
-    place, whose level-20 leaf is longer than a pack.  1e-6 is some ten roundings of 6e-8."""
-    rng = np.random.default_rng(batch + 1)
-    P = ics.plummer(n=200000, seed=batch + 3)
+def test_packs_match_single_groups(gpu_ctx, ics_kind):
+    """Leaf groups over all particles share traversals in packs of up to eight groups and 32 targets where
+    there are enough of them: the same walk with one group per warp agrees to FP32 summation,
+    accelerations and potential, in both output orders, with clumps and jumps of the Morton curve between
+    them, and with 40 particles in one place, whose level-20 leaf is longer than a pack."""
+    n = 500000
+    rng = np.random.default_rng(1)
+    P = ics.plummer(n=n, seed=3)
     if ics_kind == "clumps":
         for k in ("x", "y", "z"):
-            P[k] = 0.01 * P[k] + rng.integers(0, 4, 200000) * 2.0
+            P[k] = 0.01 * P[k] + rng.integers(0, 4, n) * 2.0
     if ics_kind == "collocated":
         for k in ("x", "y", "z"):
             P[k][1000:1040] = P[k][1000]
     T = gpu_ctx.build(P, key_mode=g.GT_KEY_MORTON)
-    kw = dict(theta=0.7, batch=batch, group_mode=g.GT_GROUP_BATCH if batch else g.GT_GROUP_LEAF, want_phi=True)
-    a = gpu_ctx.accel_grouped(T, None, **kw)
-    b = gpu_ctx.accel_grouped(T, None, window_pairs=False, **kw)
+    a, b = packed_leaves(gpu_ctx, T, theta=0.7, want_phi=True)
+    packs_agree(a, b)
     aold = gpu_ctx.form_aold(*b[:3], 0.0025)
-    kw["theta"] = 0.0
-    c = gpu_ctx.accel_grouped(T, None, aold=aold, **kw)
-    d = gpu_ctx.accel_grouped(T, None, aold=aold, window_pairs=False, **kw)
-    o = gpu_ctx.accel_grouped(T, None, aold=aold, out_order=g.GT_OUT_ORIGINAL, **kw)
+    c, d = packed_leaves(gpu_ctx, T, aold=aold, want_phi=True)
+    packs_agree(c, d)
+    o = gpu_ctx.accel_grouped(T, None, aold=aold, out_order=g.GT_OUT_ORIGINAL, want_phi=True)
     ob = T.download(nodes=False)["orderbuf"]
-    for p, q in ((a, b), (c, d)):
-        e = relerr(*p[:3], *q[:3])
-        assert np.median(e) <= 3e-7 and np.quantile(e, 0.999) <= 1e-4
-        n = np.sqrt(sum((x - y) ** 2 for x, y in zip(p[:3], q[:3])).sum() / sum(y ** 2 for y in q[:3]).sum())
-        assert n <= 1e-6
-        assert np.median(np.abs(p[3] / q[3] - 1)) <= 1e-6
     for k in range(4):
         assert np.array_equal(o[k][ob], c[k])
+
+
+def test_packs_in_chunks_plans_and_forests(gpu_ctx):
+    """What else a leaf walk of packs comes through: host arrays, whose walk runs in chunks of packs (ragged
+    n), and a captured plan give the bits of one launch on device arrays; in a forest, where a pack ends
+    with its system, and with the per-node criterion, packs agree with single groups."""
+    import os
+
+    import torch
+
+    n = 500001
+    P = ics.plummer(n=n, seed=6)
+    ctx = g.Context(0, torch_stream=True)
+    T = ctx.build(P)
+    aold = ctx.form_aold(*ctx.accel_grouped(T, None, theta=0.7, batch=32, group_mode=g.GT_GROUP_BATCH), 0.0025)
+    host, single = packed_leaves(ctx, T, aold=aold, want_phi=True)
+    packs_agree(host, single)
+    dev = torch.as_tensor(aold, device="cuda")
+    one = ctx.accel_grouped(T, None, aold=dev, want_phi=True)
+    outs = tuple(torch.empty(n, dtype=torch.float64, device="cuda") for _ in range(4))
+    plan = ctx.plan(T, dev, outs[:3], phi=outs[3])
+    for o in outs:
+        o.zero_()
+    plan.launch()
+    torch.cuda.synchronize()
+    for k in range(4):
+        assert np.array_equal(host[k], one[k].cpu().numpy()) and np.array_equal(host[k], outs[k].cpu().numpy())
+    plan.free()
+    model = np.load(os.path.join(os.path.dirname(g.__file__), "mac_node_model.npy"))
+    packs_agree(*packed_leaves(ctx, T, aold=aold, mac=g.GT_MAC_NODE, mac_model=model, mac_kappa=1.0))
+    off = np.array([0, 7, 7, 200003, n], np.int64)
+    x = np.searchsorted(off, np.arange(n), side="right") * 50.0
+    F = ctx.build(dict(P, x=P["x"] + x), offsets=off)
+    packs_agree(*packed_leaves(ctx, F, theta=0.7, want_phi=True))
 
 
 @pytest.mark.parametrize("nt", [1, 7, 8, 9, 257, 4095, 8191, 8192])
