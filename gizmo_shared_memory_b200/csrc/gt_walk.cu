@@ -2658,8 +2658,9 @@ void dispatch_pack(gt_context* ctx, const WalkArgs& a, int blocks, int warps, bo
 }
 
 // The packs of a tree's cached group list, made on the first walk that uses them (under the tree's
-// lock, complete on the device before they are published).
-void make_packs(gt_context* ctx, const gt_tree* t, gt_tree::GroupCache& c) {
+// lock, complete on the device before they are published).  Without memory for them there are none,
+// and the walk takes the groups one by one.
+void make_packs(gt_context* ctx, const gt_tree* t, gt_tree::GroupCache& c) try {
     cudaStream_t st = ctx->stream;
     const int64_t runs = (c.n_groups + kPackRun - 1) / kPackRun;
     uint32_t* cnt = (uint32_t*)scratch(ctx, kSlotNodeTmp1, (size_t)runs * 4);
@@ -2683,6 +2684,8 @@ void make_packs(gt_context* ctx, const gt_tree* t, gt_tree::GroupCache& c) {
     check_cuda(cudaStreamSynchronize(st), "sync");
     c.packs = (int2*)p;
     c.n_packs = n;
+} catch (const Fail& f) {
+    if (f.status != GT_ERR_NOMEM) throw;
 }
 
 struct OutputCopy {
@@ -2805,10 +2808,11 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         if (packed)
             for (auto& c : t->group_cache)
                 if (c.mode == mode && c.param == param && c.kmax == kmax) {
-                    if (!c.packs) make_packs(ctx, t, c);
+                    if (!c.packs && !rq.capture) make_packs(ctx, t, c);
                     packs = c.packs;
                     n_packs = c.n_packs;
                 }
+        packed = packs != nullptr;
     } else {
         uint32_t* tp = (uint32_t*)scratch(ctx, kSlotGroupKey, (size_t)nt * 4);
         uint32_t* flag = (uint32_t*)scratch(ctx, kSlotTargets, (size_t)nt * 4);

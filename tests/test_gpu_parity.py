@@ -497,6 +497,46 @@ def test_packs_in_chunks_plans_and_forests(gpu_ctx):
     packs_agree(*packed_leaves(ctx, F, theta=0.7, want_phi=True))
 
 
+def test_leaf_walk_without_memory_for_packs(gpu_ctx):
+    """Packs only make a leaf walk faster: where the device's memory pool cannot hold them (a pool of a few
+    MB, used up), the walk takes the groups one by one and gives window_pairs=False's bits; once the
+    memory is there they are made."""
+    from cuda.bindings import driver as cu
+
+    def ok(r):
+        assert r[0] == cu.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) > 1 else None
+
+    T = gpu_ctx.build(ics.plummer(n=500000, seed=6))
+    one = gpu_ctx.accel_grouped(T, None, theta=0.7, window_pairs=False)
+    prop = cu.CUmemPoolProps()
+    prop.allocType = cu.CUmemAllocationType.CU_MEM_ALLOCATION_TYPE_PINNED
+    prop.location.type = cu.CUmemLocationType.CU_MEM_LOCATION_TYPE_DEVICE
+    prop.location.id = 0
+    prop.maxSize = 1 << 21
+    dev = ok(cu.cuDeviceGet(0))
+    usual, small = ok(cu.cuDeviceGetMemPool(dev)), ok(cu.cuMemPoolCreate(prop))
+    taken = []
+    ok(cu.cuDeviceSetMemPool(dev, small))
+    try:
+        while len(taken) < 100000:
+            r = cu.cuMemAllocAsync(1 << 16, cu.CUstream(0))
+            if r[0] != cu.CUresult.CUDA_SUCCESS:
+                break
+            taken.append(r[1])
+        assert len(taken) < 100000
+        none = gpu_ctx.accel_grouped(T, None, theta=0.7)
+    finally:
+        ok(cu.cuDeviceSetMemPool(dev, usual))
+        for q in taken:
+            ok(cu.cuMemFreeAsync(q, cu.CUstream(0)))
+        ok(cu.cuStreamSynchronize(cu.CUstream(0)))
+        ok(cu.cuMemPoolDestroy(small))
+    for a, b in zip(none, one):
+        assert np.array_equal(a, b)
+    packed_leaves(gpu_ctx, T, theta=0.7)
+
+
 @pytest.mark.parametrize("nt", [1, 7, 8, 9, 257, 4095, 8191, 8192])
 @pytest.mark.parametrize("mode", [g.GT_GROUP_LEAF, g.GT_GROUP_NODE, g.GT_GROUP_BATCH])
 def test_small_target_lists_group_as_long_ones(gpu_ctx, plummer, plummer_trees, nt, mode):
