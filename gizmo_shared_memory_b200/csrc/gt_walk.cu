@@ -2182,12 +2182,12 @@ __global__ void target_flags_kernel(const uint32_t* __restrict__ targets, int64_
 // block, in one launch: flags, an ordered compaction of the group starts into shared memory, then
 // the chunking of groups longer than kmax.  count[0] = groups, count[1] = chunks, as
 // finish_groups_dev leaves them; the walk reads count[1].  What bounds it is the latency of the
-// scattered reads of rank and leaf_of, so every thread takes kSmallPer consecutive targets, whose
-// reads are all in flight at once, and each scan runs once: a walk of 4194 targets of 2^22 takes
-// 210 us instead of 217.
+// scattered reads of rank and leaf_of, so every thread takes PER consecutive targets, whose
+// reads are all in flight at once, and each scan runs once: with eight a walk of 4194 targets of 2^22
+// takes 210 us instead of 217.  A list of no more targets than threads takes one each: the groups of
+// 1, 10 and 1000 targets in 4.6, 4.7 and 6.0 us, with eight 5.2, 7.4 and 8.5.
 constexpr int kSmallTargets = 8192;
 constexpr int kSmallThreads = 1024;
-constexpr int kSmallPer = kSmallTargets / kSmallThreads;
 
 // Exclusive scan of one value per thread over the 1024-thread block; *total gets the sum.
 __device__ __forceinline__ int block_excl_scan_1024(int v, int* wsum, int* total) {
@@ -2217,6 +2217,7 @@ __device__ __forceinline__ int block_excl_scan_1024(int v, int* wsum, int* total
     return r;
 }
 
+template <int PER>
 __global__ void __launch_bounds__(kSmallThreads)
 small_groups_kernel(const uint32_t* __restrict__ targets, int nt, int mode, int param,
                     const uint32_t* __restrict__ rank, const int* __restrict__ leaf_of,
@@ -2228,28 +2229,28 @@ small_groups_kernel(const uint32_t* __restrict__ targets, int nt, int mode, int 
     __shared__ int wsum[32];
     __shared__ int last[32];  // the key of each warp's last target
     __shared__ int total;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k0 = (int)threadIdx.x * kSmallPer;
-    uint32_t p[kSmallPer], pos[kSmallPer];
-    int key[kSmallPer];  // what two neighbours of one group share (windows: their system)
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k0 = (int)threadIdx.x * PER;
+    uint32_t p[PER], pos[PER];
+    int key[PER];  // what two neighbours of one group share (windows: their system)
 #pragma unroll
-    for (int i = 0; i < kSmallPer; ++i) p[i] = k0 + i < nt ? checked_target(targets, k0 + i, n, bad) : 0u;
+    for (int i = 0; i < PER; ++i) p[i] = k0 + i < nt ? checked_target(targets, k0 + i, n, bad) : 0u;
 #pragma unroll
-    for (int i = 0; i < kSmallPer; ++i) pos[i] = k0 + i < nt ? rank[p[i]] : 0u;
+    for (int i = 0; i < PER; ++i) pos[i] = k0 + i < nt ? rank[p[i]] : 0u;
 #pragma unroll
-    for (int i = 0; i < kSmallPer; ++i) {
+    for (int i = 0; i < PER; ++i) {
         key[i] = 0;
         if (k0 + i >= nt) continue;
         if (mode == GT_GROUP_LEAF) key[i] = leaf_of[p[i]];
         else if (mode == GT_GROUP_NODE) key[i] = gid[pos[i]];
         else if (mode == GT_GROUP_BATCH && n_systems > 1) key[i] = system_of(in_off, n_systems, (int64_t)p[i]);
     }
-    if (lane == 31) last[w] = key[kSmallPer - 1];
+    if (lane == 31) last[w] = key[PER - 1];
     __syncthreads();
-    int prev = __shfl_up_sync(kFull, key[kSmallPer - 1], 1);
+    int prev = __shfl_up_sync(kFull, key[PER - 1], 1);
     if (lane == 0) prev = w > 0 ? last[w - 1] : 0;
     unsigned flags = 0;
 #pragma unroll
-    for (int i = 0; i < kSmallPer; ++i) {
+    for (int i = 0; i < PER; ++i) {
         const int k = k0 + i, q = i > 0 ? key[i - 1] : prev;
         if (k >= nt) continue;
         tpos[k] = pos[i];
@@ -2262,16 +2263,16 @@ small_groups_kernel(const uint32_t* __restrict__ targets, int nt, int mode, int 
     }
     int at = block_excl_scan_1024(__popc(flags), wsum, &total);
 #pragma unroll
-    for (int i = 0; i < kSmallPer; ++i)
+    for (int i = 0; i < PER; ++i)
         if ((flags >> i) & 1u) starts[at++] = k0 + i;
     const int ng = total;
     if (threadIdx.x == 0) starts[ng] = nt;
     __syncthreads();
-    // chunks of the groups, kSmallPer groups per thread
+    // chunks of the groups, PER groups per thread
     int c = 0;
-    for (int g = k0; g < min(k0 + kSmallPer, ng); ++g) c += (starts[g + 1] - starts[g] + kmax - 1) / kmax;
+    for (int g = k0; g < min(k0 + PER, ng); ++g) c += (starts[g + 1] - starts[g] + kmax - 1) / kmax;
     int o = block_excl_scan_1024(c, wsum, &total);
-    for (int g = k0; g < min(k0 + kSmallPer, ng); ++g)
+    for (int g = k0; g < min(k0 + PER, ng); ++g)
         for (int a = starts[g]; a < starts[g + 1]; a += kmax, ++o) groups[o] = make_int2(a, min(a + kmax, starts[g + 1]));
     if (threadIdx.x == 0) { count[0] = (uint32_t)ng; count[1] = (uint32_t)total; }
 }
@@ -2832,9 +2833,9 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         unsigned* bad = gc + 2;
         if (nt <= kSmallTargets) {
             groups = (int2*)scratch(ctx, kSlotGroupsB, (size_t)nt * sizeof(int2));
-            small_groups_kernel<<<1, kSmallThreads, 0, st>>>(rq.targets, (int)nt, mode, param, t->rank, t->leaf_of,
-                                                             gid, tp, t->sys_off_dev, t->in_off_dev, t->n_systems,
-                                                             kmax, groups, gc, t->n, bad);
+            auto small = nt <= kSmallThreads ? small_groups_kernel<1> : small_groups_kernel<kSmallTargets / kSmallThreads>;
+            small<<<1, kSmallThreads, 0, st>>>(rq.targets, (int)nt, mode, param, t->rank, t->leaf_of, gid, tp,
+                                               t->sys_off_dev, t->in_off_dev, t->n_systems, kmax, groups, gc, t->n, bad);
             check_launch(ctx, "small_groups_kernel");
             ng_dev = gc + 1;
         } else {
