@@ -835,9 +835,12 @@ walk_kernel(const WalkArgs A) {
         bool overflow = false;
         for (;;) {
             const bool done = top == 0 && base >= qtot;
-            if (npn > 0 && (done || npn > A.pn_cap - 32)) { flush_pn(npn); npn = 0; }
-            if (npp > 0 && (done || npp > A.pp_cap - 32)) { flush_pp(npp); npp = 0; }
-            if (done) break;
+            // (one branch around the two calls where most passes have neither: 1 % for small groups)
+            if (done || npn > A.pn_cap - 32 || npp > A.pp_cap - 32) {
+                if (npn > 0 && (done || npn > A.pn_cap - 32)) { flush_pn(npn); npn = 0; }
+                if (npp > 0 && (done || npp > A.pp_cap - 32)) { flush_pp(npp); npp = 0; }
+                if (done) break;
+            }
 
             if (qtot - base >= 32 || (base < qtot && (top == 0 || qn > kLeafQueue - 32))) {
                 // 32 particles of opened leaves, one per lane.  A particle farther from the group
