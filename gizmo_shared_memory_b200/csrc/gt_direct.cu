@@ -13,6 +13,7 @@
 #include <climits>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 #include "gt_internal.cuh"
 
@@ -144,6 +145,41 @@ __device__ __forceinline__ double rsqrt_d(double x) {
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+// A pair inside the larger softening, or within a part in 10^6 of it, at a normal r^2: the spline of
+// spline_d from 1/r by rsqrt_d and 1/h, which every target and source brings along, so that no
+// division or square root and no branch keeps the pairs of an iteration apart.  hinv = 1/h.
+__device__ __forceinline__ void inside_d(double r2, double h, double hinv, double& ri, double& u, double& f, double& p) {
+    ri = rsqrt_d(r2);
+    u = r2 * ri * hinv;
+    const double u2 = u * u, iu = h * ri, hinv3 = hinv * hinv * hinv;
+    const bool low = u < 0.5;
+    f = low ? 10.666666666666667 + u2 * (32.0 * u - 38.4)
+            : 21.333333333333332 - 48.0 * u + 38.4 * u2 - 10.666666666666667 * u2 * u - 0.06666666666666667 * (iu * iu * iu);
+    p = low ? -2.8 + u2 * (5.333333333333333 + u2 * (6.4 * u - 9.6))
+            : -3.2 + 0.06666666666666667 * iu + u2 * (10.666666666666667 + u * (-16.0 + u * (9.6 - 2.1333333333333333 * u)));
+    f = u < 1.0 ? hinv3 * f : ri * (ri * ri);
+    p = u < 1.0 ? hinv * p : -ri;
+}
+// dW/dr / r (kernel_dwdr_d) from u = r / h
+__device__ __forceinline__ double dwdr_r_d(double u, double ri, double hinv) {
+    const double v = 1.0 - u, fp = u < 0.5 ? -12.0 * u + 18.0 * u * u : -6.0 * v * v;
+    return u < 1.0 ? (8.0 / M_PI) * (hinv * hinv) * (hinv * hinv) * fp * ri : 0.0;
+}
+// The same in FP32; the root is corrected by its remainder.
+__device__ __forceinline__ void inside_f(float r2, float h, float hinv, float& f, float& p) {
+    const float ri = rsqrtf(r2);
+    float r = r2 * ri;
+    r = fmaf(fmaf(-r, r, r2), 0.5f * ri, r);
+    const float u = r * hinv, u2 = u * u, iu = h * ri, hinv3 = hinv * hinv * hinv;
+    const bool low = u < 0.5f;
+    f = low ? 10.666666666666667f + u2 * (32.0f * u - 38.4f)
+            : 21.333333333333332f - 48.0f * u + 38.4f * u2 - 10.666666666666667f * u2 * u - 0.06666666666666667f * (iu * iu * iu);
+    p = low ? -2.8f + u2 * (5.333333333333333f + u2 * (6.4f * u - 9.6f))
+            : -3.2f + 0.06666666666666667f * iu + u2 * (10.666666666666667f + u * (-16.0f + u * (9.6f - 2.1333333333333333f * u)));
+    f = u < 1.0f ? hinv3 * f : ri * ri * ri;
+    p = u < 1.0f ? hinv * p : -ri;
+}
+
 // Direct sum of kDirPer targets per thread over one chunk of the sources.
 //
 // What bounds it: the FP64 pipe (64 lanes a clock per SM).  A pair outside both softenings needs 18
@@ -167,6 +203,7 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
               const double* __restrict__ zeta = nullptr) {
     __shared__ DirSrc sh[kDirTile];
     __shared__ double shs[kDirTile];
+    __shared__ std::conditional_t<FP64, double, float> shi[kDirTile];  // 1 / softening
     __shared__ int shlim[kDirTile];
     __shared__ float shm[FP64 ? 1 : kDirTile];
     __shared__ double shzeta[GAS ? kDirTile : 1];
@@ -177,8 +214,13 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
         const float f = (float)s;
         return __float_as_int(f * f);
     };
+    auto inverse = [](double s) {
+        if constexpr (FP64) return 1.0 / fmax(s, 1e-300);
+        else return 1.0f / ((float)s > 0.0f ? (float)s : 1e-30f);
+    };
     const int64_t t0 = (int64_t)blockIdx.x * (kDirThreads * kDirPer) + threadIdx.x;
     int64_t self[kDirPer];
+    std::conditional_t<FP64, double, float> pinv[kDirPer];
     double px[kDirPer], py[kDirPer], pz[kDirPer], ps[kDirPer];
     int plim[kDirPer];
     GasTarget gas[GAS ? kDirPer : 1];
@@ -190,11 +232,14 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
         const int64_t t = t0 + k * kDirThreads;
         self[k] = t < nt ? (int64_t)targets[t] : n;
         const bool live = self[k] < n;
-        px[k] = live ? x[self[k]] : 0.0;
-        py[k] = live ? y[self[k]] : 0.0;
-        pz[k] = live ? z[self[k]] : 0.0;
+        // (a target that is none is far from everything, so that its pairs stay on the short path)
+        constexpr double kFar = FP64 ? 1e150 : 1e15;
+        px[k] = live ? x[self[k]] : kFar;
+        py[k] = live ? y[self[k]] : kFar;
+        pz[k] = live ? z[self[k]] : kFar;
         ps[k] = (live && soft) ? soft[self[k]] : 0.0;
         plim[k] = limit(ps[k]);
+        pinv[k] = inverse(ps[k]);
         ax[k] = ay[k] = az[k] = ap[k] = 0.0;
         if (GAS && live) {
             GasTarget& g = gas[GAS ? k : 0];
@@ -205,12 +250,18 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
         }
     }
     const int64_t s0 = (int64_t)blockIdx.y * chunk, s1 = min(n, s0 + chunk);
+    int n_live = 0;          // targets of this warp
+#pragma unroll
+    for (int k = 0; k < kDirPer; ++k) n_live += __popc(__ballot_sync(0xffffffffu, self[k] < n));
+    bool soft_tile = false;  // most of this warp's pairs of the last tile were inside a softening
     for (int64_t base = s0; base < s1; base += kDirTile) {
         for (int q = threadIdx.x; q < kDirTile; q += kDirThreads) {
             const int64_t j = base + q;
             if (j >= s1) {
                 shlim[q] = INT_MAX;  // past the chunk: every pair is left out of the short path
                 sh[q] = DirSrc{0.0, 0.0, 0.0, 0.0};
+                shs[q] = 0.0;
+                shi[q] = 1;
                 if (!FP64) shm[q] = 0.0f;
                 continue;
             }
@@ -221,6 +272,7 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
             sh[q] = DirSrc{x[j], y[j], z[j], fin ? mj : 0.0};
             const double s = soft ? soft[j] : 0.0;
             shs[q] = s;
+            shi[q] = inverse(s);
             shlim[q] = fin ? limit(s) : INT_MAX;
             if (!FP64) shm[q] = fin ? (float)mj : 0.0f;
             if (GAS) {
@@ -233,8 +285,10 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
         float fx[kDirPer], fy[kDirPer], fz[kDirPer], fp[kDirPer];
 #pragma unroll
         for (int k = 0; k < kDirPer; ++k) fx[k] = fy[k] = fz[k] = fp[k] = 0.0f;
+        int inside = 0;
         for (int q0 = 0; q0 < nq; q0 += kDirUnroll) {
-            unsigned slow = 0;
+            unsigned slow = soft_tile ? (1u << (kDirUnroll * kDirPer)) - 1u : 0u;
+            if (!soft_tile)
 #pragma unroll
             for (int i = 0; i < kDirUnroll; ++i) {
                 const int q = q0 + i;
@@ -268,13 +322,63 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
                     }
                 }
             }
+            if (!soft_tile) inside += __popc(slow);
             if (slow) {
-#pragma unroll 1
-                for (int i = 0; i < kDirUnroll; ++i)
+                unsigned odd = 0;  // pairs for the rule in full
+#pragma unroll 2
+                for (int i = 0; i < kDirUnroll; ++i) {
+                    const int q = q0 + i;
+                    if (((slow >> (i * kDirPer)) & ((1u << kDirPer) - 1u)) == 0u || q >= nq) continue;
+                    const DirSrc s = sh[q];
+                    const double ss = shs[q];
+                    const bool plain = shlim[q] != INT_MAX;
 #pragma unroll
                     for (int k = 0; k < kDirPer; ++k) {
+                        const unsigned bit = 1u << (i * kDirPer + k);
+                        const bool take = (slow & bit) != 0u && base + q != self[k];
+                        const double ox = s.x - px[k], oy = s.y - py[k], oz = s.z - pz[k];
+                        if constexpr (FP64) {
+                            const double r2 = ox * ox + oy * oy + oz * oz;
+                            const int hi = __double2hiint(r2);
+                            const bool ok = plain && hi >= 0x00100000 && hi < 0x7ff00000;
+                            if (take && !ok) odd |= bit;
+                            if (soft_tile && hi <= max(plim[k], shlim[q])) ++inside;
+                            double ri, u, f, p;
+                            inside_d(r2, fmax(fmax(ps[k], ss), 1e-300), fmin(pinv[k], shi[q]), ri, u, f, p);
+                            double mf = s.m * f;
+                            if (GAS && gas[GAS ? k : 0].gas && shgas[q] && gas[GAS ? k : 0].tm > 0.0) {
+                                const GasTarget& g = gas[GAS ? k : 0];
+                                if (g.tzeta != 0.0) mf -= g.tzm * dwdr_r_d(u, ri, fmin(pinv[k], shi[q]));
+                                if (shzeta[q] != 0.0) mf -= shzeta[q] / g.tm * dwdr_r_d(r2 * ri * shi[q], ri, shi[q]);
+                            }
+                            if (take && ok) {
+                                ax[k] += ox * mf; ay[k] += oy * mf; az[k] += oz * mf;
+                                ap[k] += s.m * p;
+                            }
+                        } else {
+                            const float dx = (float)ox, dy = (float)oy, dz = (float)oz;
+                            const float r2 = dx * dx + dy * dy + dz * dz;
+                            const int hi = __float_as_int(r2);
+                            const bool ok = plain && hi >= 0x00800000 && hi < 0x7f800000;
+                            if (take && !ok) odd |= bit;
+                            if (soft_tile && hi <= max(plim[k], shlim[q])) ++inside;
+                            const float h = fmaxf((float)ps[k], (float)ss);
+                            float f, p;
+                            inside_f(r2, h > 0.0f ? h : 1e-30f, fminf(pinv[k], shi[q]), f, p);
+                            const float mf = shm[q] * f;
+                            if (take && ok) {
+                                fx[k] += dx * mf; fy[k] += dy * mf; fz[k] += dz * mf;
+                                fp[k] += shm[q] * p;
+                            }
+                        }
+                    }
+                }
+#pragma unroll 1
+                for (int i = 0; odd != 0u && i < kDirUnroll; ++i)
+#pragma unroll
+                    for (int k = 0; k < kDirPer; ++k) {
+                        if (!((odd >> (i * kDirPer + k)) & 1u)) continue;
                         const int q = q0 + i;
-                        if (!((slow >> (i * kDirPer + k)) & 1u) || q >= nq || base + q == self[k]) continue;
                         const DirSrc s = sh[q];
                         const double ox = s.x - px[k], oy = s.y - py[k], oz = s.z - pz[k];
                         const double mj = __ldg(m + base + q);  // as it was given
@@ -294,6 +398,7 @@ direct_kernel(const double* __restrict__ x, const double* __restrict__ y, const 
                     }
             }
         }
+        soft_tile = 2 * __reduce_add_sync(0xffffffffu, inside) > n_live * nq;
         if (!FP64) {
 #pragma unroll
             for (int k = 0; k < kDirPer; ++k) {

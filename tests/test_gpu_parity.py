@@ -602,6 +602,60 @@ def test_direct_edges_of_tiles(gpu_ctx, oracle, n, soft):
         assert (np.abs(phi - op) <= tol * pscale)[seen].all()
 
 
+@pytest.mark.parametrize("precision,eps", [(g.GT_DIRECT_FP64, 2.0 ** -53), (g.GT_DIRECT_FP32, 2.0 ** -24)])
+def test_direct_reciprocal_root_in_ulps(gpu_ctx, precision, eps):
+    """One source with mass 1 at the origin and massless targets on an axis: phi = -1/r and a = 1/r^2, over
+    the exponents at which r^2 is an ordinary number.  r^2 is rounded once, which 1/r halves; CUDA's FP32
+    reciprocal root is within 2 ulp, which is 4 eps, and the FP64 one is held to the same: 5 eps for phi,
+    and for a, three of them and three products, 18.  FP32 offsets are exact here (20 bits)."""
+    rng = np.random.default_rng(2)
+    top = 500 if precision == g.GT_DIRECT_FP64 else 60
+    bits = 52 if precision == g.GT_DIRECT_FP64 else 20
+    r = np.ldexp(1.0 + np.floor(rng.uniform(size=4000) * 2.0 ** bits) / 2.0 ** bits, rng.integers(-top, top, 4000))
+    n = len(r) + 1
+    P = dict(x=np.concatenate([[0.0], r]), y=np.zeros(n), z=np.zeros(n), m=np.zeros(n), soft=np.zeros(n))
+    P["m"][0] = 1.0
+    if precision == g.GT_DIRECT_FP32:  # 1/r^2 within the FP32 range
+        P["x"] = np.where(np.abs(P["x"]) > 0, np.clip(P["x"], 2.0 ** -40, 2.0 ** 40), 0.0)
+    x = P["x"][1:]
+    ax, ay, az, phi = gpu_ctx.direct(P, np.arange(1, n, dtype=np.uint32), precision=precision)
+    assert np.abs(phi * x + 1.0).max() <= 5 * eps
+    ok = (x < 2.0 ** 250) & (x > 2.0 ** -250)  # 1/r^3 in range
+    assert np.abs(ax[ok] * x[ok] * x[ok] + 1.0).max() <= 18 * eps
+    assert not ay[ok].any() and not az[ok].any()
+
+
+@pytest.mark.parametrize("n,nt", [(300, 300), (4096, 64), (3001, 1000)])
+@pytest.mark.parametrize("low,high", [(1.0, 3.0), (20.0, 80.0), (0.0, 1.0)])
+def test_direct_inside_the_softening(gpu_ctx, oracle, n, nt, low, high):
+    """Pairs on both sides of u = 1/2 and u = 1, each target and source with its own softening, and with
+    80 every pair inside, where whole tiles leave the short path; with a coincident pair, a softening of
+    zero and a particle 1e-160 from another.  The spline's terms cancel to about a tenth of their sum, so
+    FP64 to 1e-13 of the sum of the pairs' absolute forces (the tree's own tests bound 1e-12 of it) and
+    FP32 to 2e-6."""
+    P = ics.plummer(n=n, seed=n)
+    rng = np.random.default_rng(n)
+    P["soft"] = rng.uniform(low, high, n)
+    P["soft"][7] = 0.0
+    for k in ("x", "y", "z"):
+        P[k][4], P[k][6] = P[k][3], 0.0
+        P[k][7] = 1e-160 if k == "x" else 0.0
+    tg = np.sort(rng.choice(n, nt, replace=False)).astype(np.uint32)
+    tg[:5] = [3, 4, 5, 6, 7]
+    o = np.stack(oracle.direct(P, tg))
+    X = np.stack([P[k] for k in ("x", "y", "z")], 1)
+    scale = np.zeros(nt)
+    for i, t in enumerate(tg):
+        r = np.sqrt(((X - X[t]) ** 2).sum(1))
+        h = np.maximum(np.maximum(P["soft"], P["soft"][t]), 1e-300)
+        scale[i] = (P["m"] * np.where(r > 0, np.minimum(11.0 * r / h / h / h, 1.0 / np.maximum(r, 1e-150) ** 2), 0.0)).sum()
+    for prec, tol in ((g.GT_DIRECT_FP64, 1e-13), (g.GT_DIRECT_FP32, 2e-6)):
+        a = np.stack(gpu_ctx.direct(P, tg, precision=prec))
+        assert (np.sqrt(((a[:3] - o[:3]) ** 2).sum(0)) <= tol * scale).all()
+        seen = ~np.isin(tg, [6, 7]) | (prec == g.GT_DIRECT_FP64)  # FP32 narrows their offset to 0
+        assert (np.abs(a[3] / o[3] - 1.0) <= tol)[seen].all()
+
+
 @pytest.mark.parametrize("mass,precision", [(np.inf, g.GT_DIRECT_FP64), (np.nan, g.GT_DIRECT_FP64),
                                             (np.inf, g.GT_DIRECT_FP32), (np.nan, g.GT_DIRECT_FP32),
                                             (1e39, g.GT_DIRECT_FP32)])
