@@ -321,3 +321,59 @@ def test_counted_lists_of_moved_particles(gpu_ctx):
     assert min(len(w) for w in want) > 64  # past what the counting pass keeps
     assert (plain > np.diff(st)).any()     # the two prunes differ here
     assert np.array_equal(np.diff(st), [len(w) for w in want]) and np.array_equal(f, np.concatenate(want))
+
+
+@pytest.mark.parametrize("power", [-70, -40, 40, 70])
+def test_search_and_density_scale_with_the_lengths(gpu_ctx, power):
+    """Lengths times a power of two change no decision: the prune's squares leave the FP32 range at 2^-70
+    (below 1e-45) and at 2^70, and may then admit nodes that hold nothing but must not drop any.  The lists,
+    the iterations and the neighbour counts stay; h and the density, whose iteration takes roots and
+    exponentials, scale to this file's 1e-10."""
+    f = 2.0 ** power
+    rng = np.random.default_rng(11)
+    x = np.concatenate([0.05 * rng.normal(size=(3000, 3)), rng.uniform(-1, 1, (3000, 3))])
+    m = rng.uniform(0.5, 1.5, 6000)
+    rad = 10 ** rng.uniform(-2.5, -0.5, 6000)
+    tg = np.arange(6000, dtype=np.uint32)
+    r = []
+    for s in (1.0, f):
+        P = {k: x[:, i] * s for i, k in enumerate("xyz")}
+        P["m"] = m
+        T = gpu_ctx.build(P, key_mode=g.GT_KEY_MORTON)
+        hs = rad * s
+        gpu_ctx.tree_hmax(T, hs, 6000)
+        r.append([gpu_ctx.ngb_search(T, *(P[k] for k in "xyz"), hs),
+                  gpu_ctx.ngb_search(T, *(P[k] for k in "xyz"), 0.5 * hs, mode=g.GT_NGB_PAIRS, h=hs, n_gas=6000),
+                  gpu_ctx.density(T, tg, h_start=0.1 * s * np.ones(6000))])
+    for a, b in zip(r[0][:2], r[1][:2]):
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    a, b = r[0][2], r[1][2]
+    assert np.array_equal(a["iters"], b["iters"]) and np.array_equal(a["nngb"], b["nngb"])
+    assert np.abs(a["h"] * f / b["h"] - 1).max() <= 1e-10 and np.abs(b["rho"] * f ** 3 / a["rho"] - 1).max() <= 1e-10
+
+
+@pytest.mark.parametrize("scale", [1e-9, 1.0, 1e9])
+def test_density_weights_in_ulps(gpu_ctx, scale):
+    """One particle outweighs all others by 1e30, so a target's density is that one's kernel weight at the h
+    the solve ends with: 8 / (pi h^3) times the spline of q = r / h, against extended precision.  r by the
+    root of the sum of squares, q by the reciprocal of h and the norm are each a few roundings (2^-53) off,
+    which the spline passes on q f'/f times: 16 + 4 q f'/f roundings."""
+    rng = np.random.default_rng(5)
+    x = scale * rng.uniform(-1, 1, (2000, 3))
+    heavy = int(np.argmin((x ** 2).sum(1)))
+    P = {k: x[:, i].copy() for i, k in enumerate("xyz")}
+    P["m"] = np.full(2000, 1e-30)
+    P["m"][heavy] = 1.0
+    T = gpu_ctx.build(P, key_mode=g.GT_KEY_MORTON)
+    near = np.argsort(((x - x[heavy]) ** 2).sum(1))[1:40].astype(np.uint32)
+    d = gpu_ctx.density(T, near, h_start=np.full(39, 0.5 * scale))
+    X, h = x.astype(np.longdouble), d["h"].astype(np.longdouble)
+    q = np.sqrt(((X[near] - X[heavy]) ** 2).sum(1)) / h
+    q, rho, h = q[q < 0.98], d["rho"][q < 0.98], h[q < 0.98]
+    assert len(q) >= 15 and (q < 0.5).any() and (q > 0.5).any()
+    low = q < 0.5
+    f = np.where(low, 1 - 6 * q * q + 6 * q ** 3, 2 * (1 - q) ** 3)
+    slope = np.where(low, 12 * q - 18 * q * q, 6 * (1 - q) ** 2)
+    pi = np.longdouble("3.14159265358979323846264338327950288")
+    e = np.abs(rho / (8 / (pi * h ** 3) * f) - 1)
+    assert (e <= (16 + 4 * q * slope / f) * 2.0 ** -53).all()
