@@ -861,6 +861,26 @@ def test_large_host_outputs_cross_the_ring_unchanged(gpu_ctx, n):
     assert np.array_equal(gpu_ctx.form_aold(*v, 0.005, G=2.0), dev.cpu().numpy())
 
 
+@pytest.mark.parametrize("n", [2 ** 20, 5 * 2 ** 20 + 3])
+def test_large_host_outputs_into_used_and_fresh_pages(gpu_ctx, n):
+    """Large outputs go through the ring into pages that were never touched, and by the driver's copy into
+    arrays in use: the same bits in an array just written, in a fresh mapping, and in one whose first half
+    was written."""
+    import ctypes
+    import mmap
+
+    v = np.random.default_rng(n).normal(size=(3, n))
+    want = gpu_ctx.form_aold(*v, 0.005)
+    fresh, half = (np.frombuffer(mmap.mmap(-1, 8 * n), np.float64) for _ in range(2))
+    half[:n // 2] = 1.0
+    for out in (np.ones(n), fresh, half):
+        for _ in range(2):  # the second time every page was written
+            st = g.load_library().gt_form_aold(gpu_ctx.h, n, *(x.ctypes.data for x in v), 0.005, 1.0,
+                                               g._gt.GT_MEM_HOST, ctypes.c_void_p(out.ctypes.data))
+            assert st == 0 and np.array_equal(out, want)
+            out[::4096] = 0.0
+
+
 def test_host_aold_uploaded_in_chunks_is_identical(gpu_ctx):
     """A walk given a host aold and host outputs uploads aold piece by piece on the copy stream,
     each chunk waiting only for its own targets' piece, and downloads each chunk's results while the
