@@ -141,12 +141,12 @@ __device__ __forceinline__ bool is_neighbour(const SearchGeom& g, int s, double 
 // leaves in one flat loop, a particle an iteration, and the traversal goes on.  The lanes are brought
 // together after each loop: left to themselves they go on from their own last iteration, and two in
 // 32 were active by the time the neighbours' sums were formed.
-// The prune is the reference's box and circumsphere test in FP32, the centre in two floats, widened by
-// the rounding of the distances and the squares, so it never drops a node that the FP64 test keeps; the
-// particle test decides in FP64, so the lists are the same, in the same order, as long as the nodes'
-// boxes cover their particles.  (With the centre in one float the prune had to be wider by 16 roundings
-// of it, which in a cluster of 1e-4 of the box, whose lengths are some 50 of them, visited more nodes
-// than the FP64 test: 4.6 -> 5.5 ms for the reverse search of 100,000 centres, 4.3 this way.)
+// The prune is the reference's box and circumsphere test in FP32, widened by the rounding of the centre,
+// the distances and the squares, so it never drops a node that the FP64 test keeps; the particle test
+// decides in FP64, so the lists are the same, in the same order, as long as the nodes' boxes cover their
+// particles.  The widening is no more than it must be: at eight times it a cluster of 1e-4 of its box,
+// whose lengths are a few hundred roundings of its position, had more nodes visited than by the FP64
+// test (reverse search of 100,000 centres: 4.6 ms by the FP64 test, 5.3 at eight times, 3.8 now).
 constexpr int kLeafBuf = 32;
 template <bool REVERSE, typename F>
 __device__ __forceinline__ void search(const SearchGeom& g, int r0, int r1, double px, double py, double pz,
@@ -154,11 +154,11 @@ __device__ __forceinline__ void search(const SearchGeom& g, int r0, int r1, doub
                                        F&& emit) {
     const double r2max = radius * radius;
     const float fx = (float)px, fy = (float)py, fz = (float)pz;
-    const float lx = (float)(px - (double)fx), ly = (float)(py - (double)fy), lz = (float)(pz - (double)fz);
     const float fbox = (float)g.box, fhalf = 0.5f * fbox;
-    // the rounding of the box side and of a difference that the minimum image makes small, on three axes
-    // (1.74 times 2 * 2^-24), and below, where the squares leave the FP32 range, FLT_MIN above all theirs
-    const float slack = 2.0f * FLT_EPSILON * fbox;
+    // The rounding of the centre, and twice that of the box side (of itself and of a difference that the
+    // minimum image makes small), 2^-24 of each per axis, on three axes 1.74 times that.  Where the squares
+    // leave the FP32 range FLT_MIN is above all their roundings.
+    const float slack = FLT_EPSILON * (fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) + 2.0f * fbox);
     const float reach = REVERSE ? slack : __fadd_ru(__double2float_ru(radius), slack);
     const float felapsed = g.elapsed > 0 ? __double2float_ru(g.elapsed) : 0.0f;
     const bool moving = g.elapsed > 0 && g.vmax;
@@ -186,7 +186,7 @@ __device__ __forceinline__ void search(const SearchGeom& g, int r0, int r1, doub
             if (g.xpad) dist += __ldg(g.xpad + node);
             if (moving) dist = fmaf(__ldg(g.vmax + node), felapsed, dist);
             dist *= 1.000002f;
-            const float dx = image((a.x - fx) - lx), dy = image((a.y - fy) - ly), dz = image((a.z - fz) - lz);
+            const float dx = image(a.x - fx), dy = image(a.y - fy), dz = image(a.z - fz);
             const float ball = fmaf(0.73205090f, a.w, dist) * 1.000002f;
             keep = keep && !(fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz))) > dist) &&
                    !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > fmaf(ball, ball, FLT_MIN));
