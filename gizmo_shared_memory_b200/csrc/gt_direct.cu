@@ -1,9 +1,9 @@
 // O(N_targets * N) direct summation: the replacement for shmem::accel_brute (shmem/tree.cc:946-971)
 // and for the reference's only CUDA kernel, accel_bruteforce_kernel (shmem/grav_cuda.cu:66-141).
 //
-// Each block holds 256 targets in registers, two per thread, and streams one contiguous chunk of the sources
-// through shared memory in tiles of 256; the grid's second dimension splits the sources so that a
-// few thousand targets (the error sample) still fill all 148 SMs.  Per-chunk partial sums go to a
+// Each block holds 256 targets in registers, two per thread, and streams one contiguous chunk of the
+// sources through shared memory in tiles of 256; the grid's second dimension splits the sources so that
+// a few thousand targets (the error sample) still fill all 148 SMs.  Per-chunk partial sums go to a
 // scratch array and a second kernel adds the chunks in a fixed order, so results are deterministic.
 //   FP64: every operation in double, the pair rule of tree.cc:39-53 with zeta = 0 (kernel of the
 //         larger softening, self and r == 0 skipped) -- the error oracle of the walk.
@@ -148,15 +148,18 @@ __device__ __forceinline__ double rsqrt_d(double x) {
 // A pair inside the larger softening, or within a part in 10^6 of it, at a normal r^2: the spline of
 // spline_d from 1/r by rsqrt_d and 1/h, which every target and source brings along, so that no
 // division or square root and no branch keeps the pairs of an iteration apart.  hinv = 1/h.
-__device__ __forceinline__ void inside_d(double r2, double h, double hinv, double& ri, double& u, double& f, double& p) {
+__device__ __forceinline__ void inside_d(double r2, double h, double hinv, double& ri, double& u, double& f,
+                                         double& p) {
     ri = rsqrt_d(r2);
     u = r2 * ri * hinv;
     const double u2 = u * u, iu = h * ri, hinv3 = hinv * hinv * hinv;
     const bool low = u < 0.5;
     f = low ? 10.666666666666667 + u2 * (32.0 * u - 38.4)
-            : 21.333333333333332 - 48.0 * u + 38.4 * u2 - 10.666666666666667 * u2 * u - 0.06666666666666667 * (iu * iu * iu);
+            : 21.333333333333332 - 48.0 * u + 38.4 * u2 - 10.666666666666667 * u2 * u -
+                  0.06666666666666667 * (iu * iu * iu);
     p = low ? -2.8 + u2 * (5.333333333333333 + u2 * (6.4 * u - 9.6))
-            : -3.2 + 0.06666666666666667 * iu + u2 * (10.666666666666667 + u * (-16.0 + u * (9.6 - 2.1333333333333333 * u)));
+            : -3.2 + 0.06666666666666667 * iu +
+                  u2 * (10.666666666666667 + u * (-16.0 + u * (9.6 - 2.1333333333333333 * u)));
     f = u < 1.0 ? hinv3 * f : ri * (ri * ri);
     p = u < 1.0 ? hinv * p : -ri;
 }
@@ -173,9 +176,11 @@ __device__ __forceinline__ void inside_f(float r2, float h, float hinv, float& f
     const float u = r * hinv, u2 = u * u, iu = h * ri, hinv3 = hinv * hinv * hinv;
     const bool low = u < 0.5f;
     f = low ? 10.666666666666667f + u2 * (32.0f * u - 38.4f)
-            : 21.333333333333332f - 48.0f * u + 38.4f * u2 - 10.666666666666667f * u2 * u - 0.06666666666666667f * (iu * iu * iu);
+            : 21.333333333333332f - 48.0f * u + 38.4f * u2 - 10.666666666666667f * u2 * u -
+                  0.06666666666666667f * (iu * iu * iu);
     p = low ? -2.8f + u2 * (5.333333333333333f + u2 * (6.4f * u - 9.6f))
-            : -3.2f + 0.06666666666666667f * iu + u2 * (10.666666666666667f + u * (-16.0f + u * (9.6f - 2.1333333333333333f * u)));
+            : -3.2f + 0.06666666666666667f * iu +
+                  u2 * (10.666666666666667f + u * (-16.0f + u * (9.6f - 2.1333333333333333f * u)));
     f = u < 1.0f ? hinv3 * f : ri * ri * ri;
     p = u < 1.0f ? hinv * p : -ri;
 }
@@ -188,10 +193,15 @@ __device__ __forceinline__ void inside_f(float r2, float h, float hinv, float& f
 // outside is an integer comparison of the high words of r^2 and of the larger squared softening.  The
 // high word rounds down, so pairs within one part in 10^6 of the softening, the pair of a particle
 // with itself, r = 0 and every subnormal, infinite or NaN r^2 are left out of it (1/r taken
-// as 0) and taken by pair_d, which treats each case as the rule says, after the iteration's pairs: one
-// branch per kDirUnroll sources and kDirPer targets, rarely taken, instead of one per pair, which
-// kept every pair's chain of dependent instructions to itself.  4096 targets against 262,144 sources:
-// 5.47 -> 1.64 ms, 0.69 of the FP64 peak (34 TF/s) counting an instruction as two operations.
+// as 0) and evaluated after the iteration's pairs, by inside_d at an ordinary r^2 and else by pair_d,
+// which treats each case as the rule says: one branch per kDirUnroll sources and kDirPer targets, rarely
+// taken, instead of one per pair, which kept every pair's chain of dependent instructions to itself.
+// 4096 targets against 262,144 sources: 5.47 -> 1.64 ms, 0.69 of the FP64 peak (34 TF/s) counting an
+// instruction as two operations.
+// Where a softening holds most of a warp's pairs of a tile, the short path is work for nothing, and the
+// next tile is evaluated by inside_d alone.  20,000 particles against each other with all pairs inside:
+// 2.03 ms with one branch per pair, 4.22 with the short path and pair_d, 2.51 with inside_d, 2.09 this way
+// (FP32 1.42, 2.63, 1.91, 1.42).
 //   FP32: the offset is differenced in double and narrowed, the interaction is FP32 with the
 //   approximate reciprocal square root, and each tile's FP32 sums are added into double totals.
 template <bool FP64, bool GAS = false>

@@ -1403,8 +1403,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
                         if (have) {
                             Handover* q = record(slot);
                             if (lane == 0) { q->pair = pr; q->n = top; q->shares = shares; q->done = 0u; }
-                            q->sum[0][lane] = HandSum{make_float2(sx0, cx0), make_float2(sy0, cy0), make_float2(sz0, cz0), pot0};
-                            q->sum[1][lane] = HandSum{make_float2(sx1, cx1), make_float2(sy1, cy1), make_float2(sz1, cz1), pot1};
+                            q->sum[0][lane] = HandSum{make_float2(sx0, cx0), make_float2(sy0, cy0),
+                                                      make_float2(sz0, cz0), pot0};
+                            q->sum[1][lane] = HandSum{make_float2(sx1, cx1), make_float2(sy1, cy1),
+                                                      make_float2(sz1, cz1), pot1};
                             break;
                         }
                         left = INT_MAX;
@@ -1884,18 +1886,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pack_kernel(const Walk
         };
 
         // ---- traversal: walk_pair_kernel's loop -------------------------------------------------
-        int top = 1;
-        if (!A.group_root) {
-            if (lane == 0) stk[0] = (int)full;
-        } else {
-            // in a forest, one entry per root that the pack's groups start from
-            const int r = lane < G ? A.group_root[pk.x + lane] : -1 - lane;
-            const unsigned same = __match_any_sync(kFull, r);
-            const bool lead = lane < G && (same & lt_mask) == 0u;
-            const unsigned lm = __ballot_sync(kFull, lead);
-            if (lead) stk[__popc(lm & lt_mask)] = (int)(((unsigned)r << kPackGroups) | same);
-            top = __popc(lm);
-        }
+        int top = 1;  // the root: of the tree, or in a forest of the system, in which the whole pack lies
+        if (lane == 0) stk[0] = (int)((A.group_root ? (unsigned)A.group_root[pk.x] << kPackGroups : 0u) | full);
         __syncwarp();
         int na = 0, ns = 0, nn = 0;
         int base = 0, qtot = 0;  // the opened leaves' particles still to place: [base, qtot)
@@ -1968,7 +1960,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pack_kernel(const Walk
             __syncwarp();
             const NodeV nd = load_node(A.nodes + node);
             const bool leaf = nd.first < 0;
-            const double len = (double)nd.len, lim = 0.6 * len;
+            const double len = (double)nd.len;
             const double ml2 = MAC == 2 ? nd.mass * (double)__ldg(A.mac_l2 + node) : nd.mass * len * len;
             unsigned om = 0;  // the groups that open this node
 #pragma unroll 1
