@@ -2895,8 +2895,8 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
                : macn ? occupancy_blocks<4, true, false, false, 2>(warps, pn_cap)
                       : occupancy_blocks<4, true, false, false, 0>(warps, pn_cap);
     // Long windows hand over (Handover) where a walk of the whole tree lasts about as long as its longest
-    // pair: fewer than two pairs per resident warp.  Trees of fewer than 40 pairs keep theirs: the second
-    // launch's 12 us are a tenth of their walk.  The fewer the pairs, the more warps wait for work, and
+    // pair: fewer than two pairs per resident warp.  Trees of fewer than 40 pairs, in a forest on average,
+    // keep theirs: the second launch's 12 us are a tenth of their walk.  The fewer the pairs, the more warps wait for work, and
     // the sooner and the finer a pair is split; with more pairs than resident warps a share of fewer than
     // 64 entries is not worth its ramp-up.  The rule reads the tree's size and not the call's targets, so
     // a slice of the targets is walked as it is in the whole.  Device time of whole calls without and
@@ -2910,7 +2910,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     const int64_t units = ((all || t->n_systems > 1 ? ng : (nt + param - 1) / std::max(1, param)) + 1) / 2;
     const int64_t resident = (int64_t)24 * ctx->num_sms;
     int budget = 0, hand_least = 64, share_least = 4, shares = 16;
-    if (paired && tree_units >= 40 && tree_units < 2 * resident) {
+    if (paired && tree_units >= (int64_t)40 * t->n_systems && tree_units < 2 * resident) {
         budget = tree_units <= resident / 3 ? 32 : tree_units <= resident * 3 / 5 ? 96 : 192;
         if (tree_units > resident) { hand_least = 256; share_least = 64; shares = 8; }
     }
