@@ -196,7 +196,7 @@ __device__ __forceinline__ void inside_f(float r2, float h, float hinv, float& f
 // as 0) and evaluated after the iteration's pairs, by inside_d at an ordinary r^2 and else by pair_d,
 // which treats each case as the rule says: one branch per kDirUnroll sources and kDirPer targets, rarely
 // taken, instead of one per pair, which kept every pair's chain of dependent instructions to itself.
-// 4096 targets against 262,144 sources: 5.47 -> 1.64 ms, 0.69 of the FP64 peak (34 TF/s) counting an
+// 4096 targets against 262,144 sources: 5.47 -> 1.48 ms, 0.77 of the FP64 peak (34 TF/s) counting an
 // instruction as two operations.
 // Where a softening holds most of a warp's pairs of a tile, the short path is work for nothing, and the
 // next tile is evaluated by inside_d alone.  20,000 particles against each other with all pairs inside:

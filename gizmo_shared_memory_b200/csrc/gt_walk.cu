@@ -2726,8 +2726,9 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     const uint32_t* ng_dev = nullptr;  // explicit targets: the group count stays on the device
     // The leaves of all live targets (the engine's grouping): packs of them share one traversal.  A list
     // of explicit targets may hold groups far from one another, which share nothing and keep a warp
-    // each; so do small windows, whose boxes span the jumps of the curve (a clustered box is suspected
-    // of 4.05 -> 7.06 ms when packed, and was not measured apart).
+    // each.  So do small windows: packed, those of 16, two to a pack, took 0.95 to 1.18 times as long
+    // (Plummer spheres, galaxies and clustered boxes of 400,000 to 4 million, at alpha 0.0025), and of 8
+    // and 5 from 1.12 and 0.85 times with few windows to 0.73 and 0.57 with many.
     bool packed = all && rq.pair_windows && !xt && tpl == 1 && rq.leaf_accept && rq.mac != GT_MAC_LEARNED &&
                   !rq.count && t->n_nodes < (1 << 24) && rq.list_capacity == 0 &&
                   mode == GT_GROUP_LEAF;

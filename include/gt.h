@@ -131,8 +131,11 @@ typedef struct {
      * window gets its own walk's decisions and interactions (sums equal to FP32 rounding, not bit
      * for bit: the list order can differ).  Forests and counting walks included; not for
      * GT_MAC_LEARNED, the tidal tensor, the jerk or the gas rules.  Likewise by default: a long
-     * window of a small tree hands part of its traversal to other warps, and in walks of all
-     * targets several leaf groups share one traversal, each again with its own decisions.  1: none of these, one warp per group. */
+     * window of a tree with fewer than two pairs of windows per resident warp (450,000 particles in
+     * windows of 32) hands part of its traversal to other warps, and in walks of all targets several
+     * leaf groups share one traversal, each again with its own decisions.  The handing over keeps a
+     * record per pair of windows in device memory, at most 213 MB per context and 190 MB per plan, and
+     * does without them where there is no room.  1: none of these, one warp per group. */
     int no_window_pairs;
 } gt_walk_options;
 
