@@ -1169,10 +1169,15 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
     unsigned long long c_nodes = 0, c_multi = 0, c_pairs = 0, c_zero = 0, c_flush = 0, c_steps = 0;
     int c_maxtop = 0;
 
-    for (;;) {
-        int unit = 0;
-        if (lane == 0) unit = (int)atomicAdd(SHARE ? A.hand_ctr + 1 : A.next_group, 1u);
-        unit = __shfl_sync(kFull, unit, 0);
+    // (a share's warp has its first unit by its number: where nobody handed over, the launch ends without
+    // an atomic per warp)
+    for (int turn = 0;; ++turn) {
+        int unit = gw;
+        if (!SHARE || turn > 0) {
+            if (lane == 0) unit = (int)atomicAdd(SHARE ? A.hand_ctr + 1 : A.next_group, 1u);
+            unit = __shfl_sync(kFull, unit, 0);
+            if (SHARE) unit += gridDim.x * (blockDim.x >> 5);
+        }
         if (unit >= n_units) break;
         if (SHARE && unit % A.shares >= record(unit / A.shares)->shares) continue;
         const int pr = SHARE ? record(unit / A.shares)->pair : unit;
@@ -2903,9 +2908,10 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     // a slice of the targets is walked as it is in the whole.  Device time of whole calls without and
     // with it, ms, at alpha 0.0025 and 0.000025: Plummer spheres of 20,000 particles 1.44 -> 0.32 and
     // 1.73 -> 0.40, of 65,536 0.84 -> 0.34 and 3.92 -> 0.94, of 150,000 6.16 -> 0.99 and 9.25 -> 2.02, of
-    // 300,000 1.29 -> 0.88 and 10.1 -> 4.4, of 440,000 1.24 -> 1.11 and 10.2 -> 6.0; galaxies of 100,000
-    // 0.64 -> 0.45 and 3.05 -> 1.23, of 300,000 0.76 -> 0.79 and 4.25 -> 3.91; clustered boxes of 150,000
-    // 0.66 -> 0.56 and 3.35 -> 1.85, of 440,000 1.29 -> 1.22 and 7.7 -> 5.5.  At 4 windows per warp
+    // 300,000 1.25 -> 0.92 and 10.0 -> 4.5, of 440,000 1.27 -> 1.09 and 10.7 -> 6.0; galaxies of 100,000
+    // 0.64 -> 0.45 and 3.05 -> 1.23, of 300,000 0.75 -> 0.78 and 4.42 -> 3.93, of 400,000 0.95 -> 0.95 at
+    // 0.0025 (with a budget of 192 1.02, with 320 0.95; the sphere of 300,000 0.87 and 1.10); clustered
+    // boxes of 150,000 0.66 -> 0.56 and 3.35 -> 1.85, of 440,000 1.32 -> 1.19 and 7.5 -> 5.4.  At 4 windows per warp
     // (2^22 particles) the hand-over only adds work.
     const int64_t tree_units = paired ? ((t->n_live + param - 1) / param + 1) / 2 : 0;
     const int64_t units = ((all || t->n_systems > 1 ? ng : (nt + param - 1) / std::max(1, param)) + 1) / 2;
@@ -2913,7 +2919,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     int budget = 0, hand_least = 64, share_least = 4, shares = 16;
     if (paired && tree_units >= (int64_t)40 * t->n_systems && tree_units < 2 * resident) {
         budget = tree_units <= resident / 3 ? 32 : tree_units <= resident * 3 / 5 ? 96 : 192;
-        if (tree_units > resident) { hand_least = 256; share_least = 64; shares = 8; }
+        if (tree_units > resident) { budget = 224; hand_least = 256; share_least = 64; shares = 8; }
     }
     // a record for every pair, within reason: a list of targets can name more windows than the tree has
     const int hand_cap = budget > 0 ? (int)std::min<int64_t>(units, 2 * resident) : 0;
