@@ -1172,8 +1172,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3) walk_pair_kernel(const Walk
     // (a share's warp has its first unit by its number: where nobody handed over, the launch ends without
     // an atomic per warp)
     for (int turn = 0;; ++turn) {
-        int unit = gw;
-        if (!SHARE || turn > 0) {
+        int unit = 0;
+        if (SHARE && turn == 0) {
+            unit = gw;
+        } else {
             if (lane == 0) unit = (int)atomicAdd(SHARE ? A.hand_ctr + 1 : A.next_group, 1u);
             unit = __shfl_sync(kFull, unit, 0);
             if (SHARE) unit += gridDim.x * (blockDim.x >> 5);
