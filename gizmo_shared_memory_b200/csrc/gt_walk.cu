@@ -2543,6 +2543,9 @@ int share_grid(gt_context* ctx, int records, int shares, int warps) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * 3, (units + warps - 1) / warps));
 }
 
+// Stack entries of a warp of that launch: it breaks up no stack and sets nothing aside.
+int share_stack(int stack_cap) { return stack_cap - kHandStack - kHandSums; }
+
 template <bool POT, bool CNT, int MAC, bool HAND, bool SHARE>
 void launch_pair_kernel(gt_context* ctx, const WalkArgs& a, int blocks, int warps) {
     prepare_pair<POT, CNT, MAC, HAND, SHARE>();
@@ -2556,8 +2559,11 @@ void launch_pair(gt_context* ctx, const WalkArgs& a, int blocks, int warps) {
         launch_pair_kernel<POT, CNT, MAC, false, false>(ctx, a, blocks, warps);
     } else {
         launch_pair_kernel<POT, CNT, MAC, true, false>(ctx, a, blocks, warps);
-        if (a.hand_cap > 0)
-            launch_pair_kernel<POT, CNT, MAC, false, true>(ctx, a, share_grid(ctx, a.hand_cap, a.shares, warps), warps);
+        if (a.hand_cap > 0) {
+            WalkArgs b = a;
+            b.stack_cap = share_stack(a.stack_cap);
+            launch_pair_kernel<POT, CNT, MAC, false, true>(ctx, b, share_grid(ctx, a.hand_cap, a.shares, warps), warps);
+        }
     }
 }
 
@@ -2953,7 +2959,11 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
     a.phi = rq.phi;
     a.out_map = (all && rq.out_original) ? t->order : nullptr;
     // a warp of either launch needs a traversal stack
-    const int total_warps = std::max(blocks, budget > 0 ? share_grid(ctx, hand_cap, shares, warps) : 0) * warps;
+    auto stacks_of = [&](int cap) {
+        const size_t first = (size_t)blocks * warps * cap;
+        if (budget <= 0) return first * 4;
+        return std::max(first, (size_t)share_grid(ctx, hand_cap, shares, warps) * warps * share_stack(cap)) * 4;
+    };
     a.pn_cap = pn_cap;
     a.pp_cap = pn_cap / 2;
     a.warp_bytes = paired ? pair_smem_bytes(a.pn_cap, a.pp_cap) : warp_smem_bytes(a.pn_cap, a.pp_cap, ext);
@@ -3064,7 +3074,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         check_cuda(cudaMemcpyAsync(ctx->pinned, bounds, sizeof(hb), cudaMemcpyDeviceToHost, st), "d2h");
         check_cuda(cudaStreamSynchronize(st), "sync");
         std::memcpy(hb, ctx->pinned, sizeof(hb));
-        const size_t stack_bytes = (size_t)total_warps * stack_cap * 4;
+        const size_t stack_bytes = stacks_of(stack_cap);
         if (wb) {
             own((void**)&wb->stack, wb->stack_bytes, stack_bytes);
             a.stack = wb->stack;
@@ -3198,9 +3208,8 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
         return true;
     }
 
-    records(a, kSlotHand, hand_cap);
     for (int attempt = 0; attempt < 3; ++attempt) {
-        const size_t stack_bytes = (size_t)total_warps * stack_cap * 4;
+        const size_t stack_bytes = stacks_of(stack_cap);
         if (wb) {
             own((void**)&wb->stack, wb->stack_bytes, stack_bytes);
             a.stack = wb->stack;
@@ -3208,6 +3217,7 @@ bool run_walk(gt_context* ctx, const gt_tree* tc, const WalkRequest& rq) {
             a.stack = (int*)scratch(ctx, kSlotStack, stack_bytes);
         }
         a.stack_cap = stack_cap;
+        if (attempt == 0) records(a, kSlotHand, hand_cap);  // after what the walk cannot do without
         check_cuda(cudaMemsetAsync(ctr, 0, kCtrBytes, st), "memset counters");
         if (!rq.capture) check_cuda(cudaEventRecord(ctx->ev0, st), "event");
         if (paired) dispatch_pair(ctx, a, blocks, warps, want_pot, rq.count, rq.mac);
